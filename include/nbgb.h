@@ -94,8 +94,8 @@ enum { NB_TREE_GEOMETRIC = 0, NB_TREE_REFERENCE = 1 };
 enum { NB_THETA_STANDARD = 0, NB_THETA_REFERENCE = 1 };
 
 /* Force accumulation precision.  NB_PRECISION_COMPENSATED keeps a TwoSum
- * low word per component; each batch of up to 32 opened children is summed
- * in FP32 and then added with one TwoSum. */
+ * low word per component; FP32 sums of at most 40 terms each, eight of them
+ * added in a fixed tree, go into it with one TwoSum. */
 enum { NB_PRECISION_FP32 = 0, NB_PRECISION_COMPENSATED = 1 };
 
 /* Cell expansion of the Barnes-Hut force.  NB_MULTIPOLE_MONOPOLE is the

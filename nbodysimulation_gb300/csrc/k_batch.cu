@@ -268,8 +268,7 @@ __global__ void __launch_bounds__(256) k_batch_sort(BatchTables t) {
 template <bool kQuad>
 struct BatchForceWarp {
     float dq[kMaxDepth];
-    int stack[kStack];
-    float4 bpm[8 * kBatch], cpm[8 * kBatch], cmeta[8 * kBatch], cqa[kQuad ? 8 * kBatch : 1];
+    WarpLists<kQuad> lists;
     // the current system's buffers and parameters: the walk reads them from
     // shared memory where the single-system kernel reads its kernel
     // parameters, instead of holding them in registers
@@ -285,7 +284,7 @@ constexpr int kBatchForceMaxWarps = 8;
 // Register budget: at most 48 a thread for the monopole walks (ten resident
 // blocks of four warps) and 64 with quadrupoles; neither spills.
 template <int kMethod, bool kComp, bool kQuad>
-__global__ void __launch_bounds__(kBatchForceMaxWarps * 32, kQuad ? 4 : 5) k_batch_force(BatchTables t) {
+__global__ void __launch_bounds__(kBatchForceMaxWarps * 32, 2) k_batch_force(BatchTables t) {
     extern __shared__ __align__(16) unsigned char force_smem[];
     BatchForceWarp<kQuad> &me = reinterpret_cast<BatchForceWarp<kQuad> *>(force_smem)[threadIdx.x >> 5];
     float *const s_dq_w = me.dq;
@@ -337,8 +336,7 @@ __global__ void __launch_bounds__(kBatchForceMaxWarps * 32, kQuad ? 4 : 5) k_bat
             if (i < s.n) s.body_next[i] = s.body_cur[i];
             continue;
         }
-        const WarpStage ws{me.stack, me.bpm, me.cpm, me.cmeta, me.cqa};
-        force_group<kMethod, kComp, false, kQuad>(s, s_par_w, s_dq_w, g, lane, ws);
+        force_group<kMethod, kComp, false, kQuad>(s, s_par_w, s_dq_w, g, lane, me.lists);
     }
 }
 

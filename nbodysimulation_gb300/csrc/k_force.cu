@@ -6,13 +6,9 @@
 namespace nbgb {
 
 template <int kMethod, bool kComp, bool kEpsZero, bool kQuad>
-__global__ void __launch_bounds__(kForceThreads) k_force(DevSim s, StepParams p) {
+__global__ void __launch_bounds__(kForceThreads, 8) k_force(DevSim s, StepParams p) {
     __shared__ float s_dq[kMaxDepth];
-    __shared__ int s_stack[kForceWarps][kStack];
-    __shared__ float4 s_bpm[kForceWarps][8 * kBatch];
-    __shared__ float4 s_cpm[kForceWarps][8 * kBatch];
-    __shared__ float4 s_cmeta[kForceWarps][8 * kBatch];
-    __shared__ float4 s_cqa[kForceWarps][kQuad ? 8 * kBatch : 1];
+    __shared__ WarpLists<kQuad> s_lists[kForceWarps];
     __shared__ int s_skip;
     Ctrl *ctrl = s.ctrl;
     const int n = s.n;
@@ -34,14 +30,13 @@ __global__ void __launch_bounds__(kForceThreads) k_force(DevSim s, StepParams p)
         return;
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const WarpStage ws{s_stack[w], s_bpm[w], s_cpm[w], s_cmeta[w], s_cqa[w]};
     const int ngroups = (n + 31) >> 5;
     while (true) {
         int g = 0;
         if (lane == 0) g = atomicAdd(&ctrl->work, 1);
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= ngroups) break;
-        force_group<kMethod, kComp, kEpsZero, kQuad>(s, p, s_dq, g, lane, ws);
+        force_group<kMethod, kComp, kEpsZero, kQuad>(s, p, s_dq, g, lane, s_lists[w]);
     }
 }
 
