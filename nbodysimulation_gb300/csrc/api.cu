@@ -51,6 +51,7 @@ struct nb_sim {
     int *top = nullptr;  // top-level tables: counts, start entries (kTopRegions each), level L-1 entries
     int top_levels = 0;
     bool quad = false;
+    int *grid = nullptr;  // collision update: counts, control words, starts, ranks
     Ctrl *ctrl = nullptr;
     Ctrl *h_ctrl = nullptr;       // pinned mirror for status read-back
     float *stage3 = nullptr;      // device staging, 3N floats
@@ -250,6 +251,9 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
         if (alloc_tree(s, cap) != NB_OK) return cleanup(NB_ERR_OUT_OF_MEMORY);
         if (dalloc(&s->sorted, n) != cudaSuccess) return cleanup(NB_ERR_OUT_OF_MEMORY);
     }
+    if (cfg->collision && s->n >= kCollideGridFrom &&
+        dalloc(&s->grid, 2 * (size_t)collide_buckets(s->n) + kGridCtl + n) != cudaSuccess)
+        return cleanup(NB_ERR_OUT_OF_MEMORY);
     if (cudaEventCreate(&s->t_begin) != cudaSuccess || cudaEventCreate(&s->t_end) != cudaSuccess)
         return cleanup(NB_ERR_CUDA);
     if (cudaDeviceSynchronize() != cudaSuccess) return cleanup(NB_ERR_CUDA);
@@ -262,7 +266,7 @@ nb_status nb_destroy(nb_sim *s) {
     cudaSetDevice(s->dev);
     if (s->stream) cudaStreamSynchronize(s->stream);
     cudaFree(s->body[0]); cudaFree(s->body[1]); cudaFree(s->vel); cudaFree(s->acc); cudaFree(s->part);
-    cudaFree(s->stage3); cudaFree(s->stage1); cudaFree(s->ctrl); cudaFree(s->sorted);
+    cudaFree(s->stage3); cudaFree(s->stage1); cudaFree(s->ctrl); cudaFree(s->sorted); cudaFree(s->grid);
     free_tree(s);
     if (s->h_ctrl) cudaFreeHost(s->h_ctrl);
     for (auto &e : s->ev)
@@ -484,8 +488,15 @@ static nb_status enqueue_step(nb_sim *s, float dt, int timed) {
         s->stage_ran[kStDirect] = true;
     }
     if (c.collision) {
-        NB_CUDA(s, launch_collision(d, s->tree ? 1 : 0, s->sm_count, st));
-        s->launches += 1;
+        CollideGrid g{};
+        if (s->grid) {  // the partial-sum buffer is free after the force stage
+            const int buckets = collide_buckets(s->n);
+            g = CollideGrid{s->grid, s->grid + buckets, s->grid + buckets + kGridCtl,
+                            s->grid + 2 * buckets + kGridCtl, s->part, (unsigned)buckets - 1u};
+        }
+        int collide_launches = 1;
+        NB_CUDA(s, launch_collision(d, g, s->tree ? 1 : 0, s->sm_count, st, &collide_launches));
+        s->launches += collide_launches;
         s->stage_ran[kStCollision] = true;
     }
     mark(6);

@@ -1,6 +1,6 @@
 // collide_device.cuh -- the collision update (update_collision_local,
 // kernels/collision_update.cl:17-83), shared by the single-system kernels
-// (k_direct.cu) and the batched one (k_batch.cu), so a batched system's
+// (k_collide.cu) and the batched one (k_batch.cu), so a batched system's
 // velocities equal a standalone handle's bit for bit.
 //
 // For target i, every other body j in ascending order: if |p_i - p_j| <=
@@ -33,8 +33,9 @@ constexpr int kCollideThreads = kCollideBlockBodies;  // targets per block of th
 constexpr int kCollideTile = 256;                     // bodies per staged tile (4 KiB)
 constexpr int kCollideWarps = 8;                      // targets per block of the warp form
 
-// The warp form serves systems with fewer blocks of targets than SMs (N <
-// 38,912 bodies on 152 SMs), the block form the rest.  Measured on a GB300,
+// Where the grid form (k_collide.cu) does not apply, the warp form serves fewer
+// blocks of targets than SMs (38,912 targets on 152 SMs), the block form the
+// rest.  Measured on a GB300,
 // unit ball, tree systems (targets in sort order), warp against block form:
 // N = 8,192 0.078 / 0.467 ms, 32,768 1.12 / 1.79 ms, 65,536 4.09 / 3.67 ms,
 // 262,144 62.0 / 25.6 ms.
@@ -84,11 +85,12 @@ __device__ __forceinline__ void reflect(const float4 me, const float4 q, float4 
 // Every thread of the block calls it.  Writes vel only when every wait
 // succeeded.
 __device__ __forceinline__ void collide_block(const float4 *__restrict__ pos, float4 *__restrict__ vel,
-                                              const int *__restrict__ order, int n, int i0, Ctrl *ctrl) {
+                                              const int *__restrict__ order, int targets, int n, int i0,
+                                              Ctrl *ctrl) {
     __shared__ __align__(128) float4 tile[2][kCollideTile];
     __shared__ __align__(8) uint64_t bar[2];
     const int it = i0 + (int)threadIdx.x;
-    const int i = it < n ? (order ? order[it] : it) : n;
+    const int i = it < targets ? (order ? order[it] : it) : n;
     const float4 me = i < n ? pos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float4 v = i < n ? vel[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const float rr = contact_distance();

@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kCollideThreads) k_batch_collision(BatchTables
     const SysDesc &d = t.sys[k];
     if (!system_live(d.v.ctrl) || read_status(d.v.ctrl)) return;  // block-uniform, before any barrier
     const DevSim s = system_view(d);
-    collide_block(s.body_next, s.vel, d.kind == kSysBH ? s.sorted : nullptr, s.n,
+    collide_block(s.body_next, s.vel, d.kind == kSysBH ? s.sorted : nullptr, s.n, s.n,
                   (blockIdx.x - d.cblock_begin) * kCollideThreads, s.ctrl);
 }
 

@@ -1,7 +1,6 @@
 // k_direct.cu -- all-pairs kernels: the direct sums (update /
-// update_local, kernels/brute_force_update.cl), the collision update
-// (kernels/collision_update.cl) and copy_vertices (kernels/copy_vertices.cl),
-// plus the host-layout pack/unpack kernels.
+// update_local, kernels/brute_force_update.cl) and copy_vertices
+// (kernels/copy_vertices.cl), plus the host-layout pack/unpack kernels.
 //
 // The tiled kernels stage j-tiles of packed {x,y,z,m} bodies into shared
 // memory with TMA bulk copies (cp.async.bulk ... mbarrier::complete_tx),
@@ -10,7 +9,7 @@
 // interactions.  Small systems split the j range over gridDim.y blocks and
 // combine partial accelerations with float atomics before a separate
 // integrate pass.
-#include "collide_device.cuh"
+#include "nbgb_internal.cuh"
 #include "tma.cuh"
 
 namespace nbgb {
@@ -249,26 +248,6 @@ __global__ void k_integrate_partial(DevSim s, StepParams p, const float4 *part) 
     integrate_one<kMethod>(s, p, i, s.body_cur[i], a.x * p.G, a.y * p.G, a.z * p.G);
 }
 
-// ---------------------------------------------------------------------------
-// collision update (update_collision_local, kernels/collision_update.cl:17-83;
-// collide_device.cuh).  It reads the positions the integrator of the same step
-// wrote, as the reference runs it after the force kernel
-// (src/MyApp.cpp:593-596).  A step that failed keeps its step-start state,
-// so the update does not run then.  Block form: one target per thread;
-// warp form (systems too small to fill the GPU with blocks): one target per
-// warp, 32 bodies tested at a time.  Both give the same bits.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kCollideThreads) k_collision(DevSim s, const int *order) {
-    if (read_status(s.ctrl)) return;  // block-uniform, before any barrier
-    collide_block(s.body_next, s.vel, order, s.n, blockIdx.x * kCollideThreads, s.ctrl);
-}
-
-__global__ void __launch_bounds__(kCollideWarps * 32) k_collision_warp(DevSim s) {
-    if (read_status(s.ctrl)) return;  // warp-uniform
-    const int lane = threadIdx.x & 31;
-    collide_warp(s.body_next, s.vel, s.n, blockIdx.x * kCollideWarps + (threadIdx.x >> 5), lane);
-}
-
 __global__ void k_copy_vertices(const float4 *__restrict__ b, int n, float4 *__restrict__ dst) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 p = b[i];
@@ -442,15 +421,6 @@ cudaError_t launch_direct(const DevSim &s, const StepParams &p, int tiled, int q
     case 3: return launch_direct_m<3>(s, p, p.eps, tiled, quirk, sm_count, st, part);
     default: return launch_direct_m<0>(s, p, p.eps, tiled, quirk, sm_count, st, part);
     }
-}
-
-cudaError_t launch_collision(const DevSim &s, int tree, int sm_count, cudaStream_t st) {
-    const int blocks = (s.n + kCollideThreads - 1) / kCollideThreads;
-    if (blocks < collide_warp_form_below(sm_count))
-        k_collision_warp<<<(s.n + kCollideWarps - 1) / kCollideWarps, kCollideWarps * 32, 0, st>>>(s);
-    else
-        k_collision<<<blocks, kCollideThreads, 0, st>>>(s, tree ? s.sorted : nullptr);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_copy_vertices(const float4 *body, int n, float4 *dst, cudaStream_t st) {

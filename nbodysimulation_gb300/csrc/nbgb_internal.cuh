@@ -250,8 +250,30 @@ cudaError_t launch_sort(const DevSim &s, int sm_count, cudaStream_t st);
 cudaError_t launch_force(const DevSim &s, const StepParams &p, int compensated, int sm_count, cudaStream_t st);
 cudaError_t launch_direct(const DevSim &s, const StepParams &p, int tiled, int quirk, int sm_count,
                           cudaStream_t st);
-// tree != 0: s.sorted holds this step's in-order sort (targets handed out in it)
-cudaError_t launch_collision(const DevSim &s, int tree, int sm_count, cudaStream_t st);
+// Scratch of the collision update's grid form (k_collide.cu): bucket counts
+// and, behind them, the control words; bucket starts; each body's place in its
+// bucket (then the overflow list); the bodies in bucket order.  All null: the
+// system takes the warp form.
+enum { kGridCursor = 0, kGridNoCell = 1, kGridOverflow = 2, kGridCtl = 4 };
+struct CollideGrid {
+    int *count, *ctl, *start, *rank;
+    float4 *body;
+    unsigned mask;  // buckets - 1
+};
+constexpr int kGridMinBuckets = 1024;  // one block of the scan
+inline int collide_buckets(int n) {
+    int b = kGridMinBuckets;
+    while (b < n) b <<= 1;
+    return b;
+}
+// Smallest system that takes the grid form: its six launches cost more than
+// the pair tests of a small system (unit ball, warp form against grid: N =
+// 2,048 0.024 / 0.044 ms, 4,096 0.042 / 0.046, 8,192 0.078 / 0.048).
+constexpr int kCollideGridFrom = 5120;
+// tree != 0: s.sorted holds this step's in-order sort (the block form hands
+// its targets out in it); *launches gets the kernel count
+cudaError_t launch_collision(const DevSim &s, const CollideGrid &g, int tree, int sm_count, cudaStream_t st,
+                             int *launches);
 cudaError_t launch_copy_vertices(const float4 *body, int n, float4 *dst, cudaStream_t st);
 cudaError_t launch_pack(const float *pos3, const float *mass, const float *vel3, float4 *body, float4 *vel,
                         float4 *acc, int n, cudaStream_t st);
