@@ -51,6 +51,8 @@ struct nb_sim {
     int *top = nullptr;  // top-level tables: counts, start entries (kTopRegions each), level L-1 entries
     int top_levels = 0;
     bool quad = false;
+    DirectPlan plan{1, 1};    // direct sum: how it is spread over the GPU
+    int *arrived = nullptr;   // and its slices' counters (behind part)
     int *grid = nullptr;  // collision update: counts, control words, starts, ranks
     Ctrl *ctrl = nullptr;
     Ctrl *h_ctrl = nullptr;       // pinned mirror for status read-back
@@ -233,16 +235,21 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->dev);
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return cleanup(NB_ERR_CUDA);
     const size_t n = (size_t)s->n;
+    s->tree = cfg->algo_config == NB_BARNES_HUT;
+    if (!s->tree) s->plan = direct_plan(s->n, s->sm_count, direct_slices_limit(s->n));
     bool ok = dalloc(&s->body[0], n) == cudaSuccess && dalloc(&s->body[1], n) == cudaSuccess &&
               dalloc(&s->vel, n) == cudaSuccess && dalloc(&s->acc, n) == cudaSuccess &&
-              dalloc(&s->part, n) == cudaSuccess && dalloc(&s->stage3, 3 * n) == cudaSuccess &&
+              dalloc(&s->part, n * s->plan.slices + (s->tree ? 0 : (n + 127) / 128)) == cudaSuccess && dalloc(&s->stage3, 3 * n) == cudaSuccess &&
               dalloc(&s->stage1, n) == cudaSuccess && dalloc(&s->ctrl, 1) == cudaSuccess;
     if (!ok) return cleanup(NB_ERR_OUT_OF_MEMORY);
     if (cudaMallocHost((void **)&s->h_ctrl, sizeof(Ctrl)) != cudaSuccess) return cleanup(NB_ERR_OUT_OF_MEMORY);
     cudaMemset(s->ctrl, 0, sizeof(Ctrl));
     cudaMemset(s->vel, 0, sizeof(float4) * n);
     cudaMemset(s->acc, 0, sizeof(float4) * n);
-    s->tree = cfg->algo_config == NB_BARNES_HUT;
+    if (!s->tree) {  // the counters lie behind the slices' sums
+        s->arrived = reinterpret_cast<int *>(s->part + n * s->plan.slices);
+        cudaMemset(s->arrived, 0, sizeof(int) * ((n + 31) / 32));
+    }
     s->quad = cfg->multipole == NB_MULTIPOLE_QUADRUPOLE;
     if (s->tree) {
         int cap = cfg->cell_capacity > 0 ? cfg->cell_capacity : default_capacity(s->n, s->sm_count);
@@ -483,8 +490,8 @@ static nb_status enqueue_step(nb_sim *s, float dt, int timed) {
         else p.eps = c.direct_epsilon >= 0.0f ? c.direct_epsilon : c.epsilon;
         mark(0);
         for (int k = 1; k <= 5; ++k) mark(k);
-        NB_CUDA(s, launch_direct(d, p, tiled ? 1 : 0, quirk ? 1 : 0, s->sm_count, st));
-        s->launches += 2;
+        NB_CUDA(s, launch_direct(d, p, s->plan, s->arrived, tiled ? 1 : 0, quirk ? 1 : 0, st));
+        s->launches += 1;
         s->stage_ran[kStDirect] = true;
     }
     if (c.collision) {

@@ -2,7 +2,7 @@
 // together.  Every stage of a step is one launch over all systems (the
 // kernels of k_batch.cu walk a device table of SysDesc), and one whole step
 // is captured into a CUDA graph that is replayed once per step.  The
-// direct-sum kernel's shape (bodies per thread, threads per block, j-tile)
+// direct-sum kernel's shape (targets per lane, warps per block)
 // is chosen by an autotuner that times the candidates on the batch and
 // keeps the choice in a JSON cache keyed by the batch's size profile.
 #include <cuda_runtime.h>
@@ -39,7 +39,7 @@ struct nb_batch {
     float *d_stage = nullptr;   // 4 * max N floats of transfer staging
     BatchTables t{};
     int method = NB_EULER, comp = 0, quad = 0;
-    int variant = 5;
+    int variant = kBatchDirectDefault;
     TreeShape shape{};  // launch shapes of the tree stages (autotuned)
     float dt = NAN;
     cudaGraph_t graph = nullptr;

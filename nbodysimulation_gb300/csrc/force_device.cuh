@@ -57,7 +57,8 @@
 // sees step-start positions (the reference integrates in place while other
 // work-items still read positions, :159-180).
 #pragma once
-#include "nbgb_internal.cuh"
+#include "integrate.cuh"
+#include "packed.cuh"
 
 namespace nbgb {
 
@@ -69,46 +70,6 @@ static_assert(kBatch == 8, "lane L holds child slot L%8 of popped cells L/8 and 
 constexpr int kBatchBelow = 128;  // batch pops only while the stack holds at most this many
 constexpr int kNodeBits = 26;
 constexpr int kNodeMask = (1 << kNodeBits) - 1;
-
-template <int kMethod>
-__device__ __forceinline__ void integrate_body(const DevSim &s, const StepParams &p, int b, const float4 P, float ax,
-                                               float ay, float az) {
-    const float dt = p.dt;
-    const float4 v = s.vel[b];
-    float4 x = P, vo = v;
-    if constexpr (kMethod == 2) {  // Euler (calculate_forces.cl:168-181)
-        vo.x = __fadd_rn(v.x, __fmul_rn(ax, dt));
-        vo.y = __fadd_rn(v.y, __fmul_rn(ay, dt));
-        vo.z = __fadd_rn(v.z, __fmul_rn(az, dt));
-        x.x = __fadd_rn(P.x, __fmul_rn(vo.x, dt));
-        x.y = __fadd_rn(P.y, __fmul_rn(vo.y, dt));
-        x.z = __fadd_rn(P.z, __fmul_rn(vo.z, dt));
-        s.acc[b] = make_float4(ax, ay, az, 0.0f);
-    } else if constexpr (kMethod == 1) {  // "Leapfrog" as written (:152-167): acc read, not written
-        const float4 ap = s.acc[b];
-        const float hx = __fadd_rn(v.x, __fmul_rn(__fmul_rn(ap.x, dt), 0.5f));
-        const float hy = __fadd_rn(v.y, __fmul_rn(__fmul_rn(ap.y, dt), 0.5f));
-        const float hz = __fadd_rn(v.z, __fmul_rn(__fmul_rn(ap.z, dt), 0.5f));
-        x.x = __fadd_rn(P.x, __fmul_rn(hx, dt));
-        x.y = __fadd_rn(P.y, __fmul_rn(hy, dt));
-        x.z = __fadd_rn(P.z, __fmul_rn(hz, dt));
-        vo.x = __fadd_rn(hx, __fmul_rn(__fmul_rn(ax, dt), 0.5f));
-        vo.y = __fadd_rn(hy, __fmul_rn(__fmul_rn(ay, dt), 0.5f));
-        vo.z = __fadd_rn(hz, __fmul_rn(__fmul_rn(az, dt), 0.5f));
-    } else if constexpr (kMethod == 3) {  // kick-drift-kick, velocities at half steps
-        const float h = p.kdk_primed ? dt : __fmul_rn(dt, 0.5f);
-        vo.x = __fadd_rn(v.x, __fmul_rn(ax, h));
-        vo.y = __fadd_rn(v.y, __fmul_rn(ay, h));
-        vo.z = __fadd_rn(v.z, __fmul_rn(az, h));
-        x.x = __fadd_rn(P.x, __fmul_rn(vo.x, dt));
-        x.y = __fadd_rn(P.y, __fmul_rn(vo.y, dt));
-        x.z = __fadd_rn(P.z, __fmul_rn(vo.z, dt));
-        s.acc[b] = make_float4(ax, ay, az, 0.0f);
-    } else {  // any other method value moves nothing (the as-wired reference)
-    }
-    s.vel[b] = vo;
-    s.body_next[b] = x;
-}
 
 // TwoSum (Knuth): hi + t = s + e exactly; e goes to the low word.
 __device__ __forceinline__ void two_sum_add(float &hi, float &lo, float t) {
@@ -152,10 +113,6 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 lo2(const float4 v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(const float4 v) { return make_float2(v.z, v.w); }
-
 // entry k's place is float 4 (k/2) + k%2 of the first row; the others follow
 // every kListC / 2 float4
 __device__ __forceinline__ void put_source(float *at, const float4 q) {
@@ -180,10 +137,6 @@ struct LaneBodies {
     float2 nx[4], ny[4], nz[4];
     float2 ax[4], ay[4], az[4];
 };
-
-__device__ __forceinline__ float2 pair_dist2(const float2 dx, const float2 dy, const float2 dz, float2 eps2) {
-    return __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, eps2)));
-}
 
 // One tile of monopole sources: the lane's pair over its four bodies.
 template <bool kEpsZero>

@@ -4,14 +4,14 @@
 // chunks, cell slots, warp groups, direct-sum target blocks) and a thread
 // finds its system with a binary search in the stage's prefix table.
 // Barnes-Hut systems run the same per-item code as the single-system
-// kernels (bh_device.cuh, force_device.cuh); small systems take the
-// TMA-tiled direct sum.  A step is: reset, bbox, top-level counts, top cells,
+// kernels (bh_device.cuh, force_device.cuh); small systems take the direct
+// sum (direct_device.cuh).  A step is: reset, bbox, top-level counts, top cells,
 // build, used-cell scan, summarize, sort, force, direct, flip -- captured
 // once into a CUDA graph by the host.
 #include "bh_device.cuh"
 #include "collide_device.cuh"
+#include "direct_device.cuh"
 #include "force_device.cuh"
-#include "tma.cuh"
 
 namespace nbgb {
 
@@ -341,90 +341,29 @@ __global__ void __launch_bounds__(kBatchForceMaxWarps * 32, 2) k_batch_force(Bat
 }
 
 // ---------------------------------------------------------------------------
-// direct: one block per kThreads*kI targets of one system; j-tiles of kTileB
-// bodies staged by TMA bulk copies (double-buffered mbarriers); Plummer
-// softening; fused integrator.  kI, kThreads and kTileB come from the
-// autotuner.
+// direct: one block per 32 kI targets of one system, its kW warps sharing the
+// system's bodies (direct_device.cuh); Plummer softening; fused integrator.  kI
+// and kW come from the autotuner; a system's sums depend on them and on nothing
+// beside it.
 // ---------------------------------------------------------------------------
-template <int kI, int kThreads, int kTileB>
-__global__ void __launch_bounds__(kThreads) k_batch_direct(BatchTables t) {
-    __shared__ __align__(128) float4 tile[2][kTileB];
-    __shared__ __align__(8) uint64_t bar[2];
+template <int kI, int kW>
+__global__ void __launch_bounds__(32 * kW) k_batch_direct(BatchTables t) {
+    __shared__ DirectShared<kW> sh;
     const int k = find_system(t.dblock_prefix, t.nsys, blockIdx.x);
     const SysDesc &d = t.sys[k];
     if (!system_live(d.v.ctrl)) return;  // block-uniform, before any barrier
     const DevSim s = system_view(d);
     StepParams p = d.p;
     p.kdk_primed = s.ctrl->kdk_primed;
-    const int n = s.n;
-    const int base = (blockIdx.x - d.dblock_begin) * (kThreads * kI);
-    const float eps2 = p.eps * p.eps;
-    int idx[kI];
-    float4 me[kI];
-    float ax[kI], ay[kI], az[kI];
-#pragma unroll
-    for (int r = 0; r < kI; ++r) {
-        idx[r] = base + r * kThreads + threadIdx.x;
-        me[r] = idx[r] < n ? s.body_cur[idx[r]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        ax[r] = ay[r] = az[r] = 0.0f;
-    }
-    if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    const int ntiles = (n + kTileB - 1) / kTileB;
-    auto issue = [&](int tt, int stage) {
-        const int cnt = min(kTileB, n - tt * kTileB);
-        const uint32_t bytes = (uint32_t)cnt * 16u;
-        mbar_expect_tx(&bar[stage], bytes);
-        bulk_g2s(&tile[stage][0], s.body_cur + (size_t)tt * kTileB, bytes, &bar[stage]);
-    };
-    if (threadIdx.x == 0 && ntiles > 0) issue(0, 0);
-    bool ok = true;
-    for (int tt = 0; tt < ntiles; ++tt) {
-        const int stage = tt & 1;
-        if (threadIdx.x == 0 && tt + 1 < ntiles) issue(tt + 1, stage ^ 1);
-        if (!mbar_wait_bounded(&bar[stage], (uint32_t)((tt >> 1) & 1), s.ctrl)) ok = false;
-        const int cnt = min(kTileB, n - tt * kTileB);
-        const float4 *tl = tile[stage];
-#pragma unroll 4
-        for (int j = 0; j < cnt; ++j) {
-            const float4 q = tl[j];
-#pragma unroll
-            for (int r = 0; r < kI; ++r) {
-                const float dx = q.x - me[r].x, dy = q.y - me[r].y, dz = q.z - me[r].z;
-                const float d2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-                const float rr = rsqrt_fast(d2);
-                const float F = (q.w * rr) * (rr * rr);
-                ax[r] = fmaf(dx, F, ax[r]);
-                ay[r] = fmaf(dy, F, ay[r]);
-                az[r] = fmaf(dz, F, az[r]);
-            }
-        }
-        if (!__syncthreads_and(ok)) {
-            if (threadIdx.x == 0 && tt + 1 < ntiles)
-                mbar_wait_bounded(&bar[stage ^ 1], (uint32_t)(((tt + 1) >> 1) & 1), s.ctrl);
-            ok = false;
-            break;
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < kI; ++r) {
-        if (idx[r] >= n) continue;
-        if (!ok) {
-            s.body_next[idx[r]] = me[r];
-            continue;
-        }
-        const float gx = ax[r] * p.G, gy = ay[r] * p.G, gz = az[r] * p.G;
-        switch (p.method) {
-        case 1: integrate_body<1>(s, p, idx[r], me[r], gx, gy, gz); break;
-        case 2: integrate_body<2>(s, p, idx[r], me[r], gx, gy, gz); break;
-        case 3: integrate_body<3>(s, p, idx[r], me[r], gx, gy, gz); break;
-        default: integrate_body<0>(s, p, idx[r], me[r], gx, gy, gz); break;
-        }
-    }
+    const int n = s.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int base = (blockIdx.x - d.dblock_begin) * (32 * kI), i0 = base + lane;
+    DirectTargets<kI> T;
+    direct_load_targets<kI>(s.body_cur, i0, n, T);
+    direct_sum<kI, kW, false, kZeroAdds>(s.body_cur, 0, n, i0, p.eps, warp, lane, sh, T);
+    const float3 a = direct_block_sum<kI, kW>(sh, T, warp, lane);
+    const int i = base + (int)threadIdx.x;
+    if (threadIdx.x < 32 * kI && i < n)
+        integrate_any(s, p, i, s.body_cur[i], a.x * p.G, a.y * p.G, a.z * p.G);
 }
 
 // ---------------------------------------------------------------------------
@@ -472,36 +411,33 @@ static int resident(const void *fn, int threads, int sm_count) {
     return per_sm * sm_count;
 }
 
-// Direct-sum variants the autotuner chooses from: {bodies per thread,
-// threads per block, j-tile bodies}.
+// Direct-sum variants the autotuner chooses from: {targets per lane, warps per
+// block}.
 struct DirectVariant {
-    int ki, threads, tile;
+    int ki, warps;
 };
-static const DirectVariant kDirectVariants[] = {{1, 128, 128}, {1, 128, 256}, {1, 256, 256}, {2, 128, 128},
-                                                {2, 128, 256}, {2, 256, 256}, {4, 128, 256}, {4, 256, 256},
-                                                {1, 64, 256},  {2, 64, 256},  {4, 64, 256}};
+static const DirectVariant kDirectVariants[] = {{1, 4}, {1, 8},  {2, 4}, {2, 8},  {4, 4}, {4, 8},
+                                                {1, 2}, {1, 16}, {2, 2}, {2, 16}, {4, 16}};
 constexpr int kNumDirectVariants = sizeof(kDirectVariants) / sizeof(kDirectVariants[0]);
+static_assert(kBatchDirectDefault < kNumDirectVariants, "the default is one of the variants");
 
 int batch_direct_variants() { return kNumDirectVariants; }
-int batch_direct_block_bodies(int variant) {
-    const DirectVariant &v = kDirectVariants[variant];
-    return v.ki * v.threads;
-}
+int batch_direct_block_bodies(int variant) { return 32 * kDirectVariants[variant].ki; }
 
 static cudaError_t launch_direct_variant(const BatchTables &t, int variant, cudaStream_t st) {
     const int b = t.dblocks;
     switch (variant) {
-    case 0: k_batch_direct<1, 128, 128><<<b, 128, 0, st>>>(t); break;
-    case 1: k_batch_direct<1, 128, 256><<<b, 128, 0, st>>>(t); break;
-    case 2: k_batch_direct<1, 256, 256><<<b, 256, 0, st>>>(t); break;
-    case 3: k_batch_direct<2, 128, 128><<<b, 128, 0, st>>>(t); break;
-    case 4: k_batch_direct<2, 128, 256><<<b, 128, 0, st>>>(t); break;
-    case 5: k_batch_direct<2, 256, 256><<<b, 256, 0, st>>>(t); break;
-    case 6: k_batch_direct<4, 128, 256><<<b, 128, 0, st>>>(t); break;
-    case 7: k_batch_direct<4, 256, 256><<<b, 256, 0, st>>>(t); break;
-    case 8: k_batch_direct<1, 64, 256><<<b, 64, 0, st>>>(t); break;
-    case 9: k_batch_direct<2, 64, 256><<<b, 64, 0, st>>>(t); break;
-    default: k_batch_direct<4, 64, 256><<<b, 64, 0, st>>>(t); break;
+    case 0: k_batch_direct<1, 4><<<b, 128, 0, st>>>(t); break;
+    case 1: k_batch_direct<1, 8><<<b, 256, 0, st>>>(t); break;
+    case 2: k_batch_direct<2, 4><<<b, 128, 0, st>>>(t); break;
+    case 3: k_batch_direct<2, 8><<<b, 256, 0, st>>>(t); break;
+    case 4: k_batch_direct<4, 4><<<b, 128, 0, st>>>(t); break;
+    case 5: k_batch_direct<4, 8><<<b, 256, 0, st>>>(t); break;
+    case 6: k_batch_direct<1, 2><<<b, 64, 0, st>>>(t); break;
+    case 7: k_batch_direct<1, 16><<<b, 512, 0, st>>>(t); break;
+    case 8: k_batch_direct<2, 2><<<b, 64, 0, st>>>(t); break;
+    case 9: k_batch_direct<2, 16><<<b, 512, 0, st>>>(t); break;
+    default: k_batch_direct<4, 16><<<b, 512, 0, st>>>(t); break;
     }
     return cudaGetLastError();
 }

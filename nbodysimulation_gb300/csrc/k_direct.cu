@@ -2,250 +2,63 @@
 // update_local, kernels/brute_force_update.cl) and copy_vertices
 // (kernels/copy_vertices.cl), plus the host-layout pack/unpack kernels.
 //
-// The tiled kernels stage j-tiles of packed {x,y,z,m} bodies into shared
-// memory with TMA bulk copies (cp.async.bulk ... mbarrier::complete_tx),
-// double-buffered, no cluster and no multicast; each thread keeps kI target
-// bodies in registers so one broadcast shared-memory load feeds kI
-// interactions.  Small systems split the j range over gridDim.y blocks and
-// combine partial accelerations with float atomics before a separate
-// integrate pass.
-#include "nbgb_internal.cuh"
-#include "tma.cuh"
+// The direct sums are direct_device.cuh's; this file splits them over the GPU.
+#include <algorithm>
+
+#include "direct_device.cuh"
+#include "integrate.cuh"
 
 namespace nbgb {
 
-constexpr int kTile = 256;          // bodies per staged tile (4 KiB)
-constexpr int kDirectThreads = 256;  // allocation-free all-pairs kernel
-constexpr int kTiledThreads = 64;    // tiled direct sum: small blocks, many per SM, even load
-
-// ---- pair interactions ----
-template <bool kQuirk, bool kEpsZero>
-__device__ __forceinline__ void pair(const float4 me, const float4 q, float eps2, float &ax, float &ay, float &az) {
-    const float dx = q.x - me.x, dy = q.y - me.y, dz = q.z - me.z;
-    if constexpr (!kQuirk) {
-        const float d2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
-        const float r = rsqrt_fast(d2);
-        float F = (q.w * r) * (r * r);
-        if constexpr (kEpsZero) F = d2 > 0.0f ? F : 0.0f;
-        ax = fmaf(dx, F, ax);
-        ay = fmaf(dy, F, ay);
-        az = fmaf(dz, F, az);
-    } else {
-        // the reference's brute-force arithmetic: n = normalize(r),
-        // s = m / (|n|^2 + e^2) (brute_force_update.cl:54-60, 114-123);
-        // the zero vector normalises to zero, so the self pair adds nothing
-        const float l2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        const float inv = l2 > 0.0f ? rsqrtf(l2) : 0.0f;
-        const float nx = dx * inv, ny = dy * inv, nz = dz * inv;
-        const float dist_sqr = fmaf(nz, nz, fmaf(ny, ny, fmaf(nx, nx, eps2)));
-        const float s = __fdividef(q.w, dist_sqr);
-        ax = fmaf(nx, s, ax);
-        ay = fmaf(ny, s, ay);
-        az = fmaf(nz, s, az);
-    }
-}
-
-template <int kMethod>
-__device__ __forceinline__ void integrate_one(const DevSim &s, const StepParams &p, int b, const float4 P, float ax,
-                                              float ay, float az) {
-    const float dt = p.dt;
-    const float4 v = s.vel[b];
-    float4 x = P, vo = v;
-    if constexpr (kMethod == 2) {
-        vo.x = __fadd_rn(v.x, __fmul_rn(ax, dt));
-        vo.y = __fadd_rn(v.y, __fmul_rn(ay, dt));
-        vo.z = __fadd_rn(v.z, __fmul_rn(az, dt));
-        x.x = __fadd_rn(P.x, __fmul_rn(vo.x, dt));
-        x.y = __fadd_rn(P.y, __fmul_rn(vo.y, dt));
-        x.z = __fadd_rn(P.z, __fmul_rn(vo.z, dt));
-        s.acc[b] = make_float4(ax, ay, az, 0.0f);
-    } else if constexpr (kMethod == 1) {
-        const float4 ap = s.acc[b];
-        const float hx = __fadd_rn(v.x, __fmul_rn(__fmul_rn(ap.x, dt), 0.5f));
-        const float hy = __fadd_rn(v.y, __fmul_rn(__fmul_rn(ap.y, dt), 0.5f));
-        const float hz = __fadd_rn(v.z, __fmul_rn(__fmul_rn(ap.z, dt), 0.5f));
-        x.x = __fadd_rn(P.x, __fmul_rn(hx, dt));
-        x.y = __fadd_rn(P.y, __fmul_rn(hy, dt));
-        x.z = __fadd_rn(P.z, __fmul_rn(hz, dt));
-        vo.x = __fadd_rn(hx, __fmul_rn(__fmul_rn(ax, dt), 0.5f));
-        vo.y = __fadd_rn(hy, __fmul_rn(__fmul_rn(ay, dt), 0.5f));
-        vo.z = __fadd_rn(hz, __fmul_rn(__fmul_rn(az, dt), 0.5f));
-    } else if constexpr (kMethod == 3) {
-        const float h = p.kdk_primed ? dt : __fmul_rn(dt, 0.5f);
-        vo.x = __fadd_rn(v.x, __fmul_rn(ax, h));
-        vo.y = __fadd_rn(v.y, __fmul_rn(ay, h));
-        vo.z = __fadd_rn(v.z, __fmul_rn(az, h));
-        x.x = __fadd_rn(P.x, __fmul_rn(vo.x, dt));
-        x.y = __fadd_rn(P.y, __fmul_rn(vo.y, dt));
-        x.z = __fadd_rn(P.z, __fmul_rn(vo.z, dt));
-        s.acc[b] = make_float4(ax, ay, az, 0.0f);
-    }
-    s.vel[b] = vo;
-    s.body_next[b] = x;
-}
-
 // ---------------------------------------------------------------------------
-// direct_global: one thread per body, j straight from global memory through
-// L1 (update, brute_force_update.cl:3-105), no shared-memory staging.  When
-// the bodies alone do not fill the GPU (the reference runs this variant at
-// N = 4096: 32 blocks for 152 SMs), gridDim.y blocks split the j range and
-// add partial accelerations into `part` (float atomics) for a separate
-// integrate pass.
+// One block: 32 kI targets (blockIdx.x) over one of gridDim.y slices of the
+// bodies.  With one slice the block integrates its targets; with more it
+// writes its sums to part[slice][target], and the block that finishes a
+// target set last adds the slices in order and integrates: one launch, no
+// atomics on the sums, the same bits every time.  `arrived` counts the blocks
+// of each set that are done; the last one puts it back to zero.
+// out (allocation-free form): accelerations instead of the integrator.
 // ---------------------------------------------------------------------------
-constexpr int kGlobalThreads = 128;
-template <int kMethod, bool kQuirk, bool kEpsZero>
-__global__ void __launch_bounds__(kGlobalThreads) k_direct_global(DevSim s, StepParams p, float eps, float4 *part) {
-    const int n = s.n;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int per = (n + gridDim.y - 1) / gridDim.y;
+constexpr int kDirectWarps = 8;
+template <int kI, bool kQuirk, int kZero>
+__global__ void __launch_bounds__(32 * kDirectWarps, kI == 4 ? 2 : 3)
+    k_direct(DevSim s, StepParams p, float4 *part, int *arrived, float4 *out) {
+    __shared__ DirectShared<kDirectWarps> sh;
+    __shared__ int last;
+    const int n = s.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int base = blockIdx.x * (32 * kI), i0 = base + lane;
+    // slices of whole tiles
+    const int tiles = (n + kDirectTile - 1) / kDirectTile;
+    const int per = (tiles + gridDim.y - 1) / gridDim.y * kDirectTile;
     const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
-    const float4 me = s.body_cur[i];
-    const float eps2 = eps * eps;
-    float ax = 0.0f, ay = 0.0f, az = 0.0f;
-    for (int j = j0; j < j1; ++j) {
-        const float4 q = __ldg(&s.body_cur[j]);
-        if (!kQuirk && kEpsZero && j == i) continue;
-        pair<kQuirk, false>(me, q, eps2, ax, ay, az);
-    }
-    if (gridDim.y == 1) {
-        integrate_one<kMethod>(s, p, i, me, ax * p.G, ay * p.G, az * p.G);
-    } else {
-        atomicAdd(&part[i].x, ax);
-        atomicAdd(&part[i].y, ay);
-        atomicAdd(&part[i].z, az);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// direct_tiled (update_local, brute_force_update.cl:128-228): TMA-staged
-// j-tiles.  The reference's tile loop reloads tile 0 and skips the wrong body
-// (:167-184); here every j is visited once.
-//
-// A block is kG groups of 64 threads that share the same 64*kI targets and
-// split the j range between them: each stage brings kG consecutive tiles,
-// group g takes the g-th, and at the end the groups' partial sums are added
-// in group order (deterministic).  More warps per target set hide the MUFU
-// and shared-memory latencies without more shared-memory loads per pair.
-// gridDim.y > 1 splits the j range over blocks as well and accumulates the
-// partial accelerations into `part` (float atomics).
-// ---------------------------------------------------------------------------
-template <int kI, int kG, int kMethod, bool kQuirk, bool kEpsZero>
-__global__ void __launch_bounds__(kTiledThreads *kG) k_direct_tiled(DevSim s, StepParams p, float eps, float4 *part) {
-    __shared__ __align__(128) float4 tile[2][kG][kTile];
-    __shared__ __align__(8) uint64_t bar[2];
-    __shared__ float red[kG > 1 ? kG - 1 : 1][3 * kI][kTiledThreads];
-    const int n = s.n;
-    const int grp = threadIdx.x / kTiledThreads, gl = threadIdx.x % kTiledThreads;
-    const int ntiles = (n + kTile - 1) / kTile;
-    const int per_split = (ntiles + gridDim.y - 1) / gridDim.y;
-    const int t0 = blockIdx.y * per_split;
-    const int t1 = min(ntiles, t0 + per_split);
-    const int nst = (t1 - t0 + kG - 1) / kG;  // stages of kG tiles
-    const float eps2 = eps * eps;
-    int idx[kI];
-    float4 me[kI];
-    float ax[kI], ay[kI], az[kI];
-#pragma unroll
-    for (int r = 0; r < kI; ++r) {
-        idx[r] = blockIdx.x * (kTiledThreads * kI) + r * kTiledThreads + gl;
-        me[r] = idx[r] < n ? s.body_cur[idx[r]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        ax[r] = ay[r] = az[r] = 0.0f;
-    }
-    if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    auto issue = [&](int st, int stage) {
-        uint32_t total = 0;
-#pragma unroll
-        for (int g = 0; g < kG; ++g) {
-            const int t = t0 + st * kG + g;
-            if (t < t1) total += (uint32_t)min(kTile, n - t * kTile) * 16u;
-        }
-        mbar_expect_tx(&bar[stage], total);
-#pragma unroll
-        for (int g = 0; g < kG; ++g) {
-            const int t = t0 + st * kG + g;
-            if (t < t1)
-                bulk_g2s(&tile[stage][g][0], s.body_cur + (size_t)t * kTile,
-                         (uint32_t)min(kTile, n - t * kTile) * 16u, &bar[stage]);
-        }
-    };
-    if (threadIdx.x == 0 && nst > 0) issue(0, 0);
-    bool ok = true;
-    for (int st = 0; st < nst; ++st) {
-        const int stage = st & 1;
-        if (threadIdx.x == 0 && st + 1 < nst) issue(st + 1, stage ^ 1);
-        if (!mbar_wait_bounded(&bar[stage], (uint32_t)((st >> 1) & 1), s.ctrl)) ok = false;
-        const int t = t0 + st * kG + grp;
-        const int cnt = t < t1 ? min(kTile, n - t * kTile) : 0;
-        const float4 *tl = tile[stage][grp];
-        if (cnt == kTile) {
-#pragma unroll 4
-            for (int j = 0; j < kTile; ++j) {
-                const float4 q = tl[j];
-#pragma unroll
-                for (int r = 0; r < kI; ++r) pair<kQuirk, kEpsZero>(me[r], q, eps2, ax[r], ay[r], az[r]);
-            }
-        } else {
-            for (int j = 0; j < cnt; ++j) {
-                const float4 q = tl[j];
-#pragma unroll
-                for (int r = 0; r < kI; ++r) pair<kQuirk, kEpsZero>(me[r], q, eps2, ax[r], ay[r], az[r]);
-            }
-        }
-        if (!__syncthreads_and(ok)) {
-            // drain the copies already issued for the next stage before leaving
-            if (threadIdx.x == 0 && st + 1 < nst)
-                mbar_wait_bounded(&bar[stage ^ 1], (uint32_t)(((st + 1) >> 1) & 1), s.ctrl);
-            ok = false;
-            break;
-        }
-    }
-    if (!ok) return;
-    if constexpr (kG > 1) {
-        if (grp > 0) {
-#pragma unroll
-            for (int r = 0; r < kI; ++r) {
-                red[grp - 1][3 * r][gl] = ax[r];
-                red[grp - 1][3 * r + 1][gl] = ay[r];
-                red[grp - 1][3 * r + 2][gl] = az[r];
-            }
-        }
+    DirectTargets<kI> T;
+    direct_load_targets<kI>(s.body_cur, i0, n, T);
+    direct_sum<kI, kDirectWarps, kQuirk, kZero>(s.body_cur, j0, j1, i0, p.eps, warp, lane, sh, T);
+    float3 a = direct_block_sum<kI, kDirectWarps>(sh, T, warp, lane);
+    const int i = base + (int)threadIdx.x;
+    const bool mine = threadIdx.x < 32 * kI && i < n;
+    if (gridDim.y > 1) {
+        if (mine) part[(size_t)blockIdx.y * n + i] = make_float4(a.x, a.y, a.z, 0.0f);
+        __threadfence();  // the sums before the arrival
         __syncthreads();
-        if (grp > 0) return;
-#pragma unroll
-        for (int g = 1; g < kG; ++g) {
-#pragma unroll
-            for (int r = 0; r < kI; ++r) {
-                ax[r] += red[g - 1][3 * r][gl];
-                ay[r] += red[g - 1][3 * r + 1][gl];
-                az[r] += red[g - 1][3 * r + 2][gl];
+        if (threadIdx.x == 0) last = atomicAdd(&arrived[blockIdx.x], 1) == (int)gridDim.y - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        if (threadIdx.x == 0) arrived[blockIdx.x] = 0;
+        if (mine) {
+            a = make_float3(0.0f, 0.0f, 0.0f);
+            for (int k = 0; k < (int)gridDim.y; ++k) {
+                const float4 v = __ldcg(&part[(size_t)k * n + i]);
+                a.x += v.x;
+                a.y += v.y;
+                a.z += v.z;
             }
         }
     }
-#pragma unroll
-    for (int r = 0; r < kI; ++r) {
-        if (idx[r] >= n) continue;
-        if (gridDim.y == 1) {
-            integrate_one<kMethod>(s, p, idx[r], me[r], ax[r] * p.G, ay[r] * p.G, az[r] * p.G);
-        } else {
-            atomicAdd(&part[idx[r]].x, ax[r]);
-            atomicAdd(&part[idx[r]].y, ay[r]);
-            atomicAdd(&part[idx[r]].z, az[r]);
-        }
-    }
-}
-
-template <int kMethod>
-__global__ void k_integrate_partial(DevSim s, StepParams p, const float4 *part) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= s.n) return;
-    const float4 a = part[i];
-    integrate_one<kMethod>(s, p, i, s.body_cur[i], a.x * p.G, a.y * p.G, a.z * p.G);
+    if (!mine) return;
+    if (out) out[i] = make_float4(a.x * p.G, a.y * p.G, a.z * p.G, 0.0f);
+    else integrate_any(s, p, i, s.body_cur[i], a.x * p.G, a.y * p.G, a.z * p.G);
 }
 
 __global__ void k_copy_vertices(const float4 *__restrict__ b, int n, float4 *__restrict__ dst) {
@@ -339,88 +152,57 @@ __global__ void __launch_bounds__(kPackTile) k_unpack(const float4 *__restrict__
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-template <int kMethod, bool kQuirk, bool kEpsZero>
-static cudaError_t launch_direct_t(const DevSim &s, const StepParams &p, float eps, int tiled, int sm_count,
-                                   cudaStream_t st, float4 *part) {
-    const int n = s.n;
-    if (!tiled) {
-        const int bx = (n + kGlobalThreads - 1) / kGlobalThreads;
-        int split = (sm_count * 6 + bx - 1) / bx;
-        if (split > (n + 63) / 64) split = (n + 63) / 64;  // at least 64 j per block
-        if (split <= 1) {
-            k_direct_global<kMethod, kQuirk, kEpsZero><<<dim3(bx, 1), kGlobalThreads, 0, st>>>(s, p, eps, part);
-            return cudaGetLastError();
+// Targets per lane and slices of the bodies: the pair that a model of the
+// busiest SM finds fastest.  A block costs its tiles (64 bodies against 32 kI
+// targets, divided over the warps), a pair somewhat more at small kI, plus a
+// fixed part; an SM with one block is not kept busy by its eight warps; slices
+// cost the exchange of their sums.  In units of one round of tiles of 32
+// targets.  Fitted to every (kI, slices) timed on a GB300 at twelve sizes; what
+// it takes is within 1 % of the best of them from 8,192 bodies up (20,000: kI =
+// 2, 10 slices 160 us, best 158, one slice of kI = 4 252; 262,144: kI = 4 24.65
+// ms, kI = 2 24.91, kI = 1 26.57) and within one launch quantum (2 us) below.
+DirectPlan direct_plan(int n, int sm_count, int max_slices) {
+    static const float kPair[3] = {1.05f, 1.02f, 1.0f};  // kI = 1, 2, 4
+    const int tiles = (n + kDirectTile - 1) / kDirectTile;
+    DirectPlan best{1, 1};
+    float best_cost = 0.0f;
+    for (int v = 0; v < 3; ++v) {
+        const int ki = 1 << v;
+        const long long sets = ((long long)n + 32 * ki - 1) / (32 * ki);
+        for (int slices = 1; slices <= max_slices; ++slices) {
+            const int per = (tiles + slices - 1) / slices;  // tiles a block
+            if (slices > 1 && (long long)(slices - 1) * per >= tiles) continue;  // an empty slice
+            const long long on_sm = (sets * slices + sm_count - 1) / sm_count;
+            const float sum = (float)((per + kDirectWarps - 1) / kDirectWarps) * ki * kPair[v];
+            const float cost = (float)on_sm * (sum * (on_sm == 1 ? 1.4f : 1.0f) + 0.3f) + (slices > 1 ? 2.0f : 0.0f);
+            if (best_cost == 0.0f || cost < best_cost) {
+                best_cost = cost;
+                best = DirectPlan{ki, slices};
+            }
         }
-        cudaError_t e = cudaMemsetAsync(part, 0, sizeof(float4) * (size_t)n, st);
-        if (e != cudaSuccess) return e;
-        k_direct_global<kMethod, kQuirk, kEpsZero><<<dim3(bx, split), kGlobalThreads, 0, st>>>(s, p, eps, part);
-        k_integrate_partial<kMethod><<<(n + 255) / 256, 256, 0, st>>>(s, p, part);
-        return cudaGetLastError();
     }
-    // bodies per thread: the most that still gives at least six blocks per
-    // SM (every block does the same work, so many small blocks keep the SMs
-    // evenly loaded), two j-groups per block; below that, split the j range
-    // over gridDim.y
-    const int want = sm_count * 6;
-    const int bx4 = (n + kTiledThreads * 4 - 1) / (kTiledThreads * 4);
-    const int bx3 = (n + kTiledThreads * 3 - 1) / (kTiledThreads * 3);
-    const int bx2 = (n + kTiledThreads * 2 - 1) / (kTiledThreads * 2);
-    const int bx1 = (n + kTiledThreads - 1) / kTiledThreads;
-    const int ntiles = (n + kTile - 1) / kTile;
-    if (bx4 >= want) {
-        // every block does the same work, so the busiest SM holds
-        // ceil(blocks / SMs) of them: 3 targets per thread when that evens
-        // the SMs out enough to pay for the extra shared-memory load per pair
-        // (N = 262,144: 1024 blocks of 4 -> 7 on the busiest SM, 28 target
-        // rows; 1366 blocks of 3 -> 9, 27)
-        const long long cost4 = 4LL * ((bx4 + sm_count - 1) / sm_count);
-        const long long cost3 = 3LL * ((bx3 + sm_count - 1) / sm_count);
-        if (cost3 < cost4) {
-            k_direct_tiled<3, 2, kMethod, kQuirk, kEpsZero><<<dim3(bx3, 1), 2 * kTiledThreads, 0, st>>>(s, p, eps,
-                                                                                                     part);
-            return cudaGetLastError();
-        }
-        k_direct_tiled<4, 2, kMethod, kQuirk, kEpsZero><<<dim3(bx4, 1), 2 * kTiledThreads, 0, st>>>(s, p, eps, part);
-        return cudaGetLastError();
-    }
-    if (bx2 >= want) {
-        k_direct_tiled<2, 2, kMethod, kQuirk, kEpsZero><<<dim3(bx2, 1), 2 * kTiledThreads, 0, st>>>(s, p, eps, part);
-        return cudaGetLastError();
-    }
-    int split = (want + bx1 - 1) / bx1;
-    if (split > ntiles) split = ntiles;
-    if (split < 1) split = 1;
-    if (split == 1) {
-        k_direct_tiled<1, 1, kMethod, kQuirk, kEpsZero><<<dim3(bx1, 1), kTiledThreads, 0, st>>>(s, p, eps, part);
-        return cudaGetLastError();
-    }
-    cudaError_t e = cudaMemsetAsync(part, 0, sizeof(float4) * (size_t)n, st);
-    if (e != cudaSuccess) return e;
-    k_direct_tiled<1, 1, kMethod, kQuirk, kEpsZero><<<dim3(bx1, split), kTiledThreads, 0, st>>>(s, p, eps, part);
-    k_integrate_partial<kMethod><<<(n + 255) / 256, 256, 0, st>>>(s, p, part);
+    return best;
+}
+
+template <bool kQuirk, int kZero>
+static cudaError_t launch_direct_z(const DevSim &s, const StepParams &p, const DirectPlan &d, float4 *part,
+                                   int *arrived, float4 *out, cudaStream_t st) {
+    const dim3 grid((unsigned)((s.n + 32 * d.ki - 1) / (32 * d.ki)), (unsigned)d.slices);
+    const int threads = 32 * kDirectWarps;
+    if (d.ki == 4) k_direct<4, kQuirk, kZero><<<grid, threads, 0, st>>>(s, p, part, arrived, out);
+    else if (d.ki == 2) k_direct<2, kQuirk, kZero><<<grid, threads, 0, st>>>(s, p, part, arrived, out);
+    else k_direct<1, kQuirk, kZero><<<grid, threads, 0, st>>>(s, p, part, arrived, out);
     return cudaGetLastError();
 }
 
-template <int kMethod>
-static cudaError_t launch_direct_m(const DevSim &s, const StepParams &p, float eps, int tiled, int quirk,
-                                   int sm_count, cudaStream_t st, float4 *part) {
-    const bool ez = !(eps > 0.0f);
-    if (quirk) return launch_direct_t<kMethod, true, false>(s, p, eps, tiled, sm_count, st, part);
-    if (ez) return launch_direct_t<kMethod, false, true>(s, p, eps, tiled, sm_count, st, part);
-    return launch_direct_t<kMethod, false, false>(s, p, eps, tiled, sm_count, st, part);
-}
-
-// `p.eps` is the softening to use; s.part (N float4) holds the partial sums
-// of a split j range.
-cudaError_t launch_direct(const DevSim &s, const StepParams &p, int tiled, int quirk, int sm_count,
-                          cudaStream_t st) {
-    float4 *part = s.part;
-    switch (p.method) {
-    case 1: return launch_direct_m<1>(s, p, p.eps, tiled, quirk, sm_count, st, part);
-    case 2: return launch_direct_m<2>(s, p, p.eps, tiled, quirk, sm_count, st, part);
-    case 3: return launch_direct_m<3>(s, p, p.eps, tiled, quirk, sm_count, st, part);
-    default: return launch_direct_m<0>(s, p, p.eps, tiled, quirk, sm_count, st, part);
-    }
+// `p.eps` is the softening to use; s.part (direct_part_bodies float4) holds
+// the sums of the slices.
+cudaError_t launch_direct(const DevSim &s, const StepParams &p, const DirectPlan &plan, int *arrived, int tiled,
+                          int quirk, cudaStream_t st) {
+    if (quirk) return launch_direct_z<true, kZeroAdds>(s, p, plan, s.part, arrived, nullptr, st);
+    if (p.eps > 0.0f) return launch_direct_z<false, kZeroAdds>(s, p, plan, s.part, arrived, nullptr, st);
+    if (tiled) return launch_direct_z<false, kZeroSkips>(s, p, plan, s.part, arrived, nullptr, st);
+    return launch_direct_z<false, kZeroSkipsSelf>(s, p, plan, s.part, arrived, nullptr, st);
 }
 
 cudaError_t launch_copy_vertices(const float4 *body, int n, float4 *dst, cudaStream_t st) {
@@ -460,69 +242,14 @@ namespace nbgb {
 // or a frame loop where a cudaMalloc (which can synchronise the device and
 // take an allocator lock) is not allowed.  The caller passes the bodies and
 // the output; the one piece of scratch the split all-pairs sum needs -- the
-// partial accelerations of the j slices -- lives in a file-scope device
-// array of fixed size, together with a status word for the bounded waits.
-// Every GPU that loads this library holds that array (1 MiB + 80 B) until
-// the process exits.  All calls share it: calls that overlap on the GPU race.
+// partial accelerations of the body slices -- lives in a file-scope device
+// array of fixed size, together with the counters of the slices that are
+// done.  Every GPU that loads this library holds that array (1 MiB + 8 KiB)
+// until the process exits.  All calls share it: calls that overlap on the GPU race.
 // ===========================================================================
 constexpr int kNoAllocMaxBodies = 65536;  // = NB_NOALLOC_MAX_BODIES
 static __device__ __align__(256) float4 g_noalloc_part[kNoAllocMaxBodies];
-static __device__ __align__(256) Ctrl g_noalloc_ctrl;
-
-// The tiled all-pairs kernel above with the j range split over gridDim.y and
-// every slice adding its partial sums into `part`; no integrator.
-template <bool kEpsZero>
-__global__ void __launch_bounds__(kDirectThreads) k_noalloc_partial(const float4 *__restrict__ body, int n,
-                                                                     float eps2, float4 *part, Ctrl *ctrl) {
-    __shared__ __align__(128) float4 tile[2][kTile];
-    __shared__ __align__(8) uint64_t bar[2];
-    const int ntiles = (n + kTile - 1) / kTile;
-    const int per_split = (ntiles + gridDim.y - 1) / gridDim.y;
-    const int t0 = blockIdx.y * per_split;
-    const int t1 = min(ntiles, t0 + per_split);
-    const int i = blockIdx.x * kDirectThreads + threadIdx.x;
-    const float4 me = i < n ? body[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float ax = 0.0f, ay = 0.0f, az = 0.0f;
-    if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    auto issue = [&](int t, int stage) {
-        const int cnt = min(kTile, n - t * kTile);
-        const uint32_t bytes = (uint32_t)cnt * 16u;
-        mbar_expect_tx(&bar[stage], bytes);
-        bulk_g2s(&tile[stage][0], body + (size_t)t * kTile, bytes, &bar[stage]);
-    };
-    if (threadIdx.x == 0 && t0 < t1) issue(t0, 0);
-    bool ok = true;
-    for (int t = t0; t < t1; ++t) {
-        const int it = t - t0;
-        const int stage = it & 1;
-        if (threadIdx.x == 0 && t + 1 < t1) issue(t + 1, stage ^ 1);
-        if (!mbar_wait_bounded(&bar[stage], (uint32_t)((it >> 1) & 1), ctrl)) ok = false;
-        const int cnt = min(kTile, n - t * kTile);
-        for (int j = 0; j < cnt; ++j) pair<false, kEpsZero>(me, tile[stage][j], eps2, ax, ay, az);
-        if (!__syncthreads_and(ok)) {
-            if (threadIdx.x == 0 && t + 1 < t1)
-                mbar_wait_bounded(&bar[stage ^ 1], (uint32_t)(((it + 1) >> 1) & 1), ctrl);
-            ok = false;
-            break;
-        }
-    }
-    if (!ok || i >= n) return;
-    atomicAdd(&part[i].x, ax);
-    atomicAdd(&part[i].y, ay);
-    atomicAdd(&part[i].z, az);
-}
-
-__global__ void k_noalloc_finish(const float4 *__restrict__ part, int n, float G, float4 *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = part[i];
-    out[i] = make_float4(a.x * G, a.y * G, a.z * G, 0.0f);
-}
+static __device__ __align__(256) int g_noalloc_arrived[kNoAllocMaxBodies / 32];
 
 }  // namespace nbgb
 
@@ -542,19 +269,19 @@ namespace {
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mu;
 void *g_noalloc_part_ptr[kMaxDevices] = {};
-void *g_noalloc_ctrl_ptr[kMaxDevices] = {};
+void *g_noalloc_arrived_ptr[kMaxDevices] = {};
 
-bool noalloc_setup(int dev, float4 **part, nbgb::Ctrl **ctrl) {
+bool noalloc_setup(int dev, float4 **part, int **arrived) {
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_part_ptr[dev]) {
         void *p = nullptr, *c = nullptr;
         if (cudaGetSymbolAddress(&p, nbgb::g_noalloc_part) != cudaSuccess) return false;
-        if (cudaGetSymbolAddress(&c, nbgb::g_noalloc_ctrl) != cudaSuccess) return false;
+        if (cudaGetSymbolAddress(&c, nbgb::g_noalloc_arrived) != cudaSuccess) return false;
         g_noalloc_part_ptr[dev] = p;
-        g_noalloc_ctrl_ptr[dev] = c;
+        g_noalloc_arrived_ptr[dev] = c;
     }
     *part = static_cast<float4 *>(g_noalloc_part_ptr[dev]);
-    *ctrl = static_cast<nbgb::Ctrl *>(g_noalloc_ctrl_ptr[dev]);
+    *arrived = static_cast<int *>(g_noalloc_arrived_ptr[dev]);
     return true;
 }
 }  // namespace
@@ -568,30 +295,28 @@ extern "C" nb_status nb_direct_accel_noalloc(const float *d_body4, int32_t n, fl
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return NB_ERR_NO_DEVICE;
     float4 *part = nullptr;
-    Ctrl *ctrl = nullptr;
-    if (!noalloc_setup(dev, &part, &ctrl)) return NB_ERR_CUDA;
+    int *arrived = nullptr;
+    if (!noalloc_setup(dev, &part, &arrived)) return NB_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // the scratch keeps the previous call's contents: clear what must start at 0
-    if (cudaMemsetAsync(part, 0, sizeof(float4) * (size_t)n, st) != cudaSuccess) return NB_ERR_CUDA;
-    if (cudaMemsetAsync(ctrl, 0, sizeof(Ctrl), st) != cudaSuccess) return NB_ERR_CUDA;
     int sm_count = 0;
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    const int bx = (n + kDirectThreads - 1) / kDirectThreads;
-    const int ntiles = (n + kTile - 1) / kTile;
-    int split = (2 * sm_count + bx - 1) / bx;
-    if (split > ntiles) split = ntiles;
-    if (split < 1) split = 1;
-    const float eps2 = eps * eps;
-    const float4 *body = reinterpret_cast<const float4 *>(d_body4);
-    if (eps > 0.0f) k_noalloc_partial<false><<<dim3(bx, split), kDirectThreads, 0, st>>>(body, n, eps2, part, ctrl);
-    else k_noalloc_partial<true><<<dim3(bx, split), kDirectThreads, 0, st>>>(body, n, eps2, part, ctrl);
-    k_noalloc_finish<<<bx, kDirectThreads, 0, st>>>(part, n, G, reinterpret_cast<float4 *>(d_acc4));
-    if (cudaGetLastError() != cudaSuccess) return NB_ERR_CUDA;
-    // wait, then read the status of the bounded waits (no allocation: a
-    // stack variable receives it)
-    int status = 0;
-    if (cudaMemcpyAsync(&status, &ctrl->status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    DevSim s{};
+    s.n = n;
+    s.body_cur = reinterpret_cast<const float4 *>(d_body4);
+    StepParams p{};
+    p.eps = eps;
+    p.G = G;
+    float4 *out = reinterpret_cast<float4 *>(d_acc4);
+    // the caller may have the accelerations written over the bodies: then
+    // they go through the scratch, in one slice
+    const uintptr_t b0 = (uintptr_t)d_body4, a0 = (uintptr_t)d_acc4, bytes = sizeof(float4) * (size_t)n;
+    const bool overlap = a0 < b0 + bytes && b0 < a0 + bytes;
+    const DirectPlan plan = direct_plan(n, sm_count, overlap ? 1 : std::min(kDirectMaxSlices, kNoAllocMaxBodies / n));
+    if (overlap) out = part;
+    const cudaError_t e = eps > 0.0f ? launch_direct_z<false, kZeroAdds>(s, p, plan, part, arrived, out, st)
+                                     : launch_direct_z<false, kZeroSkips>(s, p, plan, part, arrived, out, st);
+    if (e != cudaSuccess) return NB_ERR_CUDA;
+    if (overlap && cudaMemcpyAsync(d_acc4, part, bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return NB_ERR_CUDA;
-    if (cudaStreamSynchronize(st) != cudaSuccess) return NB_ERR_CUDA;
-    return status ? (nb_status)status : NB_OK;
+    return cudaStreamSynchronize(st) == cudaSuccess ? NB_OK : NB_ERR_CUDA;
 }

@@ -69,7 +69,7 @@ struct DevSim {
     int *start;
     int *arrive;
     int *sorted;
-    float4 *part;    // N partial accelerations of a split direct sum
+    float4 *part;    // N partial accelerations per slice of a split direct sum
     float4 *cell_q;  // 2 per cell: {xx, yy, zz, xy}, {xz, yz, 0, 0} about the centre of mass
     float4 *wqa;     // (C+1)*8: quadrupole {xx, yy, zz, xy} of each packed child (0 for bodies)
     float2 *wqb;     // (C+1)*8: {xz, yz} of each packed child
@@ -248,8 +248,21 @@ cudaError_t launch_build(const DevSim &s, const TopTables &top, int tree_ref, in
 cudaError_t launch_summarize(const DevSim &s, int quadrupole, int sm_count, cudaStream_t st);
 cudaError_t launch_sort(const DevSim &s, int sm_count, cudaStream_t st);
 cudaError_t launch_force(const DevSim &s, const StepParams &p, int compensated, int sm_count, cudaStream_t st);
-cudaError_t launch_direct(const DevSim &s, const StepParams &p, int tiled, int quirk, int sm_count,
-                          cudaStream_t st);
+// How a direct sum is spread over the GPU: targets per lane and slices of the
+// bodies (k_direct.cu).
+constexpr int kDirectMaxSlices = 16;
+// slices a handle allows itself: their sums take at most 128 MiB
+inline int direct_slices_limit(int n) {
+    const int k = (1 << 23) / n;
+    return k < 1 ? 1 : (k < kDirectMaxSlices ? k : kDirectMaxSlices);
+}
+struct DirectPlan {
+    int ki, slices;
+};
+DirectPlan direct_plan(int n, int sm_count, int max_slices);
+// `arrived`: (n + 31) / 32 counters, zero between launches
+cudaError_t launch_direct(const DevSim &s, const StepParams &p, const DirectPlan &plan, int *arrived, int tiled,
+                          int quirk, cudaStream_t st);
 // Scratch of the collision update's grid form (k_collide.cu): bucket counts
 // and, behind them, the control words; bucket starts; each body's place in its
 // bucket (then the overflow list); the bodies in bucket order.  All null: the
@@ -297,6 +310,7 @@ cudaError_t launch_diagnostics(const float4 *body, const float4 *vel, int n, int
 inline int batch_chunk(int n, long long batch_tree_bodies) {
     return (n >= (1 << 19) || batch_tree_bodies >= (4LL << 20)) ? 4096 : 1024;
 }
+constexpr int kBatchDirectDefault = 3;  // the variant of a batch that is not tuned
 int batch_direct_variants();
 int batch_direct_block_bodies(int variant);
 // Optional second stream of a captured batched step: the small systems'

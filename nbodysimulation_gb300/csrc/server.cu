@@ -78,7 +78,7 @@ struct nb_server {
     nb_server_config cfg{};
     nb_job_fn fn = nullptr;
     void *user = nullptr;
-    int dev = 0, sm = 0, variant = 3;
+    int dev = 0, sm = 0, variant = kBatchDirectDefault;
     cudaStream_t compute = nullptr, upload = nullptr, out = nullptr, cap = nullptr;
     StepFork fork{};  // the captured round step's second branch (direct sums)
     Admission adm{0, 0};
@@ -533,7 +533,7 @@ nb_status nb_server_create(const nb_server_config *c, nb_job_fn fn, void *user, 
     s->fn = fn;
     s->user = user;
     s->dev = c->device;
-    s->variant = c->direct_variant >= 0 ? c->direct_variant : 3;
+    s->variant = c->direct_variant >= 0 ? c->direct_variant : kBatchDirectDefault;
     s->adm = Admission(c->hbm_budget_bytes, c->max_jobs);
     s->t0 = Clock::now();
     auto bad = [&](nb_status st) {
