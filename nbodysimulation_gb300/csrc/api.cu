@@ -48,8 +48,8 @@ struct nb_sim {
     float4 *wpm = nullptr, *cell_pm = nullptr;
     float4 *cell_q = nullptr, *wqa = nullptr;
     float2 *wqb = nullptr;
-    int *top = nullptr;  // top-level tables: counts, start entries (kTopRegions each), level L-1 entries
-    int top_levels = 0;
+    int *build_mem = nullptr;  // counters and tables of the build from sorted paths
+    BuildScratch build{};
     bool quad = false;
     DirectPlan plan{1, 1};    // direct sum: how it is spread over the GPU
     int *arrived = nullptr;   // and its slices' counters (behind part)
@@ -120,8 +120,8 @@ static DevSim dev_view(const nb_sim *s) {
 static void free_tree(nb_sim *s) {
     cudaFree(s->parent); cudaFree(s->child); cudaFree(s->wchild); cudaFree(s->wpm); cudaFree(s->cell_pm);
     cudaFree(s->count); cudaFree(s->start); cudaFree(s->arrive);
-    cudaFree(s->cell_q); cudaFree(s->wqa); cudaFree(s->wqb); cudaFree(s->top);
-    s->parent = s->child = s->wchild = s->count = s->start = s->arrive = s->top = nullptr;
+    cudaFree(s->cell_q); cudaFree(s->wqa); cudaFree(s->wqb); cudaFree(s->build_mem);
+    s->parent = s->child = s->wchild = s->count = s->start = s->arrive = s->build_mem = nullptr;
     s->wpm = s->cell_pm = s->cell_q = s->wqa = nullptr;
     s->wqb = nullptr;
 }
@@ -143,10 +143,12 @@ static nb_status alloc_tree(nb_sim *s, int cap) {
         NB_CUDA(s, dalloc(&s->wqa, cells * 8));
         NB_CUDA(s, dalloc(&s->wqb, cells * 8));
     }
-    s->top_levels = top_levels_for(s->n);
-    if (s->top_levels) {  // the counts start at zero; the build leaves them at zero
-        NB_CUDA(s, dalloc(&s->top, (size_t)2 * kTopRegions + kTopRegions / 8));
-        NB_CUDA(s, cudaMemset(s->top, 0, sizeof(int) * kTopRegions));
+    if (s->cfg.tree_semantics != NB_TREE_REFERENCE) {
+        // the paths and places lie in the transfer staging, which no step uses
+        const size_t ints = build_scratch_ints(s->n, s->sm_count);
+        NB_CUDA(s, dalloc(&s->build_mem, ints));
+        NB_CUDA(s, cudaMemset(s->build_mem, 0, sizeof(int) * ints));
+        s->build = build_scratch(s->n, s->sm_count, s->build_mem, s->part, s->stage3);
     }
     return NB_OK;
 }
@@ -467,21 +469,30 @@ static nb_status enqueue_step(nb_sim *s, float dt, int timed) {
     if (s->tree) {
         p.eps = c.epsilon;
         mark(0);
-        NB_CUDA(s, launch_reset(d, st));
-        NB_CUDA(s, launch_bbox(d, s->sm_count, st));
-        mark(1);
-        const TopTables top{s->top, s->top ? s->top + kTopRegions : nullptr, s->top ? s->top_levels : 0,
-                            s->top ? s->top + 2 * kTopRegions : nullptr};
-        int build_launches = 1;
-        NB_CUDA(s, launch_build(d, top, p.tree_ref, s->sm_count, st, &build_launches));
-        mark(2);
-        NB_CUDA(s, launch_summarize(d, p.quadrupole, s->sm_count, st));
-        mark(3);
-        NB_CUDA(s, launch_sort(d, s->sm_count, st));
+        if (p.tree_ref) {
+            NB_CUDA(s, launch_reset(d, st));
+            NB_CUDA(s, launch_bbox(d, s->sm_count, st));
+            mark(1);
+            NB_CUDA(s, launch_build(d, s->sm_count, st));
+            mark(2);
+            NB_CUDA(s, launch_summarize(d, p.quadrupole, s->sm_count, st));
+            mark(3);
+            NB_CUDA(s, launch_sort(d, s->sm_count, st));
+            s->launches += 5;
+        } else {  // the build sorts the bodies: no stage of its own
+            int build_launches = 0;
+            NB_CUDA(s, launch_tree_box(d, s->build, s->sm_count, st));
+            mark(1);
+            NB_CUDA(s, launch_tree_cells(d, s->build, s->sm_count, st, &build_launches));
+            mark(2);
+            NB_CUDA(s, launch_tree_sums(d, s->build, p.quadrupole, s->sm_count, st));
+            mark(3);
+            s->launches += 3 + build_launches;
+        }
         mark(4);
         NB_CUDA(s, launch_force(d, p, c.precision == NB_PRECISION_COMPENSATED, s->sm_count, st));
         mark(5);
-        s->launches += 5 + build_launches;
+        s->launches += 1;
         for (int k = kStBboxReset; k <= kStForce; ++k) s->stage_ran[k] = true;
     } else {
         const bool quirk = c.force_law == NB_FORCE_REFERENCE_QUIRK;

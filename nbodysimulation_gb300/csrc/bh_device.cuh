@@ -1,5 +1,5 @@
 // bh_device.cuh -- the per-item work of the Barnes-Hut stages as device
-// functions, shared by the single-system kernels (k_tree.cu, k_force.cu)
+// functions, shared by the single-system kernels (k_build.cu, k_tree.cu)
 // and the batched kernels that walk a table of systems (k_batch.cu).
 //
 // Reference stages: build_tree (kernels/build_tree.cl, build_tree.hcl),
@@ -239,13 +239,11 @@ __device__ __forceinline__ void top_count_range(const DevSim &s, const TopTables
 // One block: region counts of levels L-1..1 from the level-L counts, then
 // the cells of levels 1..L top down (each level's cells numbered below the
 // previous level's), then the start entry of every level-L region.  Clears
-// the level-L counts for the next step in every case.  With deep_out, the
-// block stops after level L-1 and leaves that level's entries in deep_out
-// (8^(L-1) ints) and the counts in place for top_leaf_cells.  Every thread of
+// the level-L counts for the next step in every case.   Every thread of
 // the block calls it; blockDim.x is a power of two with 8^L <= 32 *
 // blockDim.x, so a thread takes at most 32 regions of a level and a level has
 // at most kTopRegions / 32 (round, warp) pairs.
-__device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables &t, int *deep_out = nullptr) {
+__device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables &t) {
     __shared__ int cnt_sh[kTopInner];   // body counts, regions of levels 1..L-1
     __shared__ int deep_sh[kTopInner];  // (level << 26) | deepest existing cell of the region's path
     __shared__ int rank_sh[kTopRegions / 32];  // per (round, warp): new cells before it
@@ -281,8 +279,7 @@ __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables
         }
         const int lane = tid & 31, w = tid >> 5, nw = nt >> 5;
         const unsigned below = (1u << lane) - 1u;
-        const int last = deep_out ? L - 1 : L;
-        for (int l = 1; l <= last; ++l) {
+        for (int l = 1; l <= L; ++l) {
             // region r = j * nt + tid in round j; a level's cells are numbered
             // bottom - 1 - rank with rank in (round, warp, lane) order, so a
             // warp's new cells are consecutive and its writes coalesce
@@ -337,7 +334,6 @@ __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables
                 }
                 if (l < L) deep_sh[top_offset(l) + r] = e;
                 else t.start[r] = e;
-                if (deep_out && l == last) deep_out[r] = e;
             }
             __syncthreads();
             if (tid == 0) s_bottom = bottom - total;
@@ -345,49 +341,8 @@ __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables
         }
     }
     __syncthreads();
-    if (!deep_out)
-        for (int r = tid; r < n_last; r += nt) t.count[r] = 0;
+    for (int r = tid; r < n_last; r += nt) t.count[r] = 0;
     if (tid == 0 && !s_skip) ctrl->bottom = s_bottom;
-}
-
-// The cells of level L after top_cells_block(..., deep): one region per
-// thread, warp-aggregated numbering from the cell counter (below every cell
-// of the upper levels), the start entries, and the counts cleared.
-__device__ __forceinline__ void top_leaf_cells(const DevSim &s, const TopTables &t, const int *deep, int r) {
-    Ctrl *ctrl = s.ctrl;
-    const int n = s.n, nr = 1 << (3 * t.levels);
-    const bool skip = read_status(ctrl) != 0;  // grid-uniform: only earlier kernels set it
-    const int cnt = r < nr ? t.count[r] : 0;
-    const bool make = !skip && cnt >= 2;
-    const unsigned am = __activemask();
-    const unsigned b = __ballot_sync(am, make);
-    const int leader = __ffs(am) - 1, lane = threadIdx.x & 31;
-    int base = 0;
-    if (lane == leader && b) base = atomicSub(&ctrl->bottom, __popc(b));
-    base = __shfl_sync(am, base, leader);
-    if (r >= nr) return;
-    t.count[r] = 0;
-    if (skip) return;
-    const int pe = deep[r >> 3];
-    int e = pe;
-    if (make) {
-        const int cell = base - 1 - __popc(b & ((1u << lane) - 1u));
-        if (cell < n) {  // more top cells than the capacity
-            set_status(ctrl, kStCellOverflow, t.levels);
-            return;
-        }
-        const int c = cell - n;
-        int4 *row = reinterpret_cast<int4 *>(&s.child[c * 8]);
-        row[0] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
-        row[1] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
-        const int parent = pe & ((1 << 26) - 1);
-        s.parent[c] = parent;
-        s.arrive[c] = 0;
-        s.start[c] = -1;
-        s.child[(parent - n) * 8 + (r & 7)] = cell;
-        e = (t.levels << 26) | cell;
-    }
-    t.start[r] = e;
 }
 
 // Insertion of body i from the deepest existing top cell of its level-L path.
@@ -434,18 +389,28 @@ __device__ __forceinline__ void load_children(const int *child, int c, int chs[8
 // Fences: release before every counter update, acquire after the update that
 // completes a cell; child-cell data written in this kernel is read through L2.
 // ---------------------------------------------------------------------------
+// e = Q_child + m (3 d d^T - |d|^2 I), d = x_child - (X, Y, Z)
+__device__ __forceinline__ void quadrupole_term(const float4 pm, float X, float Y, float Z, const float4 oa, float oxz,
+                                                float oyz, float &e0, float &e1, float &e2, float &e3, float &e4,
+                                                float &e5) {
+    const float m = pm.w;
+    const float dx = __fsub_rn(pm.x, X), dy = __fsub_rn(pm.y, Y), dz = __fsub_rn(pm.z, Z);
+    const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+    const float tx = __fmul_rn(3.0f, dx), ty = __fmul_rn(3.0f, dy);
+    e0 = __fmaf_rn(m, __fmaf_rn(tx, dx, -r2), oa.x);
+    e1 = __fmaf_rn(m, __fmaf_rn(ty, dy, -r2), oa.y);
+    e2 = __fmaf_rn(m, __fmaf_rn(__fmul_rn(3.0f, dz), dz, -r2), oa.z);
+    e3 = __fmaf_rn(m, __fmul_rn(tx, dy), oa.w);
+    e4 = __fmaf_rn(m, __fmul_rn(tx, dz), oxz);
+    e5 = __fmaf_rn(m, __fmul_rn(ty, dz), oyz);
+}
+
+// Completes cell `node`, whose children (chs, octant slots) are complete, then
+// arrives at its parent, and so on as long as it is the last to arrive.
 template <bool kQuad>
-__device__ __forceinline__ void summarize_from(const DevSim &s, int k) {
+__device__ __forceinline__ void climb(const DevSim &s, int node, int (&chs)[8]) {
     const int n = s.n, root = n + s.cap;
-    int node = k;
-    int chs[8], nch, nbody;
-    load_children(s.child, node - n, chs, nch, nbody, n);
-    if (nbody == 0) return;  // completed by its child cells
-    if (nbody != nch) {
-        const int old = atomicAdd(&s.arrive[node - n], nbody);
-        if (old + nbody != nch) return;
-        __threadfence();
-    }
+    int nch, nbody;
     while (true) {
         const int c = node - n;
         float M = 0.0f, cx = 0.0f, cy = 0.0f, cz = 0.0f;
@@ -527,16 +492,14 @@ __device__ __forceinline__ void summarize_from(const DevSim &s, int k) {
                 }
                 s.wqa[c * 8 + j] = oa;
                 s.wqb[c * 8 + j] = make_float2(ob.x, ob.y);
-                const float m = pm.w;
-                const float dx = __fsub_rn(pm.x, X), dy = __fsub_rn(pm.y, Y), dz = __fsub_rn(pm.z, Z);
-                const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-                const float tx = __fmul_rn(3.0f, dx), ty = __fmul_rn(3.0f, dy);
-                q0 = __fadd_rn(q0, __fmaf_rn(m, __fmaf_rn(tx, dx, -r2), oa.x));
-                q1 = __fadd_rn(q1, __fmaf_rn(m, __fmaf_rn(ty, dy, -r2), oa.y));
-                q2 = __fadd_rn(q2, __fmaf_rn(m, __fmaf_rn(__fmul_rn(3.0f, dz), dz, -r2), oa.z));
-                q3 = __fadd_rn(q3, __fmaf_rn(m, __fmul_rn(tx, dy), oa.w));
-                q4 = __fadd_rn(q4, __fmaf_rn(m, __fmul_rn(tx, dz), ob.x));
-                q5 = __fadd_rn(q5, __fmaf_rn(m, __fmul_rn(ty, dz), ob.y));
+                float e0, e1, e2, e3, e4, e5;
+                quadrupole_term(pm, X, Y, Z, oa, ob.x, ob.y, e0, e1, e2, e3, e4, e5);
+                q0 = __fadd_rn(q0, e0);
+                q1 = __fadd_rn(q1, e1);
+                q2 = __fadd_rn(q2, e2);
+                q3 = __fadd_rn(q3, e3);
+                q4 = __fadd_rn(q4, e4);
+                q5 = __fadd_rn(q5, e5);
             }
             s.cell_q[2 * c] = make_float4(q0, q1, q2, q3);
             s.cell_q[2 * c + 1] = make_float4(q4, q5, 0.0f, 0.0f);
@@ -550,6 +513,20 @@ __device__ __forceinline__ void summarize_from(const DevSim &s, int k) {
         __threadfence();
         node = p;
     }
+}
+
+template <bool kQuad>
+__device__ __forceinline__ void summarize_from(const DevSim &s, int k) {
+    const int n = s.n;
+    int chs[8], nch, nbody;
+    load_children(s.child, k - n, chs, nch, nbody, n);
+    if (nbody == 0) return;  // completed by its child cells
+    if (nbody != nch) {
+        const int old = atomicAdd(&s.arrive[k - n], nbody);
+        if (old + nbody != nch) return;
+        __threadfence();
+    }
+    climb<kQuad>(s, k, chs);
 }
 
 // ---------------------------------------------------------------------------

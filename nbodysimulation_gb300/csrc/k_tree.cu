@@ -1,5 +1,6 @@
 // k_tree.cu -- bounding box, octree build, centre-of-mass summarisation and
-// in-order sort of the Barnes-Hut step.
+// in-order sort with the reference's tree semantics (its boxes and super-root;
+// the cubic-root tree is k_build.cu's).
 //
 // Reference stages: boundary_reduce (kernels/boundary_reduce.cl), init
 // (kernels/init.cl), build_tree (kernels/build_tree.cl, build_tree.hcl),
@@ -83,65 +84,17 @@ __global__ void __launch_bounds__(256) k_bbox(const float4 *__restrict__ b, int 
 // ---------------------------------------------------------------------------
 // build: one body per thread, grid-stride (insert_body, bh_device.cuh).
 // ---------------------------------------------------------------------------
-template <class Geo, bool kRef>
 __global__ void __launch_bounds__(256) k_build(DevSim s) {
     Ctrl *ctrl = s.ctrl;
     if (read_status(ctrl)) return;
     float box[6];
     load_box(ctrl, box);
-    const Geo root_g = Geo::root(box);
+    const RefBox root_g = RefBox::root(box);
     int local_max = 0;
     const long long cap = tree_spin_cap(ctrl);
     const int stride = gridDim.x * blockDim.x;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += stride) {
-        const int depth = insert_body<Geo, kRef>(s, root_g, i, cap);
-        if (depth < 0) return;
-        local_max = max(local_max, depth);
-    }
-    const unsigned am = __activemask();
-    const int wmax = __reduce_max_sync(am, local_max);
-    if ((threadIdx.x & 31) == __ffs(am) - 1) atomicMax(&ctrl->max_depth, wmax);
-}
-
-// ---------------------------------------------------------------------------
-// top levels (cubic-root tree): count, cells, then the build from them.
-// ---------------------------------------------------------------------------
-// Counts per block in shared memory (8^L bins, dynamic), then one global
-// atomic per non-empty bin: regions of a dense centre hold tens of thousands
-// of bodies, which one global counter each would serialise.
-constexpr int kTopCountThreads = 1024;
-__global__ void __launch_bounds__(kTopCountThreads) k_top_count(DevSim s, TopTables t) {
-    extern __shared__ int bins[];
-    Ctrl *ctrl = s.ctrl;
-    if (read_status(ctrl)) return;  // block-uniform, before any barrier
-    float box[6];
-    load_box(ctrl, box);
-    top_count_range(s, t, GeoCube::root(box), blockIdx.x * blockDim.x, s.n, gridDim.x * blockDim.x, bins);
-}
-
-constexpr int kTopCellsThreads = 1024;
-static_assert((1 << (3 * kTopMaxLevels)) <= 32 * kTopCellsThreads, "top_cells_block: at most 32 regions a thread");
-// levels 1..L-1 in one block, then level L (most of the cells) over a grid
-__global__ void __launch_bounds__(kTopCellsThreads) k_top_cells(DevSim s, TopTables t) {
-    top_cells_block(s, t, t.deep);
-}
-
-__global__ void __launch_bounds__(256) k_top_leaf(DevSim s, TopTables t) {
-    top_leaf_cells(s, t, t.deep, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-// build from the top levels, one body per thread, grid-stride
-__global__ void __launch_bounds__(256) k_build_top(DevSim s, TopTables t) {
-    Ctrl *ctrl = s.ctrl;
-    if (read_status(ctrl)) return;
-    float box[6];
-    load_box(ctrl, box);
-    const GeoCube root_g = GeoCube::root(box);
-    int local_max = 0;
-    const long long cap = tree_spin_cap(ctrl);
-    const int stride = gridDim.x * blockDim.x;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += stride) {
-        const int depth = insert_from_top(s, t, root_g, i, cap);
+        const int depth = insert_body<RefBox, true>(s, root_g, i, cap);
         if (depth < 0) return;
         local_max = max(local_max, depth);
     }
@@ -204,38 +157,15 @@ cudaError_t launch_bbox(const DevSim &s, int sm_count, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_build(const DevSim &s, const TopTables &top, int tree_ref, int sm_count, cudaStream_t st,
-                         int *launches) {
+cudaError_t launch_build(const DevSim &s, int sm_count, cudaStream_t st) {
     const int need = (s.n + 255) / 256;
-    if (!tree_ref && top.levels >= 2 && top.levels <= kTopMaxLevels) {
-        const size_t bins_bytes = sizeof(int) << (3 * top.levels);
-        if (bins_bytes > 48 * 1024) {  // the 8^5-bin table needs the opt-in shared memory size (current device)
-            const cudaError_t e = cudaFuncSetAttribute(k_top_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)bins_bytes);
-            if (e != cudaSuccess) return e;
-        }
-        const int cblocks = std::max(1, std::min(sm_count, (s.n + kTopCountThreads - 1) / kTopCountThreads));
-        k_top_count<<<cblocks, kTopCountThreads, bins_bytes, st>>>(s, top);
-        k_top_cells<<<1, kTopCellsThreads, 0, st>>>(s, top);  // all levels in the block when top.deep is null
-        if (top.deep) k_top_leaf<<<((1 << (3 * top.levels)) + 255) / 256, 256, 0, st>>>(s, top);
-        // two blocks per SM, as for the build from the root (262k-body ball:
-        // 0.12 ms against 0.14 ms on the whole co-resident grid; 4M: equal)
-        int blocks = std::min(resident_blocks((const void *)k_build_top, 256, sm_count), 2 * sm_count);
-        if (blocks > need) blocks = need > 0 ? need : 1;
-        k_build_top<<<blocks, 256, 0, st>>>(s, top);
-        *launches = top.deep ? 4 : 3;
-        return cudaGetLastError();
-    }
-    *launches = 1;
-    const void *fn = tree_ref ? (const void *)k_build<RefBox, true> : (const void *)k_build<GeoCube, false>;
     // two blocks per SM: threads that start at the root together contend for
     // its first cells, and fewer of them insert faster (measured build time
     // with 1 / 2 / 4 / 8 blocks per SM: 262k-body ball 0.20 / 0.20 / 0.30 /
     // 0.32 ms, 1M 0.60 / 0.41 / 0.49 / 0.54 ms, 4M 2.25 / 1.26 / 1.24 / 1.32 ms)
-    int blocks = std::min(resident_blocks(fn, 256, sm_count), 2 * sm_count);
+    int blocks = std::min(resident_blocks((const void *)k_build, 256, sm_count), 2 * sm_count);
     if (blocks > need) blocks = need > 0 ? need : 1;
-    if (tree_ref) k_build<RefBox, true><<<blocks, 256, 0, st>>>(s);
-    else k_build<GeoCube, false><<<blocks, 256, 0, st>>>(s);
+    k_build<<<blocks, 256, 0, st>>>(s);
     return cudaGetLastError();
 }
 

@@ -44,7 +44,7 @@ struct Ctrl {
     int kdk_primed;        // batched systems: a KDK half-kick has happened
     int budget;            // batched systems: steps left (< 0 unlimited, 0 inert)
     int spin_cap;          // > 0: iteration cap of the tree stages' waits (a test hook); 0: kSpinCap
-    int pad0[1];
+    int insert;            // this step's tree is built by insertions (k_build.cu)
     // cleared by the host once per nb_step call (everything from here on)
     int status;
     int status_info;
@@ -161,7 +161,6 @@ struct TopTables {
     int *count;
     int *start;
     int levels;
-    int *deep;  // 8^(levels-1) entries of level levels-1 when the last level is built by a grid (else null)
 };
 constexpr int kTopMaxLevels = 5;                  // 8^5 = 32768 regions
 constexpr int kTopRegions = 1 << (3 * kTopMaxLevels);
@@ -233,18 +232,51 @@ __device__ __forceinline__ int system_parity(const SysDesc &d) { return ld_volat
 
 __device__ __forceinline__ DevSim system_view(const SysDesc &d) { return system_view_par(d, system_parity(d)); }
 
+// Scratch of the build from sorted paths (k_build.cu).
+constexpr int kScanBlocks = 256;
+enum { kBuildBoxes = 0, kBuildBarrier = 1, kBuildTop = 2, kBuildPairs = 4, kBuildCtl = 8 };  // words of ctl
+struct BuildScratch {
+    int levels;        // levels of the regions; 0: all bodies are ranked together
+    int *ctl;          // counters (zero before the first step)
+    int *total;        // k_scan: blocks' totals + 1 (kScanBlocks)
+    int *count;        // bodies per region, zero between steps
+    int *start;        // first place of every region, and n
+    int *top;          // cells that reach over a tile's edge
+    unsigned *box;     // blocks' bounding boxes
+    unsigned long long *path, *placed;  // paths by body, then sorted; and by region
+    int *rank, *who, *base;             // place in the region; body; number of the first cell that starts here
+};
+// Up to this many bodies every path is compared with every other, which saves
+// two launches; beyond, only with those of its region (6,007: all 18 us,
+// regions with the launches 10).
+constexpr int kRankAll = 2048;
+inline int build_levels(int n) {  // between a quarter and two bodies a region, up to 8^8 regions
+    if (n <= kRankAll) return 0;
+    int l = 0;
+    while (l < 8 && (8LL << (3 * l)) <= 4LL * n) ++l;
+    return l;
+}
+// a tile of 256 bodies starts at most one such cell a level; and the root
+inline size_t build_top_cells(int n) { return ((size_t)(n + 255) / 256 * 21 + 1 + 3) / 4 * 4; }
+size_t build_scratch_ints(int n, int sm_count);
+// mem: build_scratch_ints ints, zeroed; keys16 / ints12: 16 n and 12 n bytes
+// that the step may overwrite
+BuildScratch build_scratch(int n, int sm_count, int *mem, void *keys16, void *ints12);
+// bbox; paths, sort and cells (*launches kernels); sums (two kernels)
+cudaError_t launch_tree_box(const DevSim &s, const BuildScratch &b, int sm_count, cudaStream_t st);
+cudaError_t launch_tree_cells(const DevSim &s, const BuildScratch &b, int sm_count, cudaStream_t st, int *launches);
+cudaError_t launch_tree_sums(const DevSim &s, const BuildScratch &b, int quadrupole, int sm_count, cudaStream_t st);
+
 // Launch helpers implemented in the kernel translation units.
 struct LaunchShape {
     int blocks;
     int threads;
 };
 
+// the reference's tree semantics (k_tree.cu): insertions from the root
 cudaError_t launch_reset(const DevSim &s, cudaStream_t st);
 cudaError_t launch_bbox(const DevSim &s, int sm_count, cudaStream_t st);
-// Launches the build (the top-level count and cells first when top.levels >
-// 0 and the tree is the cubic-root one); *launches gets the kernel count.
-cudaError_t launch_build(const DevSim &s, const TopTables &top, int tree_ref, int sm_count, cudaStream_t st,
-                         int *launches);
+cudaError_t launch_build(const DevSim &s, int sm_count, cudaStream_t st);
 cudaError_t launch_summarize(const DevSim &s, int quadrupole, int sm_count, cudaStream_t st);
 cudaError_t launch_sort(const DevSim &s, int sm_count, cudaStream_t st);
 cudaError_t launch_force(const DevSim &s, const StepParams &p, int compensated, int sm_count, cudaStream_t st);
