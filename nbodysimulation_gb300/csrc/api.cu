@@ -56,8 +56,8 @@ struct nb_sim {
     int *grid = nullptr;  // collision update: counts, control words, starts, ranks
     Ctrl *ctrl = nullptr;
     Ctrl *h_ctrl = nullptr;       // pinned mirror for status read-back
-    float *stage3 = nullptr;      // device staging, 3N floats
-    float *stage1 = nullptr;      // device staging, N floats
+    float *stage3 = nullptr;      // device staging, 3N floats (in part)
+    float *stage1 = nullptr;      // device staging, N floats (in part)
     bool have_state = false;
     bool kdk_primed = false;
     bool profiling = false;
@@ -162,6 +162,28 @@ static int default_capacity(int n, int sm_count) {
     return (int)c;
 }
 
+// Host arrays that kernels read and write in place, without a staging copy: one
+// pass over the host link at full width.  Page-locked ones (nb_host_alloc,
+// cudaMallocHost, cudaHostRegister) allocated or registered while `dev` was
+// current; on a host whose page tables the device shares, every other one too.
+// There a kernel costs what one copy does (9 us, 30 us at 4 MB) and replaces
+// one copy per array, and fills pages that the host never touched three times
+// as fast (4 MB 0.9 against 2.8 ms).
+void *nbgb::host_device_view(const void *p, int dev) {
+    if (!p) return nullptr;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (a.type == cudaMemoryTypeHost) return a.device == dev ? a.devicePointer : nullptr;
+    if (a.type != cudaMemoryTypeUnregistered) return nullptr;
+    int shared = 0;
+    if (cudaDeviceGetAttribute(&shared, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) != cudaSuccess || !shared)
+        return nullptr;
+    return const_cast<void *>(p);
+}
+
 extern "C" {
 
 int32_t nb_abi_version(void) { return NBGB_ABI_VERSION; }
@@ -239,17 +261,22 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     const size_t n = (size_t)s->n;
     s->tree = cfg->algo_config == NB_BARNES_HUT;
     if (!s->tree) s->plan = direct_plan(s->n, s->sm_count, direct_slices_limit(s->n));
+    const size_t part = n * (size_t)std::max(2, s->plan.slices);
     bool ok = dalloc(&s->body[0], n) == cudaSuccess && dalloc(&s->body[1], n) == cudaSuccess &&
               dalloc(&s->vel, n) == cudaSuccess && dalloc(&s->acc, n) == cudaSuccess &&
-              dalloc(&s->part, n * s->plan.slices + (s->tree ? 0 : (n + 127) / 128)) == cudaSuccess && dalloc(&s->stage3, 3 * n) == cudaSuccess &&
-              dalloc(&s->stage1, n) == cudaSuccess && dalloc(&s->ctrl, 1) == cudaSuccess;
+              dalloc(&s->part, part + (s->tree ? 0 : (n + 127) / 128)) == cudaSuccess &&
+              dalloc(&s->ctrl, 1) == cudaSuccess;
     if (!ok) return cleanup(NB_ERR_OUT_OF_MEMORY);
+    // the transfer staging lies behind the first n of the sums: no step runs
+    // beside a transfer
+    s->stage3 = reinterpret_cast<float *>(s->part + n);
+    s->stage1 = s->stage3 + 3 * n;
     if (cudaMallocHost((void **)&s->h_ctrl, sizeof(Ctrl)) != cudaSuccess) return cleanup(NB_ERR_OUT_OF_MEMORY);
     cudaMemset(s->ctrl, 0, sizeof(Ctrl));
     cudaMemset(s->vel, 0, sizeof(float4) * n);
     cudaMemset(s->acc, 0, sizeof(float4) * n);
     if (!s->tree) {  // the counters lie behind the slices' sums
-        s->arrived = reinterpret_cast<int *>(s->part + n * s->plan.slices);
+        s->arrived = reinterpret_cast<int *>(s->part + part);
         cudaMemset(s->arrived, 0, sizeof(int) * ((n + 31) / 32));
     }
     s->quad = cfg->multipole == NB_MULTIPOLE_QUADRUPOLE;
@@ -275,7 +302,7 @@ nb_status nb_destroy(nb_sim *s) {
     cudaSetDevice(s->dev);
     if (s->stream) cudaStreamSynchronize(s->stream);
     cudaFree(s->body[0]); cudaFree(s->body[1]); cudaFree(s->vel); cudaFree(s->acc); cudaFree(s->part);
-    cudaFree(s->stage3); cudaFree(s->stage1); cudaFree(s->ctrl); cudaFree(s->sorted); cudaFree(s->grid);
+    cudaFree(s->ctrl); cudaFree(s->sorted); cudaFree(s->grid);
     free_tree(s);
     if (s->h_ctrl) cudaFreeHost(s->h_ctrl);
     for (auto &e : s->ev)
@@ -293,22 +320,6 @@ nb_status nb_get_config(const nb_sim *s, nb_config *out) {
     return NB_OK;
 }
 
-// The device address of a host array the device can read and write
-// directly (page-locked: nb_host_alloc, cudaMallocHost, cudaHostRegister),
-// else null.  Such arrays are packed and unpacked by the kernels in place,
-// without a staging copy: one pass over the host link at full width.
-static void *host_device_view(const void *p, int dev) {
-    if (!p) return nullptr;
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    // page-locked for this handle's device (allocated or registered while it
-    // was current); other arrays take the staging copy
-    return a.type == cudaMemoryTypeHost && a.device == dev ? a.devicePointer : nullptr;
-}
-
 nb_status nb_set_state(nb_sim *s, const float *pos3, const float *vel3, const float *mass, int32_t n) {
     if (!s || !pos3 || !mass) return fail(s, NB_ERR_INVALID_ARGUMENT, "nb_set_state: pos3 and mass are required");
     if (n != s->n) return fail(s, NB_ERR_INVALID_ARGUMENT, "nb_set_state: n differs from num_of_bodies");
@@ -318,7 +329,7 @@ nb_status nb_set_state(nb_sim *s, const float *pos3, const float *vel3, const fl
         const float *dp = static_cast<const float *>(host_device_view(pos3, s->dev));
         const float *dm = static_cast<const float *>(host_device_view(mass, s->dev));
         const float *dv = static_cast<const float *>(host_device_view(vel3, s->dev));
-        if (dp && dm && (!vel3 || dv)) {  // page-locked: the kernel reads the host arrays
+        if (dp && dm && (!vel3 || dv)) {  // the kernel reads the host arrays
             NB_CUDA(s, launch_pack(dp, dm, dv, s->body[s->cur], s->vel, s->acc, n, s->stream));
             s->launches += 1;
             NB_CUDA(s, cudaStreamSynchronize(s->stream));
@@ -362,49 +373,35 @@ nb_status nb_get_state(nb_sim *s, float *pos3, float *vel3, float *acc3, float *
     if (!s->have_state) return fail(s, NB_ERR_STATE, "nb_get_state before nb_set_state");
     cudaSetDevice(s->dev);
     const size_t nn = (size_t)s->n;
-    float *dv = reinterpret_cast<float *>(s->part);
-    float *da = nullptr;  // acceleration staged behind the positions when asked
-    std::vector<float> tmp;
-    if ((pos3 || vel3) && !acc3 && !mass) {
-        float *hp = static_cast<float *>(host_device_view(pos3, s->dev));
-        float *hv = static_cast<float *>(host_device_view(vel3, s->dev));
-        if ((!pos3 || hp) && (!vel3 || hv)) {  // page-locked: the kernel writes the host arrays
-            NB_CUDA(s, launch_unpack(s->body[s->cur], s->vel, s->acc, hp, hv, nullptr, s->n, s->stream));
-            s->launches += 1;
-            NB_CUDA(s, cudaStreamSynchronize(s->stream));
-            return NB_OK;
-        }
+    float *host[4] = {pos3, vel3, acc3, mass}, *dev[4];
+    bool direct = pos3 || vel3 || acc3 || mass;
+    for (int k = 0; k < 4; ++k) {
+        dev[k] = static_cast<float *>(host_device_view(host[k], s->dev));
+        direct = direct && (!host[k] || dev[k]);
     }
-    if (pos3 || vel3) {
-        NB_CUDA(s, launch_unpack(s->body[s->cur], s->vel, s->acc, pos3 ? s->stage3 : nullptr, vel3 ? dv : nullptr,
-                                 nullptr, s->n, s->stream));
+    if (direct) {  // the kernel writes the host arrays
+        NB_CUDA(s, launch_unpack(s->body[s->cur], s->vel, s->acc, dev[0], dev[1], dev[2], dev[3], s->n, s->stream));
         s->launches += 1;
-        if (pos3) NB_CUDA(s, cudaMemcpyAsync(pos3, s->stage3, 12 * nn, cudaMemcpyDeviceToHost, s->stream));
-        if (vel3) NB_CUDA(s, cudaMemcpyAsync(vel3, dv, 12 * nn, cudaMemcpyDeviceToHost, s->stream));
-    }
-    if (acc3 || mass) {
         NB_CUDA(s, cudaStreamSynchronize(s->stream));
-        if (acc3) {
-            da = s->stage3;
-            NB_CUDA(s, launch_unpack(nullptr, nullptr, s->acc, nullptr, nullptr, da, s->n, s->stream));
-            s->launches += 1;
-            NB_CUDA(s, cudaMemcpyAsync(acc3, da, 12 * nn, cudaMemcpyDeviceToHost, s->stream));
-        }
-        if (mass) {
-            tmp.resize(4 * nn);
-            NB_CUDA(s, cudaMemcpyAsync(tmp.data(), s->body[s->cur], 16 * nn, cudaMemcpyDeviceToHost, s->stream));
-        }
+        return NB_OK;
+    }
+    // through the staging, one array after the other
+    for (int k = 0; k < 4; ++k) {
+        if (!host[k]) continue;
+        float *st = s->stage3;
+        NB_CUDA(s, launch_unpack(s->body[s->cur], s->vel, s->acc, k == 0 ? st : nullptr, k == 1 ? st : nullptr,
+                                 k == 2 ? st : nullptr, k == 3 ? st : nullptr, s->n, s->stream));
+        s->launches += 1;
+        NB_CUDA(s, cudaMemcpyAsync(host[k], st, (k == 3 ? 4 : 12) * nn, cudaMemcpyDeviceToHost, s->stream));
     }
     NB_CUDA(s, cudaStreamSynchronize(s->stream));
-    if (mass)
-        for (size_t i = 0; i < nn; ++i) mass[i] = tmp[4 * i + 3];
     return NB_OK;
 }
 
 nb_status nb_get_state_device(nb_sim *s, float *d_pos3, float *d_vel3) {
     if (!s) return NB_ERR_INVALID_ARGUMENT;
     cudaSetDevice(s->dev);
-    NB_CUDA(s, launch_unpack(s->body[s->cur], s->vel, s->acc, d_pos3, d_vel3, nullptr, s->n, s->stream));
+    NB_CUDA(s, launch_unpack(s->body[s->cur], s->vel, s->acc, d_pos3, d_vel3, nullptr, nullptr, s->n, s->stream));
     s->launches += 1;
     NB_CUDA(s, cudaStreamSynchronize(s->stream));
     return NB_OK;
@@ -651,7 +648,7 @@ nb_status nb_copy_vertices(nb_sim *s, float *dst4, int32_t dst_is_device) {
         if (!aligned) return fail(s, NB_ERR_INVALID_ARGUMENT, "nb_copy_vertices: a device dst must be 16-byte aligned");
         NB_CUDA(s, launch_copy_vertices(s->body[s->cur], s->n, reinterpret_cast<float4 *>(dst4), s->stream));
         s->launches += 1;
-    } else if (float *hd = aligned ? static_cast<float *>(host_device_view(dst4, s->dev)) : nullptr) {  // page-locked host
+    } else if (float *hd = aligned ? static_cast<float *>(host_device_view(dst4, s->dev)) : nullptr) {  // host, in place
         NB_CUDA(s, launch_copy_vertices(s->body[s->cur], s->n, reinterpret_cast<float4 *>(hd), s->stream));
         s->launches += 1;
     } else {

@@ -32,6 +32,7 @@ struct nb_batch {
     char *arena = nullptr;
     Ctrl *d_ctrl = nullptr;     // one Ctrl per system, contiguous
     Ctrl *h_ctrl = nullptr;     // pinned mirror
+    bool ctrls_fresh = false;   // no step since it was read
     std::vector<SysDesc> h_sys;
     SysDesc *d_sys = nullptr;
     int *d_pref = nullptr;      // prefix tables of nsys + 1 (batch_prefix_device_ints; the last written on the device)
@@ -257,31 +258,41 @@ nb_status nb_batch_destroy(nb_batch *b) {
 }
 
 static nb_status read_ctrls(nb_batch *b) {
+    b->ctrls_fresh = false;
     B_CUDA(b, cudaMemcpyAsync(b->h_ctrl, b->d_ctrl, sizeof(Ctrl) * b->nsys, cudaMemcpyDeviceToHost, b->st));
     B_CUDA(b, cudaStreamSynchronize(b->st));
+    b->ctrls_fresh = true;
     return NB_OK;
 }
+
+// the systems' buffer parities, which only steps change; a step ends with
+// read_ctrls
+static nb_status fresh_ctrls(nb_batch *b) { return b->ctrls_fresh ? NB_OK : read_ctrls(b); }
 
 nb_status nb_batch_set_state(nb_batch *b, int32_t k, const float *pos3, const float *vel3, const float *mass) {
     if (!b || k < 0 || k >= b->nsys || !pos3 || !mass) return NB_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->dev);
-    nb_status r = read_ctrls(b);
+    nb_status r = fresh_ctrls(b);
     if (r != NB_OK) return r;
     const SysMem &m = b->mem[k];
     const int par = b->h_ctrl[k].parity & 1;
     const size_t n = (size_t)m.n;
-    float *sp = b->d_stage, *sm = b->d_stage + 3 * n;
-    B_CUDA(b, cudaMemcpyAsync(sp, pos3, 12 * n, cudaMemcpyHostToDevice, b->st));
-    B_CUDA(b, cudaMemcpyAsync(sm, mass, 4 * n, cudaMemcpyHostToDevice, b->st));
-    B_CUDA(b, launch_pack(sp, sm, nullptr, m.body[par], nullptr, nullptr, m.n, b->st));
-    if (vel3) {
-        B_CUDA(b, cudaMemcpyAsync(sp, vel3, 12 * n, cudaMemcpyHostToDevice, b->st));
-        B_CUDA(b, launch_pack(nullptr, nullptr, sp, nullptr, m.vel, m.acc, m.n, b->st));
+    const float *dp = static_cast<const float *>(host_device_view(pos3, b->dev)),
+                *dm = static_cast<const float *>(host_device_view(mass, b->dev)),
+                *dv = static_cast<const float *>(host_device_view(vel3, b->dev));
+    if (dp && dm && (!vel3 || dv)) {  // the kernel reads the host arrays
+        B_CUDA(b, launch_pack(dp, dm, dv, m.body[par], m.vel, m.acc, m.n, b->st));
+        b->launches += 1;
     } else {
-        B_CUDA(b, launch_pack(nullptr, nullptr, nullptr, nullptr, m.vel, m.acc, m.n, b->st));
+        float *sp = b->d_stage, *sm = b->d_stage + 3 * n;
+        B_CUDA(b, cudaMemcpyAsync(sp, pos3, 12 * n, cudaMemcpyHostToDevice, b->st));
+        B_CUDA(b, cudaMemcpyAsync(sm, mass, 4 * n, cudaMemcpyHostToDevice, b->st));
+        B_CUDA(b, launch_pack(sp, sm, nullptr, m.body[par], nullptr, nullptr, m.n, b->st));
+        if (vel3) B_CUDA(b, cudaMemcpyAsync(sp, vel3, 12 * n, cudaMemcpyHostToDevice, b->st));
+        B_CUDA(b, launch_pack(nullptr, nullptr, vel3 ? sp : nullptr, nullptr, m.vel, m.acc, m.n, b->st));
+        b->launches += 2;
     }
     B_CUDA(b, cudaMemsetAsync(&m.ctrl->kdk_primed, 0, sizeof(int), b->st));
-    b->launches += 2;
     B_CUDA(b, cudaStreamSynchronize(b->st));
     return NB_OK;
 }
@@ -289,34 +300,31 @@ nb_status nb_batch_set_state(nb_batch *b, int32_t k, const float *pos3, const fl
 nb_status nb_batch_get_state(nb_batch *b, int32_t k, float *pos3, float *vel3, float *acc3, float *mass) {
     if (!b || k < 0 || k >= b->nsys) return NB_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->dev);
-    nb_status r = read_ctrls(b);
+    nb_status r = fresh_ctrls(b);
     if (r != NB_OK) return r;
     const SysMem &m = b->mem[k];
-    const int par = b->h_ctrl[k].parity & 1;
+    const float4 *body = m.body[b->h_ctrl[k].parity & 1];
     const size_t n = (size_t)m.n;
-    float *s0 = b->d_stage;
-    if (pos3) {
-        B_CUDA(b, launch_unpack(m.body[par], nullptr, nullptr, s0, nullptr, nullptr, m.n, b->st));
-        B_CUDA(b, cudaMemcpyAsync(pos3, s0, 12 * n, cudaMemcpyDeviceToHost, b->st));
-        B_CUDA(b, cudaStreamSynchronize(b->st));
+    float *host[4] = {pos3, vel3, acc3, mass}, *dev[4];
+    bool direct = pos3 || vel3 || acc3 || mass;
+    for (int q = 0; q < 4; ++q) {
+        dev[q] = static_cast<float *>(host_device_view(host[q], b->dev));
+        direct = direct && (!host[q] || dev[q]);
     }
-    if (vel3) {
-        B_CUDA(b, launch_unpack(nullptr, m.vel, nullptr, nullptr, s0, nullptr, m.n, b->st));
-        B_CUDA(b, cudaMemcpyAsync(vel3, s0, 12 * n, cudaMemcpyDeviceToHost, b->st));
-        B_CUDA(b, cudaStreamSynchronize(b->st));
+    if (direct) {  // the kernel writes the host arrays
+        B_CUDA(b, launch_unpack(body, m.vel, m.acc, dev[0], dev[1], dev[2], dev[3], m.n, b->st));
+        b->launches += 1;
+    } else {
+        for (int q = 0; q < 4; ++q) {  // through the staging, one array after the other
+            if (!host[q]) continue;
+            float *st = b->d_stage;
+            B_CUDA(b, launch_unpack(body, m.vel, m.acc, q == 0 ? st : nullptr, q == 1 ? st : nullptr,
+                                    q == 2 ? st : nullptr, q == 3 ? st : nullptr, m.n, b->st));
+            b->launches += 1;
+            B_CUDA(b, cudaMemcpyAsync(host[q], st, (q == 3 ? 4 : 12) * n, cudaMemcpyDeviceToHost, b->st));
+        }
     }
-    if (acc3) {
-        B_CUDA(b, launch_unpack(nullptr, nullptr, m.acc, nullptr, nullptr, s0, m.n, b->st));
-        B_CUDA(b, cudaMemcpyAsync(acc3, s0, 12 * n, cudaMemcpyDeviceToHost, b->st));
-        B_CUDA(b, cudaStreamSynchronize(b->st));
-    }
-    if (mass) {
-        std::vector<float4> tmp(n);
-        B_CUDA(b, cudaMemcpyAsync(tmp.data(), m.body[par], 16 * n, cudaMemcpyDeviceToHost, b->st));
-        B_CUDA(b, cudaStreamSynchronize(b->st));
-        for (size_t i = 0; i < n; ++i) mass[i] = tmp[i].w;
-    }
-    b->launches += (pos3 ? 1 : 0) + (vel3 ? 1 : 0) + (acc3 ? 1 : 0);
+    B_CUDA(b, cudaStreamSynchronize(b->st));
     return NB_OK;
 }
 
@@ -352,6 +360,7 @@ static nb_status enqueue_steps(nb_batch *b, float dt, int nsteps) {
         B_CUDA(b, cudaGraphInstantiate(&b->exec, b->graph, 0));
         b->launches_per_step = nl;
     }
+    b->ctrls_fresh = false;
     for (int i = 0; i < nsteps; ++i) B_CUDA(b, cudaGraphLaunch(b->exec, b->st));
     b->launches += (long long)nsteps * b->launches_per_step;
     return NB_OK;

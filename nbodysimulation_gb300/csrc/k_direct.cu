@@ -71,9 +71,9 @@ __global__ void k_copy_vertices(const float4 *__restrict__ b, int n, float4 *__r
 // The reference's packed float[3N] arrays <-> the float4 body layout.  A
 // block moves tiles of kPackTile bodies; when the float[3N] arrays are 16-byte
 // aligned, a whole tile's 3 * kPackTile floats move as contiguous float4
-// loads or stores through shared memory (the arrays may be pinned host
-// memory the device reads or writes directly, where full-width accesses
-// matter), otherwise as one float at a time.
+// loads or stores through shared memory (the arrays may be host memory the
+// device reads or writes directly, where full-width accesses matter),
+// otherwise as one float at a time.
 constexpr int kPackTile = 256;
 constexpr int kPackVec = kPackTile * 3 / 4;  // float4 per tile of float[3]
 
@@ -137,7 +137,7 @@ __device__ __forceinline__ void unpack_tile(const float4 *__restrict__ src, floa
 
 __global__ void __launch_bounds__(kPackTile) k_unpack(const float4 *__restrict__ body, const float4 *__restrict__ vel,
                                                       const float4 *__restrict__ acc, float *pos3, float *vel3,
-                                                      float *acc3, int n, int vec) {
+                                                      float *acc3, float *mass, int n, int vec) {
     __shared__ float4 tile[kPackVec];
     const int ntiles = (n + kPackTile - 1) / kPackTile;
     for (int k = blockIdx.x; k < ntiles; k += gridDim.x) {
@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(kPackTile) k_unpack(const float4 *__restrict__
         if (pos3) unpack_tile(body, pos3, i0, n, full, tile);
         if (vel3) unpack_tile(vel, vel3, i0, n, full, tile);
         if (acc3) unpack_tile(acc, acc3, i0, n, full, tile);
+        if (mass && i0 + threadIdx.x < (size_t)n) mass[i0 + threadIdx.x] = body[i0 + threadIdx.x].w;
     }
 }
 
@@ -222,11 +223,11 @@ cudaError_t launch_pack(const float *pos3, const float *mass, const float *vel3,
 }
 
 cudaError_t launch_unpack(const float4 *body, const float4 *vel, const float4 *acc, float *pos3, float *vel3,
-                          float *acc3, int n, cudaStream_t st) {
+                          float *acc3, float *mass, int n, cudaStream_t st) {
     const int tiles = (n + kPackTile - 1) / kPackTile;
     const int blocks = tiles < 4096 ? tiles : 4096;
     const int vec = aligned16(pos3) && aligned16(vel3) && aligned16(acc3);
-    k_unpack<<<blocks > 0 ? blocks : 1, kPackTile, 0, st>>>(body, vel, acc, pos3, vel3, acc3, n, vec);
+    k_unpack<<<blocks > 0 ? blocks : 1, kPackTile, 0, st>>>(body, vel, acc, pos3, vel3, acc3, mass, n, vec);
     return cudaGetLastError();
 }
 

@@ -274,7 +274,7 @@ static cudaError_t enqueue_copy_out(nb_server *s, const JobP &j, bool final_stat
     const float4 *cur = j->mem.body[j->done & 1];  // every step flips the current buffer
     float *pos3 = reinterpret_cast<float *>(d.dbuf);
     float *vel3 = final_state ? pos3 + 3 * n : nullptr;
-    if ((e = launch_unpack(cur, final_state ? j->mem.vel : nullptr, nullptr, pos3, vel3, nullptr, j->n,
+    if ((e = launch_unpack(cur, final_state ? j->mem.vel : nullptr, nullptr, pos3, vel3, nullptr, nullptr, j->n,
                            s->compute)) != cudaSuccess)
         return e;
     if ((e = cudaMemcpyAsync(d.dbuf + off, j->mem.ctrl, sizeof(Ctrl), cudaMemcpyDeviceToDevice, s->compute)) !=
