@@ -40,6 +40,7 @@
 #include <algorithm>
 
 #include "bh_device.cuh"
+#include "launch.cuh"
 
 namespace nbgb {
 
@@ -150,6 +151,7 @@ __device__ __forceinline__ int octant_at(u64 key, int level) { return (int)(key 
 __device__ __forceinline__ bool build_off(const Ctrl *c) { return read_status(c) != 0 || c->insert != 0; }
 
 __global__ void __launch_bounds__(256) k_path(DevSim s, BuildScratch b) {
+    wait_for_previous();
     if (build_off(s.ctrl)) return;
     float box[6];
     load_box(s.ctrl, box);
@@ -171,6 +173,7 @@ inline __host__ __device__ int scan_chunks(int levels) {
     return (chunks + kScanBlocks - 1) / kScanBlocks;
 }
 __global__ void __launch_bounds__(kScanThreads, 2) k_scan(DevSim s, BuildScratch b) {
+    wait_for_previous();
     __shared__ int warp_tot[32];
     __shared__ u64 warp_sq[32];
     __shared__ int before;
@@ -254,6 +257,7 @@ __device__ __forceinline__ bool too_crowded(const DevSim &s, const BuildScratch 
 }
 
 __global__ void __launch_bounds__(256) k_place(DevSim s, BuildScratch b) {
+    wait_for_previous();
     if (build_off(s.ctrl) || too_crowded(s, b)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
         const u64 key = b.path[i];
@@ -269,6 +273,7 @@ __global__ void __launch_bounds__(256) k_place(DevSim s, BuildScratch b) {
 // end up side by side, where k_cells sees them.
 constexpr int kRankChunk = 1024;
 __global__ void __launch_bounds__(256) k_rank(DevSim s, BuildScratch b) {
+    wait_for_previous();
     __shared__ u64 sh[kRankChunk];
     if (__syncthreads_or(build_off(s.ctrl))) return;  // other blocks of this kernel may set `insert`
     if (too_crowded(s, b)) {                          // grid-uniform
@@ -302,6 +307,7 @@ __global__ void __launch_bounds__(256) k_rank(DevSim s, BuildScratch b) {
 constexpr int kRankWarps = 8;
 constexpr int kRankPart = 512;  // loads in flight together; n <= kRankAll takes two parts
 __global__ void __launch_bounds__(32 * kRankWarps) k_rank_all(DevSim s, BuildScratch b) {
+    wait_for_previous();
     __shared__ u64 sh[kRankWarps][kRankPart];
     __shared__ int part[kRankWarps][32];
     if (build_off(s.ctrl)) return;  // grid-uniform: only earlier kernels set either
@@ -366,6 +372,7 @@ __device__ __forceinline__ int first_sharing(Key keys, int m, u64 key, int level
 constexpr int kCellTiles = 4;
 constexpr int kCellBodies = kCellTiles * kTile;
 __global__ void __launch_bounds__(kTile) k_cells(DevSim s, BuildScratch b, const u64 *__restrict__ path) {
+    wait_for_previous();
     __shared__ u64 key_sh[kCellBodies + 2];  // the paths of bodies a - 1 .. a + kCellBodies
     __shared__ int base_sh[kCellBodies];
     __shared__ int warp_tot[32];
@@ -491,6 +498,7 @@ __device__ __forceinline__ void sum_quadrupoles(unsigned group, unsigned mask, c
 
 template <bool kQuad>
 __global__ void __launch_bounds__(kTile) k_link(DevSim s, BuildScratch b, const u64 *__restrict__ path) {
+    wait_for_previous();
     __shared__ float4 pm[kTile];
     __shared__ float q6[kQuad ? 6 : 1][kQuad ? kTile : 1];
     __shared__ u64 key_sh[kTile];
@@ -721,6 +729,7 @@ __device__ __forceinline__ void top_cell(const DevSim &s, int cell, int ch, unsi
 
 template <bool kQuad>
 __global__ void __launch_bounds__(kTopThreads, 1) k_top(DevSim s, BuildScratch b) {
+    wait_for_previous();
     Ctrl *ctrl = s.ctrl;
     const int n = s.n, root = n + s.cap;
     const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
@@ -818,38 +827,35 @@ BuildScratch build_scratch(int n, int sm_count, int *mem, void *keys16, void *in
 
 cudaError_t launch_tree_box(const DevSim &s, const BuildScratch &b, int sm_count, cudaStream_t st) {
     const int blocks = std::max(1, std::min(4 * sm_count, (s.n + 255) / 256));
-    k_box<<<blocks, 256, 0, st>>>(s, b);
+    k_box<<<blocks, 256, 0, st>>>(s, b);  // not early: see launch.cuh
     return cudaGetLastError();
 }
 
 cudaError_t launch_tree_cells(const DevSim &s, const BuildScratch &b, int sm_count, cudaStream_t st, int *launches) {
     const int all = (s.n + 255) / 256;
     const int blocks = std::min(all, 8 * sm_count);
-    k_path<<<blocks, 256, 0, st>>>(s, b);
+    cudaError_t e = launch_next(k_path, blocks, 256, st, s, b);
     if (b.levels) {
         const int per = scan_chunks(b.levels) * kScanRegions;
-        k_scan<<<((1 << (3 * b.levels)) + per - 1) / per, kScanThreads, 0, st>>>(s, b);
-        k_place<<<blocks, 256, 0, st>>>(s, b);
-        k_rank<<<all, 256, 0, st>>>(s, b);
+        if (e == cudaSuccess)
+            e = launch_next(k_scan, ((1 << (3 * b.levels)) + per - 1) / per, kScanThreads, st, s, b);
+        if (e == cudaSuccess) e = launch_next(k_place, blocks, 256, st, s, b);
+        if (e == cudaSuccess) e = launch_next(k_rank, all, 256, st, s, b);
     } else {
-        k_rank_all<<<(s.n + 31) / 32, 32 * kRankWarps, 0, st>>>(s, b);
+        if (e == cudaSuccess) e = launch_next(k_rank_all, (s.n + 31) / 32, 32 * kRankWarps, st, s, b);
     }
-    k_cells<<<(s.n + kCellBodies - 1) / kCellBodies, kTile, 0, st>>>(s, b, b.levels ? b.path : b.placed);
+    if (e == cudaSuccess)
+        e = launch_next(k_cells, (s.n + kCellBodies - 1) / kCellBodies, kTile, st, s, b, b.levels ? b.path : b.placed);
     *launches = b.levels ? 5 : 3;
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_tree_sums(const DevSim &s, const BuildScratch &b, int quadrupole, int sm_count, cudaStream_t st) {
     const int tiles = (s.n + kTile - 1) / kTile;
     const u64 *path = b.levels ? b.path : b.placed;
-    if (quadrupole) {
-        k_link<true><<<tiles, kTile, 0, st>>>(s, b, path);
-        k_top<true><<<sm_count, kTopThreads, 0, st>>>(s, b);
-    } else {
-        k_link<false><<<tiles, kTile, 0, st>>>(s, b, path);
-        k_top<false><<<sm_count, kTopThreads, 0, st>>>(s, b);
-    }
-    return cudaGetLastError();
+    cudaError_t e = launch_next(quadrupole ? k_link<true> : k_link<false>, tiles, kTile, st, s, b, path);
+    if (e == cudaSuccess) e = launch_next(quadrupole ? k_top<true> : k_top<false>, sm_count, kTopThreads, st, s, b);
+    return e;
 }
 
 }  // namespace nbgb

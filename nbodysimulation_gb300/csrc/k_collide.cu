@@ -17,10 +17,12 @@
 #include <algorithm>
 
 #include "collide_device.cuh"
+#include "launch.cuh"
 
 namespace nbgb {
 
 __global__ void __launch_bounds__(kCollideWarps * 32) k_collision_warp(DevSim s) {
+    wait_for_previous();
     if (read_status(s.ctrl)) return;  // warp-uniform
     const int lane = threadIdx.x & 31;
     collide_warp(s.body_next, s.vel, s.n, blockIdx.x * kCollideWarps + (threadIdx.x >> 5), lane);
@@ -84,6 +86,7 @@ __global__ void k_grid_count(DevSim s, CollideGrid g) {
 // start of every bucket: a block lays its kScanBuckets buckets end to end at a
 // place from one atomic
 __global__ void __launch_bounds__(kScanBuckets / 4) k_grid_scan(DevSim s, CollideGrid g) {
+    wait_for_previous();
     if (read_status(s.ctrl)) return;  // grid-uniform, before any barrier
     __shared__ int warp_tot[kScanBuckets / 128];
     __shared__ int base;
@@ -115,6 +118,7 @@ __global__ void __launch_bounds__(kScanBuckets / 4) k_grid_scan(DevSim s, Collid
 
 // bodies into their buckets: {x, y, z, index}
 __global__ void k_grid_place(DevSim s, CollideGrid g) {
+    wait_for_previous();
     if (read_status(s.ctrl) || g.ctl[kGridNoCell]) return;
     const float inv = grid_inv();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
@@ -129,6 +133,7 @@ __global__ void k_grid_place(DevSim s, CollideGrid g) {
 // one target per thread, targets in bucket order (neighbours read the same
 // candidates)
 __global__ void __launch_bounds__(kGridThreads) k_grid_collide(DevSim s, CollideGrid g) {
+    wait_for_previous();
     __shared__ int found[kGridContacts][kGridThreads];
     if (read_status(s.ctrl) || g.ctl[kGridNoCell]) return;
     const int t = blockIdx.x * kGridThreads + threadIdx.x;
@@ -184,6 +189,7 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_collide(DevSim s, Collide
 // targets of the overflow list.  Few of them take one warp each, many one
 // thread each (as collide_warp_form_below decides between whole systems).
 __global__ void __launch_bounds__(kCollideThreads) k_grid_rest(DevSim s, CollideGrid g, const int *order, int few) {
+    wait_for_previous();
     if (read_status(s.ctrl)) return;  // block-uniform, before any barrier
     const bool all = g.ctl[kGridNoCell] != 0;
     const int cnt = all ? s.n : g.ctl[kGridOverflow];
@@ -200,22 +206,24 @@ __global__ void __launch_bounds__(kCollideThreads) k_grid_rest(DevSim s, Collide
 cudaError_t launch_collision(const DevSim &s, const CollideGrid &g, int tree, int sm_count, cudaStream_t st,
                              int *launches) {
     if (!g.count) {
-        k_collision_warp<<<(s.n + kCollideWarps - 1) / kCollideWarps, kCollideWarps * 32, 0, st>>>(s);
         *launches = 1;
-        return cudaGetLastError();
+        return launch_next(k_collision_warp, (s.n + kCollideWarps - 1) / kCollideWarps, kCollideWarps * 32, st, s);
     }
+    *launches = 5;
     // counts and the control words, one array
-    const cudaError_t e = cudaMemsetAsync(g.count, 0, sizeof(int) * ((size_t)g.mask + 1 + kGridCtl), st);
+    cudaError_t e = cudaMemsetAsync(g.count, 0, sizeof(int) * ((size_t)g.mask + 1 + kGridCtl), st);
     if (e != cudaSuccess) return e;
     const int blocks = std::min((s.n + 255) / 256, sm_count * 8);
     k_grid_count<<<blocks, 256, 0, st>>>(s, g);
-    k_grid_scan<<<(int)((g.mask + 1) / kScanBuckets), kScanBuckets / 4, 0, st>>>(s, g);
-    k_grid_place<<<blocks, 256, 0, st>>>(s, g);
-    k_grid_collide<<<(s.n + kGridThreads - 1) / kGridThreads, kGridThreads, 0, st>>>(s, g);
-    k_grid_rest<<<(s.n + kCollideThreads - 1) / kCollideThreads, kCollideThreads, 0, st>>>(
-        s, g, tree ? s.sorted : nullptr, collide_warp_form_below(sm_count) * kCollideThreads);
-    *launches = 5;
-    return cudaGetLastError();
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_next(k_grid_scan, (int)((g.mask + 1) / kScanBuckets), kScanBuckets / 4, st, s, g);
+    if (e == cudaSuccess) e = launch_next(k_grid_place, blocks, 256, st, s, g);
+    if (e == cudaSuccess)
+        e = launch_next(k_grid_collide, (s.n + kGridThreads - 1) / kGridThreads, kGridThreads, st, s, g);
+    if (e == cudaSuccess)
+        e = launch_next(k_grid_rest, (s.n + kCollideThreads - 1) / kCollideThreads, kCollideThreads, st, s, g,
+                        tree ? s.sorted : nullptr, collide_warp_form_below(sm_count) * kCollideThreads);
+    return e;
 }
 
 }  // namespace nbgb

@@ -7,6 +7,7 @@
 
 #include "direct_device.cuh"
 #include "integrate.cuh"
+#include "launch.cuh"
 
 namespace nbgb {
 
@@ -23,6 +24,7 @@ constexpr int kDirectWarps = 8;
 template <int kI, bool kQuirk, int kZero>
 __global__ void __launch_bounds__(32 * kDirectWarps, kI == 4 ? 2 : 3)
     k_direct(DevSim s, StepParams p, float4 *part, int *arrived, float4 *out) {
+    wait_for_previous();
     __shared__ DirectShared<kDirectWarps> sh;
     __shared__ int last;
     const int n = s.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -190,10 +192,10 @@ static cudaError_t launch_direct_z(const DevSim &s, const StepParams &p, const D
                                    int *arrived, float4 *out, cudaStream_t st) {
     const dim3 grid((unsigned)((s.n + 32 * d.ki - 1) / (32 * d.ki)), (unsigned)d.slices);
     const int threads = 32 * kDirectWarps;
-    if (d.ki == 4) k_direct<4, kQuirk, kZero><<<grid, threads, 0, st>>>(s, p, part, arrived, out);
-    else if (d.ki == 2) k_direct<2, kQuirk, kZero><<<grid, threads, 0, st>>>(s, p, part, arrived, out);
-    else k_direct<1, kQuirk, kZero><<<grid, threads, 0, st>>>(s, p, part, arrived, out);
-    return cudaGetLastError();
+    return launch_next(d.ki == 4   ? k_direct<4, kQuirk, kZero>
+                       : d.ki == 2 ? k_direct<2, kQuirk, kZero>
+                                   : k_direct<1, kQuirk, kZero>,
+                       grid, threads, st, s, p, part, arrived, out);
 }
 
 // `p.eps` is the softening to use; s.part (direct_part_bodies float4) holds

@@ -2,11 +2,13 @@
 // groups of 32 sorted bodies from a global counter and walk the tree
 // (force_group, force_device.cuh), then integrate.
 #include "force_device.cuh"
+#include "launch.cuh"
 
 namespace nbgb {
 
 template <int kMethod, bool kComp, bool kEpsZero, bool kQuad>
 __global__ void __launch_bounds__(kForceThreads, 8) k_force(DevSim s, StepParams p) {
+    wait_for_previous();
     __shared__ float s_dq[kMaxDepth];
     __shared__ WarpLists<kQuad> s_lists[kForceWarps];
     __shared__ int s_skip;
@@ -51,8 +53,9 @@ static cudaError_t launch_force_t(const DevSim &s, const StepParams &p, int sm_c
     int blocks = per_sm * sm_count;
     const int need = ((s.n + 31) / 32 + kForceWarps - 1) / kForceWarps;
     if (blocks > need) blocks = need > 0 ? need : 1;
-    if (ez) k_force<kMethod, kComp, true, kQuad><<<blocks, kForceThreads, 0, st>>>(s, p);
-    else k_force<kMethod, kComp, false, kQuad><<<blocks, kForceThreads, 0, st>>>(s, p);
+    const auto kernel = ez ? k_force<kMethod, kComp, true, kQuad> : k_force<kMethod, kComp, false, kQuad>;
+    if (blocks == per_sm * sm_count) return launch_next(kernel, blocks, kForceThreads, st, s, p);
+    kernel<<<blocks, kForceThreads, 0, st>>>(s, p);  // a part of the GPU: spread evenly (launch.cuh)
     return cudaGetLastError();
 }
 
