@@ -85,7 +85,7 @@ static nb_status rebuild_tables(nb_batch *b) {
             sysdesc_set_top(b->h_sys[k], b->mem[k], b->cfg[k].tree_semantics == NB_TREE_REFERENCE,
                             b->shape.top_levels);
     std::vector<int> pref(batch_prefix_ints(ns), 0);
-    int totals[kBatchSpaces];
+    int totals[kBatchTotals];
     batch_prefixes(b->h_sys.data(), ns, batch_direct_block_bodies(b->variant), pref.data(), totals,
                    b->shape.build_chunk);
     B_CUDA(b, cudaMemcpyAsync(b->d_sys, b->h_sys.data(), sizeof(SysDesc) * ns, cudaMemcpyHostToDevice, b->st));
@@ -189,6 +189,7 @@ nb_status nb_batch_create(const nb_config *cfgs, int32_t nsys, nb_batch **out) {
         m.n = c.num_of_bodies;
         m.tree = c.algo_config == NB_BARNES_HUT;
         m.quad = m.tree && b->quad;
+        m.ref = c.tree_semantics == NB_TREE_REFERENCE;
         m.cap = m.tree ? (c.cell_capacity > 0 ? c.cell_capacity : sysmem_default_capacity(m.n)) : 0;
         if (m.tree && (long long)m.n + m.cap + 1 >= (1LL << 26) - 1) return fail_all(NB_ERR_UNSUPPORTED);
         total = sysmem_align(total) + sysmem_layout(m, nullptr);
@@ -208,7 +209,8 @@ nb_status nb_batch_create(const nb_config *cfgs, int32_t nsys, nb_batch **out) {
         cudaMallocHost(&b->h_ctrl, sizeof(Ctrl) * nsys) != cudaSuccess ||
         cudaMalloc(&b->d_sys, sizeof(SysDesc) * nsys) != cudaSuccess ||
         cudaMalloc(&b->d_pref, sizeof(int) * batch_prefix_device_ints(nsys)) != cudaSuccess ||
-        cudaMalloc(&b->d_work, sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&b->d_work, sizeof(int) * kBatchWorkInts) != cudaSuccess ||
+        cudaMemset(b->d_work, 0, sizeof(int) * kBatchWorkInts) != cudaSuccess ||
         cudaMalloc(&b->d_stage, sizeof(float) * 4 * (size_t)maxn) != cudaSuccess)
         return fail_all(NB_ERR_OUT_OF_MEMORY);
     memset(b->h_ctrl, 0, sizeof(Ctrl) * nsys);

@@ -244,9 +244,10 @@ __device__ __forceinline__ void top_count_range(const DevSim &s, const TopTables
 // blockDim.x, so a thread takes at most 32 regions of a level and a level has
 // at most kTopRegions / 32 (round, warp) pairs.
 __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables &t) {
-    __shared__ int cnt_sh[kTopInner];   // body counts, regions of levels 1..L-1
-    __shared__ int deep_sh[kTopInner];  // (level << 26) | deepest existing cell of the region's path
-    __shared__ int rank_sh[kTopRegions / 32];  // per (round, warp): new cells before it
+    constexpr int kRegions = 1 << (3 * kBatchTopMaxLevels), kInner = (kRegions - 8) / 7;
+    __shared__ int cnt_sh[kInner];          // body counts, regions of levels 1..L-1
+    __shared__ int deep_sh[kInner];         // (level << 26) | deepest existing cell of the region's path
+    __shared__ int rank_sh[kRegions / 32];  // per (round, warp): new cells before it
     __shared__ int warp_tot[32];
     __shared__ int s_skip, s_bottom;
     Ctrl *ctrl = s.ctrl;
@@ -349,7 +350,7 @@ __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables
 __device__ __forceinline__ int insert_from_top(const DevSim &s, const TopTables &t, const GeoCube &root_g, int i,
                                                long long spin_cap) {
     const float4 P = s.body_cur[i];
-    const int e = __ldg(&t.start[top_region(root_g, P, t.levels)]);
+    const int e = __ldcg(&t.start[top_region(root_g, P, t.levels)]);
     const int lv = (int)((unsigned)e >> 26), node = e & ((1 << 26) - 1);
     GeoCube g = root_g;
     for (int l = 0; l < lv; ++l) g.descend(P.x, P.y, P.z);

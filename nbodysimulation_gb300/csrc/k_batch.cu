@@ -1,261 +1,18 @@
 // k_batch.cu -- one launch per stage for many independent systems of uneven
 // N.  Every kernel walks the batch's table of systems (SysDesc): the work
 // of all systems is laid end to end in one index space per stage (bodies in
-// chunks, cell slots, warp groups, direct-sum target blocks) and a thread
-// finds its system with a binary search in the stage's prefix table.
-// Barnes-Hut systems run the same per-item code as the single-system
-// kernels (bh_device.cuh, force_device.cuh); small systems take the direct
-// sum (direct_device.cuh).  A step is: reset, bbox, top-level counts, top cells,
-// build, used-cell scan, summarize, sort, force, direct, flip -- captured
-// once into a CUDA graph by the host.
-#include "bh_device.cuh"
+// chunks or tiles, warp groups, direct-sum target blocks) and a warp finds its
+// system in the stage's prefix table.
+// Barnes-Hut systems run the same per-item code as the single-system kernels;
+// their trees are k_batch_build.cu's.  Small systems take the direct sum
+// (direct_device.cuh).  A step is: box, paths, places, ranks, cells, sums in
+// tiles, sums above, insertions, force, direct, flip -- captured once into a CUDA
+// graph by the host.
 #include "collide_device.cuh"
 #include "direct_device.cuh"
 #include "force_device.cuh"
 
 namespace nbgb {
-
-// ---------------------------------------------------------------------------
-// reset (init, kernels/init.cl:26-33) for every Barnes-Hut system
-// ---------------------------------------------------------------------------
-__global__ void k_batch_reset(BatchTables t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= t.nsys) return;
-    const SysDesc &d = t.sys[k];
-    if (!d.active || d.kind != kSysBH || !system_live(d.v.ctrl)) return;
-    const DevSim &s = d.v;
-    Ctrl *c = s.ctrl;
-    c->bbox_key[0] = c->bbox_key[1] = c->bbox_key[2] = 0xFFFFFFFFu;
-    c->bbox_key[3] = c->bbox_key[4] = c->bbox_key[5] = 0u;
-    int4 *row = reinterpret_cast<int4 *>(&s.child[s.cap * 8]);
-    row[0] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
-    row[1] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
-    c->bottom = s.n + s.cap;
-    c->max_depth = 0;
-    c->work = 0;
-    s.arrive[s.cap] = 0;
-    s.start[s.cap] = 0;
-    s.count[s.cap] = 0;
-    s.parent[s.cap] = -1;
-}
-
-// ---------------------------------------------------------------------------
-// bbox: one block per chunk of one system; order-preserving integer keys,
-// one atomic per component per block (as k_bbox)
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_batch_bbox(BatchTables t) {
-    const int k = find_system(t.chunk_prefix, t.nsys, blockIdx.x);
-    const SysDesc &d = t.sys[k];
-    if (!system_live(d.v.ctrl)) return;  // block-uniform
-    const DevSim s = system_view(d);
-    const int i0 = (blockIdx.x - d.chunk_begin) * d.chunk;
-    const int i1 = min(s.n, i0 + d.chunk);
-    unsigned mn0 = 0xFFFFFFFFu, mn1 = 0xFFFFFFFFu, mn2 = 0xFFFFFFFFu, mx0 = 0u, mx1 = 0u, mx2 = 0u;
-    int bad = -1;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const float4 p = __ldg(&s.body_cur[i]);
-        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) bad = i;
-        const unsigned kx = f2key(p.x), ky = f2key(p.y), kz = f2key(p.z);
-        mn0 = min(mn0, kx); mx0 = max(mx0, kx);
-        mn1 = min(mn1, ky); mx1 = max(mx1, ky);
-        mn2 = min(mn2, kz); mx2 = max(mx2, kz);
-    }
-    mn0 = __reduce_min_sync(0xffffffffu, mn0);
-    mn1 = __reduce_min_sync(0xffffffffu, mn1);
-    mn2 = __reduce_min_sync(0xffffffffu, mn2);
-    mx0 = __reduce_max_sync(0xffffffffu, mx0);
-    mx1 = __reduce_max_sync(0xffffffffu, mx1);
-    mx2 = __reduce_max_sync(0xffffffffu, mx2);
-    __shared__ unsigned red[8][6];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-        red[w][0] = mn0; red[w][1] = mn1; red[w][2] = mn2;
-        red[w][3] = mx0; red[w][4] = mx1; red[w][5] = mx2;
-    }
-    if (bad >= 0) set_status(s.ctrl, kStNonFinite, bad);
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        const int c = threadIdx.x;
-        unsigned v = red[0][c];
-        for (int j = 1; j < 8; ++j) v = c < 3 ? min(v, red[j][c]) : max(v, red[j][c]);
-        if (c < 3) atomicMin(&s.ctrl->bbox_key[c], v);
-        else atomicMax(&s.ctrl->bbox_key[c], v);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// build: one block per chunk of one system (insert_body), one max-depth
-// atomic per block.  Lock holders are always running threads, so no
-// co-residency is needed.
-// ---------------------------------------------------------------------------
-template <class Geo, bool kRef>
-__device__ __forceinline__ int build_chunk(const DevSim &s, int i0, int i1) {
-    float box[6];
-    load_box(s.ctrl, box);
-    const Geo root_g = Geo::root(box);
-    int local_max = 0;
-    const long long cap = tree_spin_cap(s.ctrl);
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const int depth = insert_body<Geo, kRef>(s, root_g, i, cap);
-        if (depth < 0) return -1;
-        local_max = max(local_max, depth);
-    }
-    return local_max;
-}
-
-// the same from the top levels (insert_from_top)
-__device__ __forceinline__ int build_chunk_top(const DevSim &s, const TopTables &top, int i0, int i1) {
-    float box[6];
-    load_box(s.ctrl, box);
-    const GeoCube root_g = GeoCube::root(box);
-    int local_max = 0;
-    const long long cap = tree_spin_cap(s.ctrl);
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
-        const int depth = insert_from_top(s, top, root_g, i, cap);
-        if (depth < 0) return -1;
-        local_max = max(local_max, depth);
-    }
-    return local_max;
-}
-
-// ---------------------------------------------------------------------------
-// top levels of every cubic-root tree that has them (top_levels): region
-// counts per chunk of bodies in shared-memory bins, then one block per tree
-// creates its top cells (top_cells_block); the build then starts every
-// insertion below them
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_batch_top_count(BatchTables t) {
-    __shared__ int bins[1 << (3 * kBatchTopMaxLevels)];
-    const int k = find_system(t.chunk_prefix, t.nsys, blockIdx.x);
-    const SysDesc &d = t.sys[k];
-    // block-uniform, before any barrier: only earlier kernels set the status
-    if (d.top.levels == 0 || !system_live(d.v.ctrl) || read_status(d.v.ctrl)) return;
-    const DevSim s = system_view(d);
-    float box[6];
-    load_box(s.ctrl, box);
-    const int i0 = (blockIdx.x - d.chunk_begin) * d.chunk;
-    top_count_range(s, d.top, GeoCube::root(box), i0, min(s.n, i0 + d.chunk), blockDim.x, bins);
-}
-
-static_assert((1 << (3 * kBatchTopMaxLevels)) <= 32 * 256, "top_cells_block: at most 32 regions a thread");
-__global__ void __launch_bounds__(256) k_batch_top_cells(BatchTables t) {
-    const SysDesc &d = t.sys[blockIdx.x];
-    if (!d.active || d.kind != kSysBH || d.top.levels == 0 || !system_live(d.v.ctrl)) return;
-    top_cells_block(system_view(d), d.top);
-}
-
-__global__ void __launch_bounds__(256) k_batch_build(BatchTables t) {
-    const int k = find_system(t.chunk_prefix, t.nsys, blockIdx.x);
-    const SysDesc &d = t.sys[k];
-    const DevSim s = system_view(d);
-    if (read_status(s.ctrl) || !system_live(s.ctrl)) return;
-    const int i0 = (blockIdx.x - d.chunk_begin) * d.chunk;
-    const int i1 = min(s.n, i0 + d.chunk);
-    const int depth = d.p.tree_ref     ? build_chunk<RefBox, true>(s, i0, i1)
-                      : d.top.levels ? build_chunk_top(s, d.top, i0, i1)
-                                     : build_chunk<GeoCube, false>(s, i0, i1);
-    if (depth < 0) return;
-    const unsigned am = __activemask();
-    const int wmax = __reduce_max_sync(am, depth);
-    if ((threadIdx.x & 31) == __ffs(am) - 1) atomicMax(&s.ctrl->max_depth, wmax);
-}
-
-// ---------------------------------------------------------------------------
-// used cells: after the build, every tree's allocated cells [bottom, root]
-// are laid end to end (one exclusive scan over the systems, one block), so
-// summarize and sort visit only cells that exist.  A tree whose step failed,
-// or that has no steps left, contributes none.
-// ---------------------------------------------------------------------------
-constexpr int kScanThreads = 1024;
-__global__ void __launch_bounds__(kScanThreads) k_batch_used(BatchTables t) {
-    __shared__ int warp_sum[kScanThreads / 32];
-    __shared__ int carry;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < t.nsys; base += kScanThreads) {
-        const int k = base + threadIdx.x;
-        int used = 0;
-        if (k < t.nsys) {
-            const SysDesc &d = t.sys[k];
-            const Ctrl *c = d.v.ctrl;
-            if (d.active && d.kind == kSysBH && system_live(c) && !read_status(c))
-                used = d.v.n + d.v.cap - c->bottom + 1;
-        }
-        int incl = used;  // inclusive scan: warps, then warp totals
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) warp_sum[w] = incl;
-        __syncthreads();
-        if (w == 0) {
-            int v = warp_sum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += u;
-            }
-            warp_sum[lane] = v;  // inclusive over warps
-        }
-        __syncthreads();
-        const int before = carry + (w > 0 ? warp_sum[w - 1] : 0) + incl - used;
-        if (k < t.nsys) t.used_prefix[k] = before;
-        __syncthreads();
-        if (threadIdx.x == kScanThreads - 1) carry = before + used;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) t.used_prefix[t.nsys] = carry;
-}
-
-// ---------------------------------------------------------------------------
-// summarize: one allocated cell per thread over all trees
-// ---------------------------------------------------------------------------
-template <bool kQuad>
-__global__ void __launch_bounds__(256) k_batch_summarize(BatchTables t) {
-    const int total = t.used_prefix[t.nsys];
-    const int stride = gridDim.x * blockDim.x;
-    int k = 0, lo = 0, hi = 0;  // the system of the last x and its range (x only grows)
-    int first = 0, par = 0;     // that system's first allocated cell and buffer parity, read once
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-        if (x >= hi) {
-            k = find_system(t.used_prefix, t.nsys, x);
-            lo = t.used_prefix[k];
-            hi = t.used_prefix[k + 1];
-            first = t.sys[k].v.ctrl->bottom;
-            par = system_parity(t.sys[k]);
-        }
-        summarize_from<kQuad>(system_view_par(t.sys[k], par), first + (x - lo));
-    }
-}
-
-// ---------------------------------------------------------------------------
-// sort: inside every tree the cells are visited from the root downward (a
-// parent before its children); the grid is no larger than what is
-// co-resident, so every bounded wait in sort_cell is for a cell another
-// running thread handles in an earlier or the same round.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_batch_sort(BatchTables t) {
-    const int total = t.used_prefix[t.nsys];
-    const int stride = gridDim.x * blockDim.x;
-    int k = 0, lo = 0, hi = 0;  // the system of the last x and its range (x only grows)
-    bool skip = false;          // that system's status and wait limit, read once per system
-    long long cap = 0;
-    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-        if (x >= hi) {
-            k = find_system(t.used_prefix, t.nsys, x);
-            lo = t.used_prefix[k];
-            hi = t.used_prefix[k + 1];
-            const Ctrl *c = t.sys[k].v.ctrl;
-            skip = read_status(c) != 0;
-            cap = tree_spin_cap(c);
-        }
-        if (skip) continue;
-        const DevSim &s = t.sys[k].v;  // the sort reads no body buffer
-        if (!sort_cell(s, s.n + s.cap - (x - lo), cap)) skip = true;
-    }
-}
 
 // ---------------------------------------------------------------------------
 // force: warps take groups from one batch-wide counter; a warp recomputes its
@@ -293,6 +50,7 @@ __global__ void __launch_bounds__(kBatchForceMaxWarps * 32, 2) k_batch_force(Bat
     int &s_cur_w = me.cur, &s_begin_w = me.begin, &s_mode_w = me.mode;
     const int lane = threadIdx.x & 31;
     if (lane == 0) s_cur_w = -1;
+    if (blockIdx.x == 0 && threadIdx.x > 0 && threadIdx.x < kBatchWorkInts) t.work[threadIdx.x] = 0;  // for the next step
     __syncwarp();
     while (true) {
         int gg = 0;
@@ -404,13 +162,6 @@ __global__ void __launch_bounds__(kCollideThreads) k_batch_collision(BatchTables
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-static int resident(const void *fn, int threads, int sm_count) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    return per_sm * sm_count;
-}
-
 // Direct-sum variants the autotuner chooses from: {targets per lane, warps per
 // block}.
 struct DirectVariant {
@@ -474,37 +225,20 @@ static cudaError_t launch_batch_force_m(const BatchTables &t, int comp, int quad
                 : launch_batch_force_t<kMethod, false, false>(t, shape, sm_count, st);
 }
 
-// bbox .. force of every tree system; *launches gets the kernel count
+// the tree stages and the force of every tree system; *launches gets the kernel count
 static cudaError_t launch_batch_tree_stages(const BatchTables &t, int method, int comp, int quad,
                                             const TreeShape &shape, int sm_count, cudaStream_t st,
-                                            const StepFork *fork, bool branch, int *launches) {
+                                            int *launches) {
     cudaError_t e = cudaSuccess;
-    const int sb = (t.nsys + 127) / 128;
-    k_batch_reset<<<sb, 128, 0, st>>>(t);
-    k_batch_bbox<<<t.chunks, 256, 0, st>>>(t);
-    k_batch_top_count<<<t.chunks, 256, 0, st>>>(t);
-    k_batch_top_cells<<<t.nsys, 256, 0, st>>>(t);
-    k_batch_build<<<t.chunks, 256, 0, st>>>(t);
-    k_batch_used<<<1, kScanThreads, 0, st>>>(t);
-    // many blocks, so the grid-stride tail is short (512 systems: 8 per SM
-    // 4.79 ms, 32 per SM 2.90 ms)
-    int sblocks = sm_count * 32;
-    const int need = (t.cells + 255) / 256;
-    if (sblocks > need) sblocks = need;
-    if (quad) k_batch_summarize<true><<<sblocks, 256, 0, st>>>(t);
-    else k_batch_summarize<false><<<sblocks, 256, 0, st>>>(t);
-    if (branch && (e = cudaStreamWaitEvent(st, fork->join, 0)) != cudaSuccess) return e;
-    int rblocks = resident((const void *)k_batch_sort, 256, sm_count);
-    if (rblocks > need) rblocks = need;
-    k_batch_sort<<<rblocks, 256, 0, st>>>(t);
-    if ((e = cudaMemsetAsync(t.work, 0, sizeof(int), st)) != cudaSuccess) return e;
+    int built = 0;
+    if ((e = launch_batch_build(t, quad, sm_count, st, &built)) != cudaSuccess) return e;
     switch (method) {
     case 1: e = launch_batch_force_m<1>(t, comp, quad, shape, sm_count, st); break;
     case 2: e = launch_batch_force_m<2>(t, comp, quad, shape, sm_count, st); break;
     case 3: e = launch_batch_force_m<3>(t, comp, quad, shape, sm_count, st); break;
     default: e = launch_batch_force_m<0>(t, comp, quad, shape, sm_count, st); break;
     }
-    if (launches) *launches = 9;
+    if (launches) *launches = built + 1;
     return e;
 }
 
@@ -529,11 +263,10 @@ cudaError_t launch_batch_step(const BatchTables &t, int method, int comp, int qu
     }
     if (t.chunks > 0) {
         int tl = 0;
-        if ((e = launch_batch_tree_stages(t, method, comp, quad, shape, sm_count, st, fork, branch, &tl)) !=
-            cudaSuccess)
-            return e;
+        if ((e = launch_batch_tree_stages(t, method, comp, quad, shape, sm_count, st, &tl)) != cudaSuccess) return e;
         nl += tl;
     }
+    if (branch && (e = cudaStreamWaitEvent(st, fork->join, 0)) != cudaSuccess) return e;
     if (t.dblocks > 0 && !branch) {
         if ((e = launch_direct_variant(t, direct_variant, st)) != cudaSuccess) return e;
         nl += 1;

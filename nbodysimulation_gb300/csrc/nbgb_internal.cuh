@@ -153,10 +153,11 @@ __device__ __forceinline__ void load_box(const Ctrl *c, float box[6]) {
 // One system of a batch (nb_batch / nb_server): its buffers, its step
 // parameters and where its work starts in the batch-wide index spaces.
 enum SysKind { kSysBH = 0, kSysDirect = 1 };
-// Per-system tables of the top levels of the cubic-root tree (k_tree.cu):
-// body counts of the 8^levels regions of the deepest top level (zero between
-// steps) and, per region, the packed (level << 26) | cell its bodies start
-// their insertion at.  levels = 0: every insertion starts at the root.
+// Per-system tables of the top levels of a batched cubic-root tree that takes
+// the insertions: body counts of the 8^levels regions of the deepest top level
+// (zero between steps) and, per region, the packed (level << 26) | cell its
+// bodies start their insertion at.  levels = 0: every insertion starts at the
+// root.
 struct TopTables {
     int *count;
     int *start;
@@ -181,6 +182,27 @@ inline int batch_top_levels_for(int n) {
     return l < kBatchTopMaxLevels ? l : kBatchTopMaxLevels;
 }
 
+// The build's scratch of a batched tree (k_batch_build.cu), one piece: counters,
+// region counts, region starts, cells that reach over a tile's edge, and n ints.
+struct BuildTables {
+    int *mem;
+    int levels;
+};
+// regions of a batched tree: two bodies or more each on average, fewer than 16
+// (one block scans a tree's counts; 8^7 of them in 0.1 ms)
+// (With the reference's semantics one level more: their boxes divide x and z
+// only after the first levels, as the y bounds follow x, so an eighth of the
+// regions is used.)
+inline int batch_build_levels(int n, int ref) {
+    int l = 1;
+    while (l < 8 && (16LL << (3 * l)) <= (long long)n) ++l;
+    return l + (ref && l < 8);
+}
+// Larger trees with the reference's semantics take the insertions at once: some
+// two of their bodies nearly always share 20 levels.
+constexpr int kRefPathBodies = 1 << 17;
+constexpr int kBuildTileBodies = 1024;  // bodies per entry of tile_prefix
+
 struct SysDesc {
     DevSim v;          // pointers; body_cur / body_next come from body[] and ctrl->parity
     float4 *body[2];
@@ -188,32 +210,39 @@ struct SysDesc {
     int kind;          // SysKind
     int active;        // 0: skipped by every stage
     int body_begin;    // prefix over all systems' bodies
-    int chunk_begin;   // prefix over BH systems' bbox/build chunks
-    int cell_begin;    // prefix over BH systems' cell slots (cap + 1)
+    int chunk_begin;   // prefix over BH systems' chunks
     int group_begin;   // prefix over BH systems' warp groups
     int dblock_begin;  // prefix over direct systems' target blocks
     int cblock_begin;  // prefix over colliding systems' collision blocks
+    int tile_begin;    // prefix over the sorted builds' tiles of kBuildTileBodies bodies
     int collide;       // the collision update runs after the force and integrate stages
-    int chunk;         // bodies per bbox / build block (batch_chunk)
-    TopTables top;     // top-level tables; levels = 0: insertions from the root
+    int chunk;         // bodies per block of the box and the insertions (batch_chunk)
+    BuildTables build; // scratch of the build from sorted paths
+    TopTables top;     // of the insertions: top-level tables; levels = 0: insertions from the root
 };
 
 // Prefix tables (nsys + 1 entries each) and totals of a batch.
+constexpr int kBatchWorkInts = 4;
 struct BatchTables {
     const SysDesc *sys;
     int nsys;
-    const int *chunk_prefix, *cell_prefix, *group_prefix, *dblock_prefix, *cblock_prefix;
-    int chunks, cells, groups, dblocks, cblocks;
-    int *work;         // batch-wide force work counter
+    const int *chunk_prefix, *group_prefix, *dblock_prefix, *cblock_prefix, *tile_prefix;
+    int chunks, groups, dblocks, cblocks, tiles;
+    int large_refs;    // trees that take the insertions at every step (kRefPathBodies)
+    int *work;         // kBatchWorkInts batch-wide counters, zero before the first step
     int *used_prefix;  // nsys + 1: prefix over the cells each tree allocated this step (device-written)
 };
 
+// The system of entry x of a prefix table (the largest k with prefix[k] <= x), by
+// whole warps: 32 places a round.
 __device__ __forceinline__ int find_system(const int *prefix, int nsys, int x) {
-    int lo = 0, hi = nsys;  // largest k with prefix[k] <= x and prefix[k+1] > x
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = nsys;  // prefix[lo] <= x < prefix[hi]
     while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(&prefix[mid]) <= x) lo = mid;
-        else hi = mid;
+        const int step = (hi - lo + 31) >> 5, at = lo + lane * step;
+        const bool before = at < hi && __ldg(&prefix[at]) <= x;
+        lo += (__popc(__ballot_sync(0xffffffffu, before)) - 1) * step;
+        hi = min(hi, lo + step);
     }
     return lo;
 }
@@ -237,6 +266,7 @@ constexpr int kScanBlocks = 256;
 enum { kBuildBoxes = 0, kBuildBarrier = 1, kBuildTop = 2, kBuildPairs = 4, kBuildCtl = 8 };  // words of ctl
 struct BuildScratch {
     int levels;        // levels of the regions; 0: all bodies are ranked together
+    int ref;           // 1: the reference's tree semantics
     int *ctl;          // counters (zero before the first step)
     int *total;        // k_scan: blocks' totals + 1 (kScanBlocks)
     int *count;        // bodies per region, zero between steps
@@ -257,7 +287,11 @@ inline int build_levels(int n) {  // between a quarter and two bodies a region, 
     return l;
 }
 // a tile of 256 bodies starts at most one such cell a level; and the root
-inline size_t build_top_cells(int n) { return ((size_t)(n + 255) / 256 * 21 + 1 + 3) / 4 * 4; }
+inline __host__ __device__ size_t build_top_cells(int n) { return ((size_t)(n + 255) / 256 * 21 + 1 + 3) / 4 * 4; }
+// ints of BuildTables::mem
+inline size_t batch_build_ints(int n, int ref) {
+    return kBuildCtl + ((size_t)2 << (3 * batch_build_levels(n, ref))) + 4 + build_top_cells(n) + (size_t)n + 8;
+}
 size_t build_scratch_ints(int n, int sm_count);
 // mem: build_scratch_ints ints, zeroed; keys16 / ints12: 16 n and 12 n bytes
 // that the step may overwrite
@@ -335,7 +369,7 @@ cudaError_t launch_diagnostics(const float4 *body, const float4 *vel, int n, int
                                double G, double *out9, cudaStream_t st);
 
 // batched systems (k_batch.cu)
-// Bodies per bbox / build block of a batched tree.  Threads that start at a
+// Bodies per block of a batched tree's box and insertions.  Threads that start at a
 // root together contend for its first cells, so fewer per tree is better
 // once the batch as a whole has threads enough: 4096 when the batch's trees
 // hold 4M bodies or more, or for a tree of 2^19 bodies or more; 1024
@@ -349,9 +383,8 @@ constexpr int kBatchDirectDefault = 3;  // the variant of a batch that is not tu
 int batch_direct_variants();
 int batch_direct_block_bodies(int variant);
 // Optional second stream of a captured batched step: the small systems'
-// direct sum runs on it beside the tree stages up to the summarisation (a
-// parallel branch of the graph); the sort, whose waits assume its whole grid
-// is resident, starts after both.
+// direct sum runs on it beside the tree stages (a parallel branch of the
+// graph), whose few waits assume no more than that it ends by itself.
 struct StepFork {
     cudaStream_t aux;
     cudaEvent_t fork, join;
@@ -362,8 +395,8 @@ struct StepFork {
 struct TreeShape {
     int force_warps = 4;       // warps per block of the batched force kernel: 2, 4 or 8
     int force_grid_pct = 100;  // percent of the resident force blocks launched
-    int build_chunk = 0;       // bodies per bbox / build block of every tree; 0: batch_chunk's rule
-    int top_levels = kBatchTopMaxLevels;  // at most this many top levels built first
+    int build_chunk = 0;       // bodies per block of the boxes and the insertions; 0: batch_chunk's rule
+    int top_levels = kBatchTopMaxLevels;  // at most this many top levels built before insertions
 };
 // advance = false leaves out the collision update and the flip: the tree
 // stages and the direct sums as a step runs them (the direct sums beside the
@@ -371,6 +404,8 @@ struct TreeShape {
 cudaError_t launch_batch_step(const BatchTables &t, int method, int comp, int quad, int direct_variant,
                               const TreeShape &shape, int sm_count, cudaStream_t st, const StepFork *fork,
                               int *launches, bool advance = true);
+// boxes, trees, sums and sorts of a batch (k_batch_build.cu)
+cudaError_t launch_batch_build(const BatchTables &t, int quadrupole, int sm_count, cudaStream_t st, int *launches);
 // clears the status word and work counters of every system (once per call)
 cudaError_t launch_batch_clear(const BatchTables &t, cudaStream_t st);
 

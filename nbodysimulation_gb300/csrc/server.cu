@@ -104,7 +104,7 @@ struct nb_server {
     int *d_pref[2] = {nullptr, nullptr}, *h_pref[2] = {nullptr, nullptr};
     int *d_work = nullptr;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
-    int exec_totals[2][kBatchSpaces + 1] = {};
+    int exec_totals[2][kBatchTotals + 1] = {};
     cudaEvent_t round_ev[2] = {nullptr, nullptr};
 
     std::string err;
@@ -137,6 +137,7 @@ static int64_t job_bytes(nb_server *s, Job &j) {
     m.n = j.n;
     m.tree = j.cfg.algo_config == NB_BARNES_HUT;
     m.quad = m.tree && s->cfg.multipole == NB_MULTIPOLE_QUADRUPOLE;
+    m.ref = j.cfg.tree_semantics == NB_TREE_REFERENCE;
     m.cap = m.tree ? (j.cfg.cell_capacity > 0 ? j.cfg.cell_capacity : sysmem_default_capacity(j.n)) : 0;
     return (int64_t)(sysmem_layout(m, nullptr) + kCtrlBytes);
 }
@@ -288,7 +289,7 @@ static cudaError_t launch_round(nb_server *s, std::vector<JobP> &run, int steps,
                                 std::deque<Delivery> &outs, std::vector<JobP> &finished) {
     const int ns = (int)run.size();
     for (int k = 0; k < ns; ++k) s->h_sys[buf][k] = run[k]->desc;
-    int totals[kBatchSpaces];
+    int totals[kBatchTotals];
     batch_prefixes(s->h_sys[buf], ns, batch_direct_block_bodies(s->variant), s->h_pref[buf], totals);
     cudaError_t e;
     if ((e = cudaMemcpyAsync(s->d_sys[buf], s->h_sys[buf], sizeof(SysDesc) * ns, cudaMemcpyHostToDevice,
@@ -297,7 +298,8 @@ static cudaError_t launch_round(nb_server *s, std::vector<JobP> &run, int steps,
     if ((e = cudaMemcpyAsync(s->d_pref[buf], s->h_pref[buf], sizeof(int) * batch_prefix_ints(ns),
                              cudaMemcpyHostToDevice, s->compute)) != cudaSuccess)
         return e;
-    const int key[kBatchSpaces + 1] = {ns, totals[0], totals[1], totals[2], totals[3], totals[4]};
+    int key[kBatchTotals + 1] = {ns};
+    memcpy(key + 1, totals, sizeof(totals));
     if (!s->exec[buf] || memcmp(key, s->exec_totals[buf], sizeof(key)) != 0) {
         // the kernels read everything else from the device tables; only the
         // totals (grid sizes) and the system count live in the graph
@@ -556,7 +558,9 @@ nb_status nb_server_create(const nb_server_config *c, nb_job_fn fn, void *user, 
               cudaStreamCreateWithFlags(&s->fork.aux, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&s->fork.fork, cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&s->fork.join, cudaEventDisableTiming) == cudaSuccess &&
-              cudaMalloc(&s->d_work, sizeof(int)) == cudaSuccess;
+              cudaMalloc(&s->d_work, sizeof(int) * kBatchWorkInts) == cudaSuccess &&
+              cudaMemset(s->d_work, 0, sizeof(int) * kBatchWorkInts) == cudaSuccess &&
+              cudaDeviceSynchronize() == cudaSuccess;
     for (int b = 0; b < 2 && ok; ++b) {
         ok = cudaMalloc(&s->d_sys[b], sizeof(SysDesc) * ns) == cudaSuccess &&
              cudaMalloc(&s->d_pref[b], sizeof(int) * batch_prefix_device_ints((int)ns)) == cudaSuccess &&

@@ -12,7 +12,7 @@ namespace nbgb {
 
 struct SysMem {
     int n = 0, cap = 0;
-    bool tree = false, quad = false;
+    bool tree = false, quad = false, ref = false;  // ref: the reference's tree semantics
     float4 *body[2] = {nullptr, nullptr};
     float4 *vel = nullptr, *acc = nullptr, *part = nullptr;
     int *parent = nullptr, *child = nullptr, *wchild = nullptr, *count = nullptr, *start = nullptr,
@@ -21,6 +21,7 @@ struct SysMem {
     float2 *wqb = nullptr;
     int *top = nullptr;  // top-level tables (batch_top_levels_for): counts, then start entries
     int top_levels = 0;
+    int *build = nullptr;  // scratch of the build from sorted paths (batch_build_ints)
     Ctrl *ctrl = nullptr;
 };
 
@@ -70,6 +71,7 @@ inline size_t sysmem_layout(SysMem &m, char *base) {
         }
         m.top_levels = batch_top_levels_for(m.n);
         if (m.top_levels) take(m.top, (size_t)2 << (3 * m.top_levels));
+        take(m.build, batch_build_ints(m.n, m.ref));
     }
     return sysmem_align(off);
 }
@@ -126,6 +128,7 @@ inline SysDesc sysmem_desc(const SysMem &m, const nb_config &c, float dt) {
     v.wqb = m.wqb;
     v.ctrl = m.ctrl;
     sysdesc_set_top(d, m, c.tree_semantics == NB_TREE_REFERENCE, kBatchTopMaxLevels);
+    d.build = BuildTables{m.build, batch_build_levels(m.n, m.ref)};
     d.body[0] = m.body[0];
     d.body[1] = m.body[1];
     StepParams &p = d.p;
@@ -144,9 +147,10 @@ inline SysDesc sysmem_desc(const SysMem &m, const nb_config &c, float dt) {
     return d;
 }
 
-// The batch-wide index spaces: bbox/build chunks, cell slots, force warp
-// groups, direct-sum blocks, collision blocks.
-constexpr int kBatchSpaces = 5;
+// The batch-wide index spaces: box / insertion chunks, force warp groups,
+// direct-sum blocks, collision blocks, tiles of the sorted builds.
+// (The last total has no table: trees that always take the insertions.)
+constexpr int kBatchSpaces = 5, kBatchTotals = kBatchSpaces + 1;
 // host-written prefix tables, nsys + 1 entries each
 inline size_t batch_prefix_ints(int nsys) { return (size_t)kBatchSpaces * (size_t)(nsys + 1); }
 // on the device they are followed by the device-written table of used cells
@@ -154,60 +158,64 @@ inline size_t batch_prefix_device_ints(int nsys) { return (size_t)(kBatchSpaces 
 
 // Where every system's work starts in the batch-wide index spaces (direct-sum
 // blocks of `direct_block` bodies, collision blocks of kCollideBlockBodies,
-// bbox / build chunks of chunk_override bodies when > 0, else batch_chunk's).
+// chunks of chunk_override bodies when > 0, else batch_chunk's).
 // Fills the *_begin fields of sys, the prefix tables (nsys + 1 entries each,
 // back to back in pref) and their totals.
-inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, int totals[kBatchSpaces],
+inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, int totals[kBatchTotals],
                            int chunk_override = 0) {
-    int *chunk = pref, *cell = pref + (nsys + 1), *group = pref + 2 * (nsys + 1), *dblock = pref + 3 * (nsys + 1),
-        *cblock = pref + 4 * (nsys + 1);
-    chunk[0] = cell[0] = group[0] = dblock[0] = cblock[0] = 0;
+    int *chunk = pref, *group = pref + (nsys + 1), *dblock = pref + 2 * (nsys + 1), *cblock = pref + 3 * (nsys + 1),
+        *tile = pref + 4 * (nsys + 1);
+    chunk[0] = group[0] = dblock[0] = cblock[0] = tile[0] = 0;
     long long tree_bodies = 0;
     for (int k = 0; k < nsys; ++k)
         if (sys[k].active && sys[k].kind == kSysBH) tree_bodies += sys[k].v.n;
-    int body = 0;
+    int body = 0, large_refs = 0;
     for (int k = 0; k < nsys; ++k) {
         SysDesc &d = sys[k];
         const int n = d.v.n;
         d.body_begin = body;
         d.chunk_begin = chunk[k];
-        d.cell_begin = cell[k];
         d.group_begin = group[k];
         d.dblock_begin = dblock[k];
         d.cblock_begin = cblock[k];
+        d.tile_begin = tile[k];
         const bool bh = d.active && d.kind == kSysBH, direct = d.active && d.kind == kSysDirect;
+        const bool large_ref = bh && d.p.tree_ref && n > kRefPathBodies;
         d.chunk = chunk_override > 0 ? chunk_override : batch_chunk(n, tree_bodies);
         chunk[k + 1] = chunk[k] + (bh ? (n + d.chunk - 1) / d.chunk : 0);
-        cell[k + 1] = cell[k] + (bh ? d.v.cap + 1 : 0);
         group[k + 1] = group[k] + (bh ? (n + 31) / 32 : 0);
         dblock[k + 1] = dblock[k] + (direct ? (n + direct_block - 1) / direct_block : 0);
         cblock[k + 1] = cblock[k] + (d.active && d.collide ? (n + kCollideBlockBodies - 1) / kCollideBlockBodies : 0);
+        tile[k + 1] = tile[k] + (bh && !large_ref ? (n + kBuildTileBodies - 1) / kBuildTileBodies : 0);
+        large_refs += large_ref;
         body += n;
     }
     totals[0] = chunk[nsys];
-    totals[1] = cell[nsys];
-    totals[2] = group[nsys];
-    totals[3] = dblock[nsys];
-    totals[4] = cblock[nsys];
+    totals[1] = group[nsys];
+    totals[2] = dblock[nsys];
+    totals[3] = cblock[nsys];
+    totals[4] = tile[nsys];
+    totals[5] = large_refs;
 }
 
 // d_pref holds the prefix tables of batch_prefixes followed by room for the
 // device-written table of used cells: batch_prefix_device_ints(nsys) ints.
-inline BatchTables batch_tables(const SysDesc *d_sys, int nsys, int *d_pref, const int totals[kBatchSpaces],
+inline BatchTables batch_tables(const SysDesc *d_sys, int nsys, int *d_pref, const int totals[kBatchTotals],
                                 int *work) {
     BatchTables t{};
     t.sys = d_sys;
     t.nsys = nsys;
     t.chunk_prefix = d_pref;
-    t.cell_prefix = d_pref + (nsys + 1);
-    t.group_prefix = d_pref + 2 * (nsys + 1);
-    t.dblock_prefix = d_pref + 3 * (nsys + 1);
-    t.cblock_prefix = d_pref + 4 * (nsys + 1);
+    t.group_prefix = d_pref + (nsys + 1);
+    t.dblock_prefix = d_pref + 2 * (nsys + 1);
+    t.cblock_prefix = d_pref + 3 * (nsys + 1);
+    t.tile_prefix = d_pref + 4 * (nsys + 1);
     t.chunks = totals[0];
-    t.cells = totals[1];
-    t.groups = totals[2];
-    t.dblocks = totals[3];
-    t.cblocks = totals[4];
+    t.groups = totals[1];
+    t.dblocks = totals[2];
+    t.cblocks = totals[3];
+    t.tiles = totals[4];
+    t.large_refs = totals[5];
     t.work = work;
     t.used_prefix = d_pref + kBatchSpaces * (nsys + 1);
     return t;
