@@ -6,8 +6,18 @@
 
 namespace nbgb {
 
-template <int kMethod, bool kComp, bool kEpsZero, bool kQuad>
-__global__ void __launch_bounds__(kForceThreads, 8) k_force(DevSim s, StepParams p) {
+// kBlocks: resident blocks per SM the registers allow.  Eight (128 registers),
+// or nine (96) where the groups fill the GPU more than twice over: the extra
+// warps then hide more of the walk than its tighter schedule costs.  With
+// quadrupoles and without compensation they do not (GB300, the walk in ms,
+// eight / nine blocks: monopoles, ball, 6,007 bodies 0.0635 / 0.0657, 131,072
+// 0.207 / 0.207, 200,000 0.290 / 0.287, 262,144 0.365 / 0.353, 1,000,000 1.303 /
+// 1.246; quadrupoles compensated, 200,000 0.522 / 0.515, 4,194,304 11.78 / 11.57;
+// quadrupoles, 1,000,000 1.305 / 1.310; ten blocks 0.362 and 11.99 where nine
+// take 0.353 and 11.57).
+constexpr int kFewGroups = 8, kManyGroups = 9;
+template <int kMethod, bool kComp, bool kEpsZero, bool kQuad, int kBlocks>
+__global__ void __launch_bounds__(kForceThreads, kBlocks) k_force(DevSim s, StepParams p) {
     wait_for_previous();
     __shared__ float s_dq[kMaxDepth];
     __shared__ WarpLists<kQuad> s_lists[kForceWarps];
@@ -42,21 +52,27 @@ __global__ void __launch_bounds__(kForceThreads, 8) k_force(DevSim s, StepParams
     }
 }
 
-template <int kMethod, bool kComp, bool kQuad>
-static cudaError_t launch_force_t(const DevSim &s, const StepParams &p, int sm_count, cudaStream_t st) {
+template <int kMethod, bool kComp, bool kQuad, int kBlocks>
+static cudaError_t launch_force_b(const DevSim &s, const StepParams &p, int sm_count, cudaStream_t st) {
     const bool ez = !(p.eps > 0.0f);
-    const void *fn = ez ? (const void *)k_force<kMethod, kComp, true, kQuad>
-                        : (const void *)k_force<kMethod, kComp, false, kQuad>;
+    const auto kernel = ez ? k_force<kMethod, kComp, true, kQuad, kBlocks> : k_force<kMethod, kComp, false, kQuad, kBlocks>;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kForceThreads, 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kForceThreads, 0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     int blocks = per_sm * sm_count;
     const int need = ((s.n + 31) / 32 + kForceWarps - 1) / kForceWarps;
     if (blocks > need) blocks = need > 0 ? need : 1;
-    const auto kernel = ez ? k_force<kMethod, kComp, true, kQuad> : k_force<kMethod, kComp, false, kQuad>;
     if (blocks == per_sm * sm_count) return launch_next(kernel, blocks, kForceThreads, st, s, p);
     kernel<<<blocks, kForceThreads, 0, st>>>(s, p);  // a part of the GPU: spread evenly (launch.cuh)
     return cudaGetLastError();
+}
+
+template <int kMethod, bool kComp, bool kQuad>
+static cudaError_t launch_force_t(const DevSim &s, const StepParams &p, int sm_count, cudaStream_t st) {
+    if constexpr (kQuad && !kComp) return launch_force_b<kMethod, kComp, kQuad, kFewGroups>(s, p, sm_count, st);
+    const bool many = (s.n + 31) / 32 >= 2 * kFewGroups * kForceWarps * sm_count;
+    return many ? launch_force_b<kMethod, kComp, kQuad, kManyGroups>(s, p, sm_count, st)
+                : launch_force_b<kMethod, kComp, kQuad, kFewGroups>(s, p, sm_count, st);
 }
 
 template <int kMethod>

@@ -41,3 +41,25 @@ def test_walk_edges(gpu, oracle, layout, n, quad, comp):
     acc = sim.get_state()[2].astype(np.float64)
     scale = np.sqrt(np.mean(np.sum(acc_o.astype(np.float64) ** 2, axis=1)))
     assert np.max(np.linalg.norm(acc - acc_o, axis=1)) < 2e-5 * scale
+
+
+@pytest.mark.parametrize("quad,comp", [(0, 0), (0, 1), (1, 1)])
+def test_walk_of_many_groups(gpu, quad, comp):
+    """The walk with more warps per SM, which systems take whose groups fill the
+    GPU twice over (152 SMs: 4,864 groups): bit for bit the batched walk, which
+    has one form."""
+    nb = gpu
+    sizes = (155616, 155617, 200000)
+    cfgs = [nb.default_config(num_of_bodies=n, algo_config=nb.BARNES_HUT, theta=0.8, epsilon=0.01,
+                              gravitational_constant=1.0, multipole=quad, precision=comp) for n in sizes]
+    states = [bodies("normal", n) for n in sizes]
+    with nb.Batch(cfgs) as b:
+        for k, (pos, mass) in enumerate(states):
+            b.set_state(k, pos, mass)
+        b.step(1e-3, 1)
+        for k, (pos, mass) in enumerate(states):
+            with nb.Simulation(cfgs[k]) as sim:
+                sim.set_state(pos, mass)
+                sim.step(1e-3, 1)
+                for one, batched in zip(sim.get_state(), b.get_state(k)):
+                    np.testing.assert_array_equal(one, batched)
