@@ -48,7 +48,6 @@ struct nb_sim {
     float4 *wpm = nullptr, *cell_pm = nullptr;
     float4 *cell_q = nullptr, *wqa = nullptr;
     float2 *wqb = nullptr;
-    int *build_mem = nullptr;  // counters and tables of the build from sorted paths
     BuildScratch build{};
     bool quad = false;
     DirectPlan plan{1, 1};    // direct sum: how it is spread over the GPU
@@ -120,8 +119,8 @@ static DevSim dev_view(const nb_sim *s) {
 static void free_tree(nb_sim *s) {
     cudaFree(s->parent); cudaFree(s->child); cudaFree(s->wchild); cudaFree(s->wpm); cudaFree(s->cell_pm);
     cudaFree(s->count); cudaFree(s->start); cudaFree(s->arrive);
-    cudaFree(s->cell_q); cudaFree(s->wqa); cudaFree(s->wqb); cudaFree(s->build_mem);
-    s->parent = s->child = s->wchild = s->count = s->start = s->arrive = s->build_mem = nullptr;
+    cudaFree(s->cell_q); cudaFree(s->wqa); cudaFree(s->wqb);
+    s->parent = s->child = s->wchild = s->count = s->start = s->arrive = nullptr;
     s->wpm = s->cell_pm = s->cell_q = s->wqa = nullptr;
     s->wqb = nullptr;
 }
@@ -142,13 +141,6 @@ static nb_status alloc_tree(nb_sim *s, int cap) {
         NB_CUDA(s, dalloc(&s->cell_q, cells * 2));
         NB_CUDA(s, dalloc(&s->wqa, cells * 8));
         NB_CUDA(s, dalloc(&s->wqb, cells * 8));
-    }
-    if (s->cfg.tree_semantics != NB_TREE_REFERENCE) {
-        // the paths and places lie in the transfer staging, which no step uses
-        const size_t ints = build_scratch_ints(s->n, s->sm_count);
-        NB_CUDA(s, dalloc(&s->build_mem, ints));
-        NB_CUDA(s, cudaMemset(s->build_mem, 0, sizeof(int) * ints));
-        s->build = build_scratch(s->n, s->sm_count, s->build_mem, s->part, s->stage3);
     }
     return NB_OK;
 }
@@ -262,9 +254,12 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     s->tree = cfg->algo_config == NB_BARNES_HUT;
     if (!s->tree) s->plan = direct_plan(s->n, s->sm_count, direct_slices_limit(s->n));
     const size_t part = n * (size_t)std::max(2, s->plan.slices);
+    // counters and tables that are zero before the first step lie behind the sums
+    size_t tables = s->tree ? 0 : (n + 31) / 32;
+    if (s->tree && cfg->tree_semantics != NB_TREE_REFERENCE) tables = build_scratch_ints(s->n, s->sm_count);
     bool ok = dalloc(&s->body[0], n) == cudaSuccess && dalloc(&s->body[1], n) == cudaSuccess &&
               dalloc(&s->vel, n) == cudaSuccess && dalloc(&s->acc, n) == cudaSuccess &&
-              dalloc(&s->part, part + (s->tree ? 0 : (n + 127) / 128)) == cudaSuccess &&
+              dalloc(&s->part, part + (tables + 3) / 4) == cudaSuccess &&
               dalloc(&s->ctrl, 1) == cudaSuccess;
     if (!ok) return cleanup(NB_ERR_OUT_OF_MEMORY);
     // the transfer staging lies behind the first n of the sums: no step runs
@@ -275,10 +270,11 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     cudaMemset(s->ctrl, 0, sizeof(Ctrl));
     cudaMemset(s->vel, 0, sizeof(float4) * n);
     cudaMemset(s->acc, 0, sizeof(float4) * n);
-    if (!s->tree) {  // the counters lie behind the slices' sums
-        s->arrived = reinterpret_cast<int *>(s->part + part);
-        cudaMemset(s->arrived, 0, sizeof(int) * ((n + 31) / 32));
-    }
+    int *zeroed = reinterpret_cast<int *>(s->part + part);
+    if (tables) cudaMemset(zeroed, 0, sizeof(int) * tables);
+    if (!s->tree) s->arrived = zeroed;
+    // the build's paths and places lie in the transfer staging, which no step uses
+    else if (tables) s->build = build_scratch(s->n, s->sm_count, zeroed, s->part, s->stage3);
     s->quad = cfg->multipole == NB_MULTIPOLE_QUADRUPOLE;
     if (s->tree) {
         int cap = cfg->cell_capacity > 0 ? cfg->cell_capacity : default_capacity(s->n, s->sm_count);
