@@ -195,8 +195,9 @@ __device__ __forceinline__ void cells_tile(const DevSim &s, const BuildScratch &
                 int4 *row = reinterpret_cast<int4 *>(&s.child[k * 8]);
                 row[0] = row[1] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
                 s.arrive[k] = 0;
-                s.start[k] = 1;  // completed by k_top
-                b.top[atomicAdd(&b.ctl[kBuildTop], 1)] = cell;
+                const int at = atomicAdd(&b.ctl[kBuildTop], 1);  // completed by k_top
+                b.top[at] = cell;
+                s.start[k] = 1 + at;
             }
         }
     }
@@ -417,16 +418,15 @@ __device__ __forceinline__ void link_tile(const DevSim &s, const BuildScratch &b
 // completed by whichever eight lanes bring its arrival counter to the number
 // of its children.
 // ---------------------------------------------------------------------------
-// cell `cell` by eight lanes: lane j holds octant slot j's child ch (mask: the
-// slots that have one), complete in memory
+// The data of child ch (a body or a complete cell).
 template <bool kQuad>
-__device__ __forceinline__ void top_cell(const DevSim &s, int cell, int ch, unsigned mask, unsigned group, int j) {
-    const int n = s.n, c = cell - n;
-    const bool have = ch >= 0;
-    float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    int cnt = 1;
-    float q[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    if (have && ch < n) p = s.body_cur[ch];
+__device__ __forceinline__ void load_child(const DevSim &s, int ch, float4 &p, int &cnt, float (&q)[6]) {
+    const int n = s.n;
+    p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    cnt = 1;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) q[k] = 0.0f;
+    if (ch >= 0 && ch < n) p = s.body_cur[ch];
     if (ch >= n) {
         p = __ldcg(&s.cell_pm[ch - n]);
         cnt = __ldcg(&s.count[ch - n]);
@@ -440,6 +440,15 @@ __device__ __forceinline__ void top_cell(const DevSim &s, int cell, int ch, unsi
             q[5] = ob.y;
         }
     }
+}
+
+// cell `cell` by eight lanes: lane j holds octant slot j's child ch and its data
+// (mask: the slots that have one); q: the child's moments in, the cell's out
+template <bool kQuad>
+__device__ __forceinline__ CellSums finish_cell(const DevSim &s, int cell, int ch, unsigned mask, unsigned group, int j,
+                                                const float4 p, int cnt, float (&q)[6]) {
+    const int c = cell - s.n;
+    const bool have = ch >= 0;
     // children first, in slot order, then empty places
     const int rank = __popc(mask & ((1u << j) - 1u));
     const int at = c * 8 + (have ? rank : __popc(mask) + j - rank);
@@ -459,13 +468,101 @@ __device__ __forceinline__ void top_cell(const DevSim &s, int cell, int ch, unsi
             s.cell_q[2 * c + 1] = make_float4(q[4], q[5], 0.0f, 0.0f);
         }
     }
+    return sums;
+}
+
+// A short list in one block: every cell's row in shared memory, where a finished
+// cell is entered, so a level costs the sums and no round trips to L2 (which
+// take 2.5 us, six or seven levels deep).  Longer lists keep one block too long.
+// The sums of both kernels, by the arrival counters in memory / here (GB300, us):
+// monopoles, 3,000 bodies 37 / 27, 6,007 38 / 31, 12,000 40 / 34, 20,000 (340
+// cells) 41 / 41; quadrupoles, 3,000 bodies 39 / 33, 12,000 (190 cells) 48 / 51.
+constexpr int kTopThreads = 512;
+constexpr int kTopSharedBodies = 1 << 15;  // beyond, a list is longer anyhow (20 cells per 1,024 bodies)
+template <bool kQuad>
+constexpr int kTopShared = kQuad ? 128 : 256;
+template <bool kQuad>
+struct TopShared {
+    float4 pm[kTopShared<kQuad>][8];
+    int cnt[kTopShared<kQuad>][8], id[kTopShared<kQuad>][8];
+    float q[kQuad ? kTopShared<kQuad> : 1][6][8];
+    int cell[kTopShared<kQuad>];     // ~cell: all children were complete before this kernel
+    int up[kTopShared<kQuad>];       // 8 * place of the parent + slot there
+    int pending[kTopShared<kQuad>];  // children still to come
+};
+template <bool kQuad>
+__device__ __forceinline__ void top_cells_shared(const DevSim &s, const BuildScratch &b, int cells,
+                                                 TopShared<kQuad> &sh) {
+    const int n = s.n, j = threadIdx.x & 7, groups = blockDim.x >> 3;
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    // all of a group's cells at once: three trips to L2 in a row
+    constexpr int kRounds = kTopShared<kQuad> * 8 / kTopThreads;
+    int cell[kRounds], ch[kRounds], at[kRounds];  // at: 1 + the child's place in the list
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int k = (threadIdx.x >> 3) + r * groups;
+        cell[r] = k < cells ? b.top[k] : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) ch[r] = cell[r] >= 0 ? s.child[(cell[r] - n) * 8 + j] : kEmpty;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) at[r] = ch[r] >= n ? s.start[ch[r] - n] : 0;
+    float4 p[kRounds];
+    int cnt[kRounds];
+    float q[kRounds][6];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) load_child<kQuad>(s, at[r] > 0 ? kEmpty : ch[r], p[r], cnt[r], q[r]);
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int k = (threadIdx.x >> 3) + r * groups;
+        if (cell[r] < 0) break;
+        sh.pm[k][j] = p[r];
+        sh.cnt[k][j] = cnt[r];
+        sh.id[k][j] = ch[r];
+        if constexpr (kQuad)
+            for (int x = 0; x < 6; ++x) sh.q[k][x][j] = q[r][x];
+        if (at[r] > 0) sh.up[at[r] - 1] = 8 * k + j;
+        const int open = __popc(__ballot_sync(group, at[r] > 0));
+        if (j == 0) {
+            sh.cell[k] = open ? cell[r] : ~cell[r];
+            sh.pending[k] = open;
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x >> 3; k < cells; k += groups) {
+        if (sh.cell[k] >= 0) continue;
+        for (int c = k;;) {
+            const int cell = c == k ? ~sh.cell[c] : sh.cell[c], ch = sh.id[c][j];
+            const unsigned mask = (__ballot_sync(group, ch >= 0) >> (threadIdx.x & 24)) & 0xffu;
+            float q[6];
+            if constexpr (kQuad)
+#pragma unroll
+                for (int x = 0; x < 6; ++x) q[x] = sh.q[c][x][j];
+            const CellSums sums = finish_cell<kQuad>(s, cell, ch, mask, group, j, sh.pm[c][j], sh.cnt[c][j], q);
+            if (c == 0) break;  // the root
+            const int up = sh.up[c], parent = up >> 3, slot = up & 7;
+            int left = 0;
+            if (j == 0) {
+                sh.pm[parent][slot] = make_float4(sums.X, sums.Y, sums.Z, sums.M);
+                sh.cnt[parent][slot] = sums.cnt;
+                if constexpr (kQuad)
+#pragma unroll
+                    for (int x = 0; x < 6; ++x) sh.q[parent][x][slot] = q[x];
+                __threadfence_block();
+                left = atomicSub(&sh.pending[parent], 1);
+                __threadfence_block();
+            }
+            if (__shfl_sync(group, left, 0, 8) != 1) break;
+            __syncwarp(group);
+            c = parent;
+        }
+    }
 }
 
 // cells first, first + stride, .. of the list, eight lanes each
 template <bool kQuad>
-__device__ __forceinline__ void top_cells(const DevSim &s, const BuildScratch &b, int first, int stride) {
+__device__ __forceinline__ void top_cells(const DevSim &s, const BuildScratch &b, int cells, int first, int stride) {
     const int n = s.n, root = n + s.cap;
-    const int cells = b.ctl[kBuildTop];
     const int j = threadIdx.x & 7;
     const unsigned group = 0xffu << (threadIdx.x & 24);
     for (int k = first; k < cells; k += stride) {
@@ -485,7 +582,11 @@ __device__ __forceinline__ void top_cells(const DevSim &s, const BuildScratch &b
             // the parent's row is on its way while the cell is summed
             const int up = cell == root ? root : s.parent[cell - n];
             const int up_ch = s.child[(up - n) * 8 + j];
-            top_cell<kQuad>(s, cell, ch, mask, group, j);
+            float4 p;
+            int cnt;
+            float q[6];
+            load_child<kQuad>(s, ch, p, cnt, q);
+            finish_cell<kQuad>(s, cell, ch, mask, group, j, p, cnt, q);
             if (cell == root) break;
             cell = up;
             ch = up_ch;

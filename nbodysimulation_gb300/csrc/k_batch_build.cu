@@ -481,13 +481,19 @@ __global__ void __launch_bounds__(kInsertThreads, 1) k_batch_insert(BatchTables 
 }
 
 template <bool kQuad>
-__global__ void __launch_bounds__(kTile) k_batch_top(BatchTables t) {
+__global__ void __launch_bounds__(kTopThreads) k_batch_top(BatchTables t) {
     wait_for_previous();
+    extern __shared__ __align__(16) unsigned char top_smem[];
     const BuildSystem v = build_system(t, blockIdx.x, 1);
     if (left_alone(v.s.ctrl)) return;
-    // an entry of 1,024 bodies has about 20 of a system's cells, a block room for 32
+    const int cells = v.b.ctl[kBuildTop];
+    if (cells <= kTopShared<kQuad>) {
+        if (v.part == 0) top_cells_shared<kQuad>(v.s, v.b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
+        return;
+    }
+    // an entry of 1,024 bodies has about 20 of a system's cells, a block room for 64
     const int entries = (v.s.n + kBuildTileBodies - 1) / kBuildTileBodies;
-    top_cells<kQuad>(v.s, v.b, v.part * (kTile / 8) + (threadIdx.x >> 3), entries * (kTile / 8));
+    top_cells<kQuad>(v.s, v.b, cells, v.part * (kTopThreads / 8) + (threadIdx.x >> 3), entries * (kTopThreads / 8));
 }
 
 cudaError_t launch_batch_build(const BatchTables &t, int quadrupole, int sm_count, cudaStream_t st, int *launches) {
@@ -502,8 +508,10 @@ cudaError_t launch_batch_build(const BatchTables &t, int quadrupole, int sm_coun
         if (e == cudaSuccess) e = launch_next(k_batch_cells, t.tiles, kTile, st, t);
         if (e == cudaSuccess)
             e = launch_next(quadrupole ? k_batch_link<true> : k_batch_link<false>, blocks, kTile, st, t);
-        if (e == cudaSuccess)
-            e = launch_next(quadrupole ? k_batch_top<true> : k_batch_top<false>, t.tiles, kTile, st, t);
+        const auto top = quadrupole ? k_batch_top<true> : k_batch_top<false>;
+        const size_t shared = quadrupole ? sizeof(TopShared<true>) : sizeof(TopShared<false>);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (e == cudaSuccess) e = launch_next_shared(top, t.tiles, kTopThreads, shared, st, t);
         *launches += 6;
     }
     const auto insert = quadrupole ? k_batch_insert<true> : k_batch_insert<false>;

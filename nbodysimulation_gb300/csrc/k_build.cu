@@ -322,15 +322,18 @@ __device__ __forceinline__ bool grid_barrier(Ctrl *c, int *arrived, int target) 
     return ok != 0;
 }
 
-constexpr int kTopThreads = 512;
 template <bool kQuad>
-__global__ void __launch_bounds__(kTopThreads, 1) k_top(DevSim s, BuildScratch b) {
+__global__ void __launch_bounds__(kTopThreads, 1) k_top(DevSim s, BuildScratch b, bool may_share) {
     wait_for_previous();
     Ctrl *ctrl = s.ctrl;
     const int n = s.n, root = n + s.cap;
     const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     if (!ctrl->insert) {  // grid-uniform: only earlier kernels set it
-        if (!read_status(ctrl)) top_cells<kQuad>(s, b, first >> 3, stride >> 3);
+        if (read_status(ctrl)) return;
+        extern __shared__ __align__(16) unsigned char top_smem[];
+        const int cells = b.ctl[kBuildTop];
+        if (!may_share || cells > kTopShared<kQuad>) top_cells<kQuad>(s, b, cells, first >> 3, stride >> 3);
+        else if (blockIdx.x == 0) top_cells_shared<kQuad>(s, b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
         return;
     }
     const int blocks = gridDim.x;
@@ -420,7 +423,14 @@ cudaError_t launch_tree_sums(const DevSim &s, const BuildScratch &b, int quadrup
     const int tiles = (s.n + kTile - 1) / kTile;
     const u64 *path = b.levels ? b.path : b.placed;
     cudaError_t e = launch_next(quadrupole ? k_link<true> : k_link<false>, tiles, kTile, st, s, b, path);
-    if (e == cudaSuccess) e = launch_next(quadrupole ? k_top<true> : k_top<false>, sm_count, kTopThreads, st, s, b);
+    const auto top = quadrupole ? k_top<true> : k_top<false>;
+    // shared memory only where the list may be short: the SMs' split of it would
+    // hold back the walk's blocks
+    const bool may_share = s.n <= kTopSharedBodies;
+    const size_t shared = !may_share ? 0 : quadrupole ? sizeof(TopShared<true>) : sizeof(TopShared<false>);
+    if (e == cudaSuccess && shared)
+        e = cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    if (e == cudaSuccess) e = launch_next_shared(top, sm_count, kTopThreads, shared, st, s, b, may_share);
     return e;
 }
 

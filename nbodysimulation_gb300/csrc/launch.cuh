@@ -23,10 +23,12 @@ __device__ __forceinline__ void wait_for_previous() {
 }
 
 template <class... Params, class... Args>
-cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t st, Args... args) {
+cudaError_t launch_next_shared(void (*kernel)(Params...), dim3 grid, int threads, size_t shared, cudaStream_t st,
+                               Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = shared;
     cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -34,6 +36,10 @@ cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, int threads, cudaS
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t st, Args... args) {
+    return launch_next_shared(kernel, grid, threads, 0, st, args...);
 }
 
 }  // namespace nbgb

@@ -71,3 +71,10 @@ def test_tree_against_oracle(gpu, oracle, kind, n, quad):
     acc = oracle.bh_step_forces(pos, mass, 0.6, 0.01, 1.0, nodes=cap, quadrupole=bool(quad))[0]
     scale = np.sqrt(np.mean(np.sum(acc.astype(np.float64) ** 2, axis=1)))
     assert np.max(np.linalg.norm(sim.get_state()[2] - acc.astype(np.float64), axis=1)) <= 2e-5 * scale
+
+
+@pytest.mark.parametrize("n", [5000, 6500, 11000, 12500, 14000, 32768, 32769])
+@pytest.mark.parametrize("quad", [0, 1])
+def test_lists_around_the_one_block_form(gpu, oracle, n, quad):
+    """Trees whose cells over a tile's edge are about as many as one block takes."""
+    test_tree_against_oracle(gpu, oracle, "ball", n, quad)
