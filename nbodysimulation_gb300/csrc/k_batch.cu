@@ -38,10 +38,10 @@ struct BatchForceWarp {
 };
 constexpr int kBatchForceMaxWarps = 8;
 
-// Register budget: at most 48 a thread for the monopole walks (ten resident
-// blocks of four warps) and 64 with quadrupoles; neither spills.
-template <int kMethod, bool kComp, bool kQuad>
-__global__ void __launch_bounds__(kBatchForceMaxWarps * 32, 2) k_batch_force(BatchTables t) {
+// Registers: 128 a thread (four blocks of four warps per SM), or 96 (five blocks)
+// where monopole groups fill the GPU (kMany, launch_batch_force_t).
+template <int kMethod, bool kComp, bool kQuad, bool kMany>
+__global__ void __maxnreg__(kMany ? 96 : 128) k_batch_force(BatchTables t) {
     extern __shared__ __align__(16) unsigned char force_smem[];
     BatchForceWarp<kQuad> &me = reinterpret_cast<BatchForceWarp<kQuad> *>(force_smem)[threadIdx.x >> 5];
     float *const s_dq_w = me.dq;
@@ -193,14 +193,14 @@ static cudaError_t launch_direct_variant(const BatchTables &t, int variant, cuda
     return cudaGetLastError();
 }
 
-template <int kMethod, bool kComp, bool kQuad>
-static cudaError_t launch_batch_force_t(const BatchTables &t, const TreeShape &shape, int sm_count,
+template <int kMethod, bool kComp, bool kQuad, bool kMany>
+static cudaError_t launch_batch_force_b(const BatchTables &t, const TreeShape &shape, int sm_count,
                                         cudaStream_t st) {
     int warps = shape.force_warps;
     if (warps < 1 || warps > kBatchForceMaxWarps) warps = kForceWarps;
     const int threads = warps * 32;
     const size_t smem = sizeof(BatchForceWarp<kQuad>) * (size_t)warps;
-    const void *fn = (const void *)k_batch_force<kMethod, kComp, kQuad>;
+    const void *fn = (const void *)k_batch_force<kMethod, kComp, kQuad, kMany>;
     if (smem > 48 * 1024) {  // beyond the default dynamic shared memory of a block: opt in
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -212,8 +212,20 @@ static cudaError_t launch_batch_force_t(const BatchTables &t, const TreeShape &s
     const int need = (t.groups + warps - 1) / warps;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
-    k_batch_force<kMethod, kComp, kQuad><<<(int)blocks, threads, smem, st>>>(t);
+    k_batch_force<kMethod, kComp, kQuad, kMany><<<(int)blocks, threads, smem, st>>>(t);
     return cudaGetLastError();
+}
+
+// Sixteen warps per SM or more of groups: 96 registers (steps of monopole trees,
+// GB300, ms, 128 / 96 registers: 18 of 20,000 bodies, 11,250 groups, 0.416 / 0.409;
+// 512 of 3,000 1.20 / 1.15; 256 of 60,000 15.08 / 14.52; but 32 of 1,500, 1,500
+// groups, 0.105 / 0.107 and 4 of 10,000 0.128 / 0.131).
+template <int kMethod, bool kComp, bool kQuad>
+static cudaError_t launch_batch_force_t(const BatchTables &t, const TreeShape &shape, int sm_count,
+                                        cudaStream_t st) {
+    if constexpr (!kQuad)
+        if (t.groups >= 16 * sm_count) return launch_batch_force_b<kMethod, kComp, kQuad, true>(t, shape, sm_count, st);
+    return launch_batch_force_b<kMethod, kComp, kQuad, false>(t, shape, sm_count, st);
 }
 
 template <int kMethod>
