@@ -22,8 +22,8 @@ The same line carries more measurements, each with its own timed region
   bh_configs  the plain Barnes-Hut configuration (N = 262,144 unit ball,
            monopole, FP32) and the 4M workload at theta 0.3 and 0.8, with
            their FP64-probe accuracy;
-  direct   the TMA-tiled direct sum on N = 262,144 (interactions/s against
-           the FP32-pipe roofline) and the naive kernel on N = 4096;
+  direct   the direct sum (tiled law) on N = 262,144 (interactions/s against
+           the FP32-pipe roofline) and the global law on N = 4096;
   collision  the collision update on the 262,144-body unit ball (pairs/s);
   batched  512 systems, N log-uniform in [1024, 262144], one CUDA graph per
            step, against a loop of plain solves (one handle per system);
@@ -278,15 +278,14 @@ def stage_roofline(stage_ms, n, cells, hbm_gbs, quad=True):
     model = {
         # body {x,y,z,m} read
         "bbox": 16 * n,
-        # body read; per cell: child row 32 B, parent/arrive/start 12 B written
-        "build": 16 * n + 44 * cells,
-        # per cell: child row read; every body and cell {x,y,z,m} read once;
-        # compacted row 32, packed line 128, centre/mass 16, count 4 written,
+        # paths, sort and cells: body read, its path and sorted index written
+        "build": 16 * n + 12 * n,
+        # path, sorted index and body read; per cell: child row 32, compacted
+        # row 32, packed line 128, centre/mass 16, counts and starts 8 written,
         # with quadrupoles cell moments 32 and packed moments 192 more
-        "summarize": 32 * cells + 16 * (n + cells) + (180 + (224 if quad else 0)) * cells,
-        # per cell: compacted row 32 + child counts 4 read, start 4 written;
-        # sorted index 4 per body written
-        "sort": 40 * cells + 4 * n,
+        "summarize": 28 * n + (216 + (224 if quad else 0)) * cells,
+        # part of the build
+        "sort": 0,
         "force": 84 * n + (352 if quad else 160) * cells,
     }
     out = {}
@@ -559,7 +558,7 @@ def run_bh_configs(args, dist: Dist):
 
 
 # ---------------------------------------------------------------------------
-# direct sum: tiled all-pairs on N = 262,144 and the naive kernel on N = 4096
+# direct sum: the tiled law on N = 262,144 and the global law on N = 4096
 # ---------------------------------------------------------------------------
 DIRECT = dict(n=262144, n_global=4096, eps=0.01, eps_global=0.05, dt=1e-3, G=1.0, steps=50)
 DIRECT_FP32_OPS = 12  # per pair: 3 FADD, 3 FFMA (d^2), 3 FMUL (r^3 m), 3 FFMA (accumulate); +1 MUFU rsqrt
@@ -585,7 +584,7 @@ def direct_leg(nb, dev, n, tiled, eps, steps, warmup, sm_count, sm_mhz):
     inter = float(n) * n * steps
     ips = inter / (ms / 1e3)
     peak_ips = FP32_LANES_PER_SM * sm_count * sm_mhz * 1e6 / DIRECT_FP32_OPS
-    return {"kernel": "k_direct_tiled" if tiled else "k_direct_global", "n_bodies": n, "eps": eps,
+    return {"kernel": "k_direct", "law": "tiled" if tiled else "global", "n_bodies": n, "eps": eps,
             "steps": steps, "ms_per_step": ms / steps, "body_updates_per_s": n * steps / (ms / 1e3),
             "interactions_per_s": ips, "fp32_gops": ips * DIRECT_FP32_OPS / 1e9,
             "roofline": {"bound": "fp32", "achieved": ips * DIRECT_FP32_OPS / 1e12,

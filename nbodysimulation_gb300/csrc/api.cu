@@ -256,7 +256,8 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     const size_t part = n * (size_t)std::max(2, s->plan.slices);
     // counters and tables that are zero before the first step lie behind the sums
     size_t tables = s->tree ? 0 : (n + 31) / 32;
-    if (s->tree && cfg->tree_semantics != NB_TREE_REFERENCE) tables = build_scratch_ints(s->n, s->sm_count);
+    const int ref = cfg->tree_semantics == NB_TREE_REFERENCE;
+    if (s->tree && !(ref && s->n > kRefPathBodies)) tables = build_scratch_ints(s->n, s->sm_count);
     bool ok = dalloc(&s->body[0], n) == cudaSuccess && dalloc(&s->body[1], n) == cudaSuccess &&
               dalloc(&s->vel, n) == cudaSuccess && dalloc(&s->acc, n) == cudaSuccess &&
               dalloc(&s->part, part + (tables + 3) / 4) == cudaSuccess &&
@@ -274,7 +275,7 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     if (tables) cudaMemset(zeroed, 0, sizeof(int) * tables);
     if (!s->tree) s->arrived = zeroed;
     // the build's paths and places lie in the transfer staging, which no step uses
-    else if (tables) s->build = build_scratch(s->n, s->sm_count, zeroed, s->part, s->stage3);
+    else if (tables) s->build = build_scratch(s->n, s->sm_count, ref, zeroed, s->part, s->stage3);
     s->quad = cfg->multipole == NB_MULTIPOLE_QUADRUPOLE;
     if (s->tree) {
         int cap = cfg->cell_capacity > 0 ? cfg->cell_capacity : default_capacity(s->n, s->sm_count);
@@ -462,7 +463,7 @@ static nb_status enqueue_step(nb_sim *s, float dt, int timed) {
     if (s->tree) {
         p.eps = c.epsilon;
         mark(0);
-        if (p.tree_ref) {
+        if (p.tree_ref && s->n > kRefPathBodies) {
             NB_CUDA(s, launch_reset(d, st));
             NB_CUDA(s, launch_bbox(d, s->sm_count, st));
             mark(1);

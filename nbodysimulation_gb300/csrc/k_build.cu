@@ -1,5 +1,6 @@
 // k_build.cu -- bounding box, octree, centres of mass and in-order sort of a
-// single system with the cubic-root tree, from sorted octant paths.
+// single system, from sorted octant paths: with the cubic root or, up to
+// kRefPathBodies, the reference's boxes and super-root.
 //
 // Reference stages: boundary_reduce, init, build_tree, saturate_tree and the
 // empty sort (kernels/*.cl).  The octree is a function of the points: a cell
@@ -131,9 +132,10 @@ __global__ void __launch_bounds__(256) k_path(DevSim s, BuildScratch b) {
     if (build_off(s.ctrl)) return;
     float box[6];
     load_box(s.ctrl, box);
-    const GeoCube root = GeoCube::root(box);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x)
-        path_body(s, b, root, i);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
+        if (b.ref) path_body(s, b, RefBox::root(box), i);
+        else path_body(s, b, GeoCube::root(box), i);
+    }
 }
 
 // Exclusive scan of the region counts (a block adds up the totals of the
@@ -346,11 +348,11 @@ __global__ void __launch_bounds__(kTopThreads, 1) k_top(DevSim s, BuildScratch b
     if (!read_status(ctrl)) {
         float box[6];
         load_box(ctrl, box);
-        const GeoCube root_g = GeoCube::root(box);
         const long long cap = tree_spin_cap(ctrl);
         int deep = 0;
         for (int i = first; i < n; i += stride) {
-            const int depth = insert_body<GeoCube, false>(s, root_g, i, cap);
+            const int depth = b.ref ? insert_body<RefBox, true>(s, RefBox::root(box), i, cap)
+                                    : insert_body<GeoCube, false>(s, GeoCube::root(box), i, cap);
             if (depth < 0) break;
             deep = max(deep, depth);
         }
@@ -375,8 +377,9 @@ size_t build_scratch_ints(int n, int sm_count) {
     return kBuildCtl + kScanBlocks + (size_t)6 * 4 * sm_count + build_top_cells(n) + 2 * regions + 4;
 }
 
-BuildScratch build_scratch(int n, int sm_count, int *mem, void *keys16, void *ints12) {
+BuildScratch build_scratch(int n, int sm_count, int ref, int *mem, void *keys16, void *ints12) {
     BuildScratch b{};
+    b.ref = ref;
     b.levels = build_levels(n);
     const size_t regions = (size_t)1 << (3 * b.levels);
     b.ctl = mem;  // 16-byte aligned, as are the tables behind it

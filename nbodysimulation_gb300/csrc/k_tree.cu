@@ -1,6 +1,7 @@
 // k_tree.cu -- bounding box, octree build, centre-of-mass summarisation and
-// in-order sort with the reference's tree semantics (its boxes and super-root;
-// the cubic-root tree is k_build.cu's).
+// in-order sort of large trees with the reference's semantics (its boxes and
+// super-root): beyond kRefPathBodies, where the paths of k_build.cu nearly always
+// leave two bodies together, and the insertions fill the GPU as kernels of their own.
 //
 // Reference stages: boundary_reduce (kernels/boundary_reduce.cl), init
 // (kernels/init.cl), build_tree (kernels/build_tree.cl, build_tree.hcl),

@@ -78,3 +78,33 @@ def test_tree_against_oracle(gpu, oracle, kind, n, quad):
 def test_lists_around_the_one_block_form(gpu, oracle, n, quad):
     """Trees whose cells over a tile's edge are about as many as one block takes."""
     test_tree_against_oracle(gpu, oracle, "ball", n, quad)
+
+
+@pytest.mark.parametrize("kind,n", [("ball", n) for n in (1, 2, 257, 2048, 2049, 20000, 131072, 131073)] +
+                         [("clumps", 3000), ("outlier", 5000), ("close", 700), ("plane", 10007)])
+@pytest.mark.parametrize("quad", [0, 1])
+def test_reference_tree_against_oracle(gpu, oracle, kind, n, quad):
+    """The reference's boxes and super-root, from paths and, beyond 131,072 bodies
+    or where paths do not part them, from insertions."""
+    nb = gpu
+    pos, mass = bodies(kind, n)
+    if kind == "close":  # the reference's boxes part bodies along x and z
+        pos[n // 2] += np.float32(1e-4)
+    sim = bh_sim(nb, pos, mass, 0.6, 0.01, tree=1, quad=quad)
+    for _ in range(2):
+        assert sim.step(0.0, 1, check=False) == 0
+    info = sim.stage_debug(nb.DEBUG_TREE_INFO)
+    cap = int(info[1])
+    t = oracle.tree_build(oracle.SEM_REFERENCE, pos, mass, sim.stage_debug(nb.DEBUG_BBOX), cap)
+    assert t.status == 0 and int(info[2]) == t.bottom
+    children = sim.stage_debug(nb.DEBUG_CHILDREN)
+    pg, dg, fg = oracle.tree_paths(children, n, n + cap)
+    po, do, fo = oracle.tree_paths(t.children, n, t.root)
+    assert fg == n and fo == n and np.array_equal(dg, do) and np.array_equal(pg, po)
+    octant = t.children.copy()
+    assert oracle.saturate(t) == 0
+    tg = cell_table(children, sim.stage_debug(nb.DEBUG_NODE_MASS), sim.stage_debug(nb.DEBUG_NODE_POS),
+                    sim.stage_debug(nb.DEBUG_BODY_COUNT), n, n + cap)
+    assert tg == cell_table(octant, t.mass, t.pos, t.body_count, n, t.root)
+    order, k = oracle.sort_bodies(t.children, n, t.root)
+    assert k == n and np.array_equal(sim.stage_debug(nb.DEBUG_SORTED), order)
