@@ -69,10 +69,10 @@ MUFU_LANES_PER_SM = 16  # rsqrt results per SM per clock
 OPS_PER_BODY_INTERACTION = 12
 OPS_PER_QUADRUPOLE_CELL = 30
 # DRAM bytes (read + write) of one force launch per body, measured by ncu on
-# the same workload at N = 1,048,576 (390.4 MB read + 75.0 MB written); the
+# the same workload at N = 1,048,576 (356.9 MB read + 74.7 MB written); the
 # tree, and the cells each body opens, grow in proportion to N at fixed
 # theta and distribution, so the per-body figure scales to 4M
-FORCE_DRAM_BYTES_PER_BODY = (390.426624e6 + 75.037696e6) / 1048576
+FORCE_DRAM_BYTES_PER_BODY = (356.932864e6 + 74.659328e6) / 1048576
 
 
 # ---------------------------------------------------------------------------
@@ -641,10 +641,11 @@ COLLIDE = dict(n=262144, steps=10)
 def run_collision(args, dist: Dist):
     """CUDA-event time of the collision stage inside Barnes-Hut steps of the
     plain configuration's bodies (unit ball, circular velocities, masses
-    1/N, theta 0.5, eps 0.01) with collision on.  Every ordered pair is
-    tested, so pairs/s = N^2 / stage time.  Roofline: the exact test of a
-    pair needs at least its x separation, one FP32-pipe operation, so pairs/s
-    over 128 FP32 lanes x SMs x clock is an upper bound of the fraction."""
+    1/N, theta 0.5, eps 0.01) with collision on.  pairs/s = N^2 / stage time:
+    the update is defined over every ordered pair, of which the hash grid
+    leaves those in the 27 cells around a body.  Roofline: each body's
+    position and velocity read and written once, over the HBM rate (the
+    stage is bound by chains of L2 accesses, far above it)."""
     import nbodysimulation_gb300 as nb
     dev = dist.local_rank
     n = COLLIDE["n"]
@@ -662,20 +663,18 @@ def run_collision(args, dist: Dist):
     if dist.rank != 0:
         return None
     peaks, _ = measured_peaks()
-    sm_count = device_sm_count(dev)
-    mhz = peaks.get("sm_max_mhz", 2070.0)
+    hbm = peaks.get("hbm_gbs", 6800.0)
     coll_ms = stage["collision"]
     pairs = float(n) * n
     pps = pairs / (coll_ms / 1e3)
-    peak = FP32_LANES_PER_SM * sm_count * mhz * 1e6
+    gbs = 64.0 * n / (coll_ms / 1e3) / 1e9
     return {"workload": "collision_ball_n262144 (Barnes-Hut steps with collision on; unit ball, masses 1/N)",
-            "kernel": "k_collision (block form, targets in sort order)", "n_bodies": n,
+            "kernel": "hash grid (csrc/k_collide.cu)", "n_bodies": n,
             "steps": COLLIDE["steps"], "ms_per_step": ms / COLLIDE["steps"], "collision_ms": coll_ms,
             "stages_ms": {k: round(v, 4) for k, v in stage.items() if v > 0},
             "pairs_per_s": pps,
-            "roofline": {"bound": "fp32", "achieved": pps / 1e12, "peak": peak / 1e12,
-                         "unit": "T pairs/s at one FP32-pipe op per pair", "frac": pps / peak,
-                         "peak_kind": "derived: 128 FP32 lanes x SMs x maximum SM clock"}}
+            "roofline": {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s (64 B per body)",
+                         "frac": gbs / hbm, "peak_kind": "measured hbm copy"}}
 
 
 # ---------------------------------------------------------------------------
