@@ -477,7 +477,6 @@ __device__ __forceinline__ CellSums finish_cell(const DevSim &s, int cell, int c
 // The sums of both kernels, by the arrival counters in memory / here (GB300, us):
 // monopoles, 3,000 bodies 37 / 27, 6,007 38 / 31, 12,000 40 / 34, 20,000 (340
 // cells) 41 / 41; quadrupoles, 3,000 bodies 39 / 33, 12,000 (190 cells) 48 / 51.
-constexpr int kTopThreads = 512;
 constexpr int kTopSharedBodies = 1 << 15;  // beyond, a list is longer anyhow (20 cells per 1,024 bodies)
 template <bool kQuad>
 constexpr int kTopShared = kQuad ? 128 : 256;
@@ -490,13 +489,13 @@ struct TopShared {
     int up[kTopShared<kQuad>];       // 8 * place of the parent + slot there
     int pending[kTopShared<kQuad>];  // children still to come
 };
-template <bool kQuad>
+template <bool kQuad, int kThreads>
 __device__ __forceinline__ void top_cells_shared(const DevSim &s, const BuildScratch &b, int cells,
                                                  TopShared<kQuad> &sh) {
-    const int n = s.n, j = threadIdx.x & 7, groups = blockDim.x >> 3;
+    const int n = s.n, j = threadIdx.x & 7, groups = kThreads >> 3;
     const unsigned group = 0xffu << (threadIdx.x & 24);
     // all of a group's cells at once: three trips to L2 in a row
-    constexpr int kRounds = kTopShared<kQuad> * 8 / kTopThreads;
+    constexpr int kRounds = kTopShared<kQuad> * 8 / kThreads;
     int cell[kRounds], ch[kRounds], at[kRounds];  // at: 1 + the child's place in the list
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {

@@ -480,6 +480,7 @@ __global__ void __launch_bounds__(kInsertThreads, 1) k_batch_insert(BatchTables 
     }
 }
 
+constexpr int kTopThreads = 512;
 template <bool kQuad>
 __global__ void __launch_bounds__(kTopThreads) k_batch_top(BatchTables t) {
     wait_for_previous();
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__(kTopThreads) k_batch_top(BatchTables t) {
     if (left_alone(v.s.ctrl)) return;
     const int cells = v.b.ctl[kBuildTop];
     if (cells <= kTopShared<kQuad>) {
-        if (v.part == 0) top_cells_shared<kQuad>(v.s, v.b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
+        if (v.part == 0) top_cells_shared<kQuad, kTopThreads>(v.s, v.b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
         return;
     }
     // an entry of 1,024 bodies has about 20 of a system's cells, a block room for 64

@@ -290,8 +290,13 @@ __global__ void __launch_bounds__(kTile) k_cells(DevSim s, BuildScratch b, const
     cells_tile(s, b, path, blockIdx.x);
 }
 
-template <bool kQuad>
-__global__ void __launch_bounds__(kTile) k_link(DevSim s, BuildScratch b, const u64 *__restrict__ path) {
+// kBlocks: least resident blocks per SM.  Five (48 registers) fill one another's
+// barriers where the tiles are two waves or more; else the compiler's choice (80 and 58)
+// (the sums, four / five blocks, ms: 4M with quadrupoles 0.705 / 0.646, 500,000
+// 0.092 / 0.084, 100,003 with quadrupoles 0.0579 / 0.0585; six 0.659 at 4M; four
+// asked for, 0.785: another schedule).
+template <bool kQuad, int kBlocks>
+__global__ void __launch_bounds__(kTile, kBlocks) k_link(DevSim s, BuildScratch b, const u64 *__restrict__ path) {
     wait_for_previous();
     link_tile<kQuad>(s, b, path, blockIdx.x);
 }
@@ -324,8 +329,8 @@ __device__ __forceinline__ bool grid_barrier(Ctrl *c, int *arrived, int target) 
     return ok != 0;
 }
 
-template <bool kQuad>
-__global__ void __launch_bounds__(kTopThreads, 1) k_top(DevSim s, BuildScratch b, bool may_share) {
+template <bool kQuad, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1) k_top(DevSim s, BuildScratch b, bool may_share) {
     wait_for_previous();
     Ctrl *ctrl = s.ctrl;
     const int n = s.n, root = n + s.cap;
@@ -335,7 +340,7 @@ __global__ void __launch_bounds__(kTopThreads, 1) k_top(DevSim s, BuildScratch b
         extern __shared__ __align__(16) unsigned char top_smem[];
         const int cells = b.ctl[kBuildTop];
         if (!may_share || cells > kTopShared<kQuad>) top_cells<kQuad>(s, b, cells, first >> 3, stride >> 3);
-        else if (blockIdx.x == 0) top_cells_shared<kQuad>(s, b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
+        else if (blockIdx.x == 0) top_cells_shared<kQuad, kThreads>(s, b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
         return;
     }
     const int blocks = gridDim.x;
@@ -425,15 +430,22 @@ cudaError_t launch_tree_cells(const DevSim &s, const BuildScratch &b, int sm_cou
 cudaError_t launch_tree_sums(const DevSim &s, const BuildScratch &b, int quadrupole, int sm_count, cudaStream_t st) {
     const int tiles = (s.n + kTile - 1) / kTile;
     const u64 *path = b.levels ? b.path : b.placed;
-    cudaError_t e = launch_next(quadrupole ? k_link<true> : k_link<false>, tiles, kTile, st, s, b, path);
-    const auto top = quadrupole ? k_top<true> : k_top<false>;
+    const auto link = tiles >= 8 * sm_count ? (quadrupole ? k_link<true, 5> : k_link<false, 5>)
+                                            : (quadrupole ? k_link<true, 1> : k_link<false, 1>);
+    cudaError_t e = launch_next(link, tiles, kTile, st, s, b, path);
     // shared memory only where the list may be short: the SMs' split of it would
     // hold back the walk's blocks
     const bool may_share = s.n <= kTopSharedBodies;
     const size_t shared = !may_share ? 0 : quadrupole ? sizeof(TopShared<true>) : sizeof(TopShared<false>);
+    // 1,024 threads a block where the list's groups fill them many times over (the
+    // sums with 512 / 1,024 threads, ms: 12,000 bodies with quadrupoles 0.049 /
+    // 0.054, 100,003 0.058 / 0.061, 262,144 0.0627 / 0.0640, 4M 0.643 / 0.600)
+    const int threads = s.n >= (1 << 20) ? 1024 : 512;
+    const auto top = threads == 1024 ? (quadrupole ? k_top<true, 1024> : k_top<false, 1024>)
+                                     : (quadrupole ? k_top<true, 512> : k_top<false, 512>);
     if (e == cudaSuccess && shared)
         e = cudaFuncSetAttribute(top, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-    if (e == cudaSuccess) e = launch_next_shared(top, sm_count, kTopThreads, shared, st, s, b, may_share);
+    if (e == cudaSuccess) e = launch_next_shared(top, sm_count, threads, shared, st, s, b, may_share);
     return e;
 }
 

@@ -108,3 +108,9 @@ def test_reference_tree_against_oracle(gpu, oracle, kind, n, quad):
     assert tg == cell_table(octant, t.mass, t.pos, t.body_count, n, t.root)
     order, k = oracle.sort_bodies(t.children, n, t.root)
     assert k == n and np.array_equal(sim.stage_debug(nb.DEBUG_SORTED), order)
+
+
+@pytest.mark.parametrize("quad", [0, 1])
+def test_large_tree_against_oracle(gpu, oracle, quad):
+    """From 2^20 bodies the upper cells' kernel has twice the threads."""
+    test_tree_against_oracle(gpu, oracle, "ball", (1 << 20) + 1, quad)
