@@ -85,7 +85,7 @@ static nb_status rebuild_tables(nb_batch *b) {
             sysdesc_set_top(b->h_sys[k], b->mem[k], b->cfg[k].tree_semantics == NB_TREE_REFERENCE,
                             b->shape.top_levels);
     std::vector<int> pref(batch_prefix_ints(ns), 0);
-    int totals[kBatchTotals];
+    int totals[kBatchSpaces];
     batch_prefixes(b->h_sys.data(), ns, batch_direct_block_bodies(b->variant), pref.data(), totals,
                    b->shape.build_chunk);
     B_CUDA(b, cudaMemcpyAsync(b->d_sys, b->h_sys.data(), sizeof(SysDesc) * ns, cudaMemcpyHostToDevice, b->st));

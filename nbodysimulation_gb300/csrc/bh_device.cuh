@@ -576,4 +576,88 @@ __device__ __forceinline__ bool sort_cell(const DevSim &s, int k, long long spin
     return true;
 }
 
+// The in-order sort without waits: a cell with bodies finds its start from the
+// counts before it in its ancestors' rows and places them.
+__device__ __forceinline__ void load_row(const DevSim &s, int c, int (&row)[8]) {
+    const int4 a0 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8]);
+    const int4 a1 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8 + 4]);
+    row[0] = a0.x; row[1] = a0.y; row[2] = a0.z; row[3] = a0.w;
+    row[4] = a1.x; row[5] = a1.y; row[6] = a1.z; row[7] = a1.w;
+}
+__device__ __forceinline__ void sort_bodies_of(const DevSim &s, int node) {
+    const int n = s.n, root = n + s.cap;
+    int own[8], row[8], cnt[8];
+    load_row(s, node - n, own);
+    bool bodies = false;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        bodies |= own[j] >= 0 && own[j] < n;
+        cnt[j] = own[j] >= n ? s.count[own[j] - n] : 1;
+    }
+    if (!bodies) return;
+    int at = 0;
+    for (int c = node, level = 0; c != root && level < 2 * kMaxDepth; ++level) {
+        const int up = s.parent[c - n];
+        load_row(s, up - n, row);
+        bool before = true;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            before = before && row[j] != c;
+            if (before) at += row[j] >= n ? s.count[row[j] - n] : 1;
+        }
+        c = up;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (own[j] < 0) break;
+        if (own[j] < n) {
+            if ((unsigned)at >= (unsigned)n) {  // inconsistent counts: never write past sorted[]
+                set_status(s.ctrl, kStSpinTimeout, at);
+                return;
+            }
+            s.sorted[at] = own[j];
+        }
+        at += cnt[j];
+    }
+}
+
+// ---------------------------------------------------------------------------
+// A phase of work in one kernel: chunk numbers handed out one at a time
+// (words[0]), and every block leaves when all chunks are done (words[1]).  A
+// block waits only for chunks that running blocks have taken, which wait for
+// nobody: no block of the grid has to be resident for another's sake, whatever
+// else (another handle's phases, say) holds the SMs.  Every thread of the block calls it;
+// both words are zero before.
+// ---------------------------------------------------------------------------
+template <class Fn>
+__device__ __forceinline__ bool run_phase(int *words, int chunks, Fn fn) {
+    __shared__ int take, ok;
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) take = atomicAdd(&words[0], 1);
+        __syncthreads();
+        const int c = take;
+        if (c >= chunks) break;
+        fn(c);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(&words[1], 1);
+        }
+    }
+    if (threadIdx.x == 0) {
+        ok = 1;
+        for (long long spins = 0; ld_volatile(&words[1]) < chunks;) {
+            if (++spins > kSpinCap) {
+                ok = 0;
+                break;
+            }
+            __nanosleep(64);
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
 }  // namespace nbgb

@@ -20,9 +20,10 @@ constexpr int kTileBlocks = kCellBodies / kTile;  // blocks of 256 bodies in an 
 static_assert(kCellBodies == kBuildTileBodies, "k_batch_cells: one block per entry of tile_prefix");
 
 // t.work: the force pass's counter, and the words of a step's insertions (zero
-// between steps)
-enum { kWorkForce = 0, kWorkInsert = 1, kWorkBarrier = 2, kWorkCells = 3 };
-static_assert(kWorkCells < kBatchWorkInts, "");
+// between steps; two a phase)
+enum { kWorkForce = 0, kWorkInsert = 1, kWorkPhases = 2 };
+constexpr int kInsertPhases = 6;
+static_assert(kWorkPhases + 2 * kInsertPhases <= kBatchWorkInts, "");
 
 // A system's buffers while its tree is built.  The paths lie in the body buffer
 // that the force pass writes next, the places in the regions where the sort
@@ -257,48 +258,15 @@ __global__ void __launch_bounds__(kTile) k_batch_link(BatchTables t) {
 // ---------------------------------------------------------------------------
 // insertions of the systems that take them (bh_device.cuh): top-level counts
 // per chunk, top cells, insertions, the used cells laid end to end,
-// summarisation and sort, with barriers over the grid.  One block per SM, so
-// that the grid is resident whatever runs beside it: an SM without a block of it
-// is free as soon as the others' blocks there (the direct sums of the small
-// systems) have ended.  (Two blocks on an SM could not count on that: the
-// first one, waiting, keeps the SM's split of shared memory as it is.)  A block
-// of 1,024 threads is faster than one of 512 or 256 (18 trees of 20,000 bodies,
-// one far out: 0.68 / 0.79 / 0.95 ms a step; one kernel per stage 0.65) and
-// costs a step without insertions no more, 2 us.  A batch that has trees that
-// insert at every step gets a launch per phase, in which the GPU is full (4
-// trees of 1,000,000 bodies, the reference's semantics: 3.15 ms a step, with
-// barriers 3.7).
+// summarisation and sort, as phases of one kernel (run_phase).  A step without
+// insertions pays 2 us for it.  18 trees of 20,000 bodies, one far out in each:
+// 0.64 ms a step, with a kernel per stage 0.65.
 // ---------------------------------------------------------------------------
-constexpr int kInsertThreads = 1024;  // a block that waits on a barrier
-constexpr int kPhaseThreads = 256;   // one of a launch per phase
-constexpr int kInsertPhases = 6;
+constexpr int kInsertThreads = 256;
 
 __device__ __forceinline__ bool inserts(const SysDesc &d) {
     const Ctrl *c = d.v.ctrl;
     return d.active && d.kind == kSysBH && system_live(c) && !read_status(c) && c->insert;
-}
-
-__device__ __forceinline__ bool insert_barrier(const BatchTables &t, int &passed) {
-    __shared__ int ok;
-    __syncthreads();
-    const int target = ++passed * gridDim.x;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&t.work[kWorkBarrier], 1);
-        ok = 1;
-        for (long long spins = 0; ld_volatile(&t.work[kWorkBarrier]) < target;) {
-            if (++spins > kSpinCap) {
-                for (int k = 0; k < t.nsys; ++k)
-                    if (inserts(t.sys[k])) set_status(t.sys[k].v.ctrl, kStSpinTimeout, target);
-                ok = 0;
-                break;
-            }
-            __nanosleep(256);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
 }
 
 // Bodies i0 + threadIdx.x .. of a system; its depth, or -1.
@@ -319,96 +287,48 @@ __device__ __forceinline__ int insert_chunk(const DevSim &s, const TopTables &to
     return deep;
 }
 
-// The in-order sort without waits (sort_cell's wait for a parent would hold up
-// its block's barriers): a cell with bodies finds its start from the
-// counts before it in its ancestors' rows and places them.
-__device__ __forceinline__ void load_row(const DevSim &s, int c, int (&row)[8]) {
-    const int4 a0 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8]);
-    const int4 a1 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8 + 4]);
-    row[0] = a0.x; row[1] = a0.y; row[2] = a0.z; row[3] = a0.w;
-    row[4] = a1.x; row[5] = a1.y; row[6] = a1.z; row[7] = a1.w;
-}
-__device__ __forceinline__ void sort_bodies_of(const DevSim &s, int node) {
-    const int n = s.n, root = n + s.cap;
-    int own[8], row[8], cnt[8];
-    load_row(s, node - n, own);
-    bool bodies = false;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        bodies |= own[j] >= 0 && own[j] < n;
-        cnt[j] = own[j] >= n ? s.count[own[j] - n] : 1;
-    }
-    if (!bodies) return;
-    int at = 0;
-    for (int c = node, level = 0; c != root && level < 2 * kMaxDepth; ++level) {
-        const int up = s.parent[c - n];
-        load_row(s, up - n, row);
-        bool before = true;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            before = before && row[j] != c;
-            if (before) at += row[j] >= n ? s.count[row[j] - n] : 1;
-        }
-        c = up;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (own[j] < 0) break;
-        if (own[j] < n) {
-            if ((unsigned)at >= (unsigned)n) {  // inconsistent counts: never write past sorted[]
-                set_status(s.ctrl, kStSpinTimeout, at);
-                return;
-            }
-            s.sorted[at] = own[j];
-        }
-        at += cnt[j];
-    }
-}
-
-static_assert((1 << (3 * kBatchTopMaxLevels)) <= 32 * kPhaseThreads, "top_cells_block: at most 32 regions a thread");
-// phase < 0: all of them
+static_assert((1 << (3 * kBatchTopMaxLevels)) <= 32 * kInsertThreads, "top_cells_block: at most 32 regions a thread");
 template <bool kQuad>
-__global__ void __launch_bounds__(kInsertThreads, 1) k_batch_insert(BatchTables t, int phase) {
+__global__ void __launch_bounds__(kInsertThreads, 4) k_batch_insert(BatchTables t) {
     wait_for_previous();
     if (!t.work[kWorkInsert]) return;  // grid-uniform: only earlier kernels set it
     __shared__ int bins[1 << (3 * kBatchTopMaxLevels)];
-    __shared__ int warp_tot[32], take;
+    __shared__ int warp_tot[32];
     const int tid = threadIdx.x;
-    int passed = 0;
+    int *phases = t.work + kWorkPhases;
+    const auto gave_up = [&]() {
+        if (tid == 0)
+            for (int k = 0; k < t.nsys; ++k)
+                if (inserts(t.sys[k])) set_status(t.sys[k].v.ctrl, kStSpinTimeout, 0);
+    };
     // top-level counts
-    if (phase <= 0) {
-        for (int x = blockIdx.x; x < t.chunks; x += gridDim.x) {
+    if (!run_phase(phases, t.chunks, [&](int x) {
             const SysDesc &d = t.sys[find_system(t.chunk_prefix, t.nsys, x)];
-            if (!inserts(d)) continue;  // block-uniform: nothing sets a status here
+            if (!inserts(d)) return;  // block-uniform: nothing sets a status here
             const DevSim s = system_view(d);
             const int i0 = (x - d.chunk_begin) * d.chunk;
             if (tid == 0 && i0 == 0) {  // without the cells numbered before `insert` was set
                 s.ctrl->bottom = s.n + s.cap;
                 s.ctrl->max_depth = 0;
             }
-            if (!d.top.levels) continue;
+            if (!d.top.levels) return;
             float box[6];
             load_box(s.ctrl, box);
-            __syncthreads();
             top_count_range(s, d.top, GeoCube::root(box), i0, min(s.n, i0 + d.chunk), blockDim.x, bins);
-        }
-        if (phase == 0 || !insert_barrier(t, passed)) return;
-    }
-    // top cells: a block per system
-    if (phase <= 1) {
-        for (int k = blockIdx.x; k < t.nsys; k += gridDim.x) {
+        }))
+        return gave_up();
+    // top cells: a block per system, whose status only it sets here
+    if (!run_phase(phases + 2, t.nsys, [&](int k) {
             const SysDesc &d = t.sys[k];
             const bool mine = inserts(d) && d.top.levels;
             __syncthreads();
             if (mine) top_cells_block(system_view(d), d.top);
-        }
-        if (phase == 1 || !insert_barrier(t, passed)) return;
-    }
+        }))
+        return gave_up();
     // insertions
-    if (phase <= 2) {
-        for (int x = blockIdx.x; x < t.chunks; x += gridDim.x) {
+    if (!run_phase(phases + 4, t.chunks, [&](int x) {
             const SysDesc &d = t.sys[find_system(t.chunk_prefix, t.nsys, x)];
-            if (!__shfl_sync(0xffffffffu, (int)inserts(d), 0)) continue;  // a status may appear meanwhile
+            if (!__shfl_sync(0xffffffffu, (int)inserts(d), 0)) return;  // a status may appear meanwhile
             const DevSim s = system_view(d);
             const int i0 = (x - d.chunk_begin) * d.chunk, i1 = min(s.n, i0 + d.chunk);
             const int depth = d.p.tree_ref     ? insert_chunk<RefBox, true, false>(s, d.top, i0, i1)
@@ -417,12 +337,10 @@ __global__ void __launch_bounds__(kInsertThreads, 1) k_batch_insert(BatchTables 
             __syncwarp();
             const int deep = __reduce_max_sync(0xffffffffu, depth);
             if ((tid & 31) == 0 && deep > 0) atomicMax(&s.ctrl->max_depth, deep);
-        }
-        if (phase == 2 || !insert_barrier(t, passed)) return;
-    }
+        }))
+        return gave_up();
     // every tree's allocated cells [bottom, root], one after another
-    if (phase <= 3) {
-        if (blockIdx.x == 0) {
+    if (!run_phase(phases + 6, 1, [&](int) {
             int carry = 0;
             for (int first = 0; first < t.nsys; first += blockDim.x) {
                 const int k = first + tid;
@@ -435,12 +353,12 @@ __global__ void __launch_bounds__(kInsertThreads, 1) k_batch_insert(BatchTables 
                 carry += total;
             }
             if (tid == 0) t.used_prefix[t.nsys] = carry;
-        }
-        if (phase == 3 || !insert_barrier(t, passed)) return;
-    }
-    const int total = __ldcg(&t.used_prefix[t.nsys]);
-    int lo = 0, hi = 0, k = 0;  // the system of the last cell and its range
-    auto locate = [&](int x) {
+        }))
+        return gave_up();
+    const int total = __ldcg(&t.used_prefix[t.nsys]), chunks = (total + kInsertThreads - 1) / kInsertThreads;
+    int lo = 0, hi = 0, k = 0, first = 0, par = 0;  // the system of the last cell, its range, first cell and parity
+    const auto locate = [&](int x) {
+        if (x >= lo && x < hi) return;
         int a = 0, z = t.nsys;
         while (z - a > 1) {
             const int mid = (a + z) >> 1;
@@ -450,34 +368,23 @@ __global__ void __launch_bounds__(kInsertThreads, 1) k_batch_insert(BatchTables 
         k = a;
         lo = __ldcg(&t.used_prefix[k]);
         hi = __ldcg(&t.used_prefix[k + 1]);
+        first = ld_volatile(&t.sys[k].v.ctrl->bottom);
+        par = system_parity(t.sys[k]);
     };
-    // sums: a cell's cost varies (the last arriver climbs), so blocks take the
-    // next cells as they go
-    if (phase <= 4) {
-        int first = 0, par = 0;
-        while (true) {
-            __syncthreads();
-            if (tid == 0) take = atomicAdd(&t.work[kWorkCells], (int)blockDim.x);
-            __syncthreads();
-            const int x = take + tid;
-            if (take >= total) break;
-            if (x >= total) continue;
-            if (x >= hi) {
-                locate(x);
-                first = ld_volatile(&t.sys[k].v.ctrl->bottom);
-                par = system_parity(t.sys[k]);
-            }
+    if (!run_phase(phases + 8, chunks, [&](int chunk) {
+            const int x = chunk * kInsertThreads + tid;
+            if (x >= total) return;
+            locate(x);
             summarize_from<kQuad>(system_view_par(t.sys[k], par), first + (x - lo));
-        }
-        if (phase == 4 || !insert_barrier(t, passed)) return;
-    }
-    // sort
-    lo = hi = 0;
-    for (int x = blockIdx.x * blockDim.x + tid; x < total; x += gridDim.x * blockDim.x) {
-        if (x >= hi) locate(x);
-        const DevSim &s = t.sys[k].v;  // the sort reads no body buffer
-        sort_bodies_of(s, s.n + s.cap - (x - lo));
-    }
+        }))
+        return gave_up();
+    if (!run_phase(phases + 10, chunks, [&](int chunk) {
+            const int x = chunk * kInsertThreads + tid;
+            if (x >= total) return;
+            locate(x);
+            sort_bodies_of(t.sys[k].v, first + (x - lo));  // reads no body buffer
+        }))
+        gave_up();
 }
 
 constexpr int kTopThreads = 512;
@@ -516,14 +423,8 @@ cudaError_t launch_batch_build(const BatchTables &t, int quadrupole, int sm_coun
         *launches += 6;
     }
     const auto insert = quadrupole ? k_batch_insert<true> : k_batch_insert<false>;
-    if (!t.large_refs) {
-        if (e == cudaSuccess) e = launch_next(insert, sm_count, kInsertThreads, st, t, -1);
-        *launches += 1;
-        return e;
-    }
-    for (int phase = 0; phase < kInsertPhases && e == cudaSuccess; ++phase)
-        e = launch_next(insert, 8 * sm_count, kPhaseThreads, st, t, phase);
-    *launches += kInsertPhases;
+    if (e == cudaSuccess) e = launch_next(insert, 4 * sm_count, kInsertThreads, st, t);
+    *launches += 1;
     return e;
 }
 

@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(256) k_box(DevSim s, BuildScratch b) {
     const unsigned all = block_reduce();
     if (threadIdx.x < 6) c->bbox_key[threadIdx.x] = all;
     b.total[threadIdx.x] = 0;  // kScanBlocks = blockDim.x
+    if (threadIdx.x < 8) b.ctl[kBuildPhases + threadIdx.x] = 0;
     if (threadIdx.x < 8) s.child[s.cap * 8 + threadIdx.x] = kEmpty;
     if (threadIdx.x == 0) {
         c->bottom = s.n + s.cap;
@@ -120,7 +121,6 @@ __global__ void __launch_bounds__(256) k_box(DevSim s, BuildScratch b) {
         s.count[s.cap] = 0;
         s.parent[s.cap] = -1;
         b.ctl[kBuildBoxes] = 0;
-        b.ctl[kBuildBarrier] = 0;
         b.ctl[kBuildTop] = 1;
         b.top[0] = s.n + s.cap;
         *reinterpret_cast<u64 *>(&b.ctl[kBuildPairs]) = 0;
@@ -304,31 +304,9 @@ __global__ void __launch_bounds__(kTile, kBlocks) k_link(DevSim s, BuildScratch 
 // ---------------------------------------------------------------------------
 // k_top: the cells that reach over a tile's edge, the root among them.  Each is
 // completed by whichever eight lanes bring its arrival counter to the number
-// of its children.  Or, when the step takes the insertions:
-// all of the build, the summarisation and the sort, with barriers over the
-// grid, which is no larger than what is resident.
+// of its children.  Or, when the step takes the insertions: all of the build,
+// the summarisation and the sort, as phases (run_phase).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool grid_barrier(Ctrl *c, int *arrived, int target) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(arrived, 1);
-        ok = 1;
-        for (long long spins = 0; ld_volatile(arrived) < target;) {
-            if (++spins > kSpinCap) {
-                set_status(c, kStSpinTimeout, target);
-                ok = 0;
-                break;
-            }
-            __nanosleep(64);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 template <bool kQuad, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1) k_top(DevSim s, BuildScratch b, bool may_share) {
     wait_for_previous();
@@ -343,35 +321,42 @@ __global__ void __launch_bounds__(kThreads, 1) k_top(DevSim s, BuildScratch b, b
         else if (blockIdx.x == 0) top_cells_shared<kQuad, kThreads>(s, b, cells, *reinterpret_cast<TopShared<kQuad> *>(top_smem));
         return;
     }
-    const int blocks = gridDim.x;
+    const int t = threadIdx.x;
+    int *phases = b.ctl + kBuildPhases;
+    const auto gave_up = [&]() {
+        if (t == 0) set_status(ctrl, kStSpinTimeout, 0);
+    };
     // cells that k_cells numbered before it met equal paths are dropped
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctrl->bottom = root;
-        ctrl->max_depth = 0;
-    }
-    if (!grid_barrier(ctrl, &b.ctl[kBuildBarrier], blocks)) return;
-    if (!read_status(ctrl)) {
-        float box[6];
-        load_box(ctrl, box);
-        const long long cap = tree_spin_cap(ctrl);
-        int deep = 0;
-        for (int i = first; i < n; i += stride) {
-            const int depth = b.ref ? insert_body<RefBox, true>(s, RefBox::root(box), i, cap)
-                                    : insert_body<GeoCube, false>(s, GeoCube::root(box), i, cap);
-            if (depth < 0) break;
-            deep = max(deep, depth);
-        }
-        if (deep > 0) atomicMax(&ctrl->max_depth, deep);
-    }
-    if (!grid_barrier(ctrl, &b.ctl[kBuildBarrier], 2 * blocks)) return;
-    const bool good = read_status(ctrl) == 0;
-    const int bottom = ctrl->bottom;
-    if (good)
-        for (int k = bottom + first; k <= root; k += stride) summarize_from<kQuad>(s, k);
-    if (!grid_barrier(ctrl, &b.ctl[kBuildBarrier], 3 * blocks) || !good) return;
+    if (!run_phase(phases, 1, [&](int) {
+            if (t > 0) return;
+            ctrl->bottom = root;
+            ctrl->max_depth = 0;
+        }))
+        return gave_up();
+    float box[6];
+    load_box(ctrl, box);
     const long long cap = tree_spin_cap(ctrl);
-    for (int k = root - first; k >= bottom; k -= stride)
-        if (!sort_cell(s, k, cap)) return;
+    int deep = 0;
+    if (!run_phase(phases + 2, (n + kThreads - 1) / kThreads, [&](int chunk) {
+            const int i = chunk * kThreads + t;
+            if (i >= n || read_status(ctrl)) return;
+            deep = max(deep, b.ref ? insert_body<RefBox, true>(s, RefBox::root(box), i, cap)
+                                   : insert_body<GeoCube, false>(s, GeoCube::root(box), i, cap));
+            if (deep > 0) atomicMax(&ctrl->max_depth, deep);
+        }))
+        return gave_up();
+    if (read_status(ctrl)) return;  // grid-uniform: the insertions are over
+    const int bottom = ld_volatile(&ctrl->bottom), chunks = (root - bottom) / kThreads + 1;
+    if (!run_phase(phases + 4, chunks, [&](int chunk) {
+            const int k = bottom + chunk * kThreads + t;
+            if (k <= root) summarize_from<kQuad>(s, k);
+        }))
+        return gave_up();
+    if (!run_phase(phases + 6, chunks, [&](int chunk) {
+            const int k = bottom + chunk * kThreads + t;
+            if (k <= root) sort_bodies_of(s, k);
+        }))
+        gave_up();
 }
 
 // ---------------------------------------------------------------------------

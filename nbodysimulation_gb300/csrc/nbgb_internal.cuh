@@ -224,13 +224,12 @@ struct SysDesc {
 };
 
 // Prefix tables (nsys + 1 entries each) and totals of a batch.
-constexpr int kBatchWorkInts = 4;
+constexpr int kBatchWorkInts = 16;
 struct BatchTables {
     const SysDesc *sys;
     int nsys;
     const int *chunk_prefix, *group_prefix, *dblock_prefix, *cblock_prefix, *tile_prefix;
     int chunks, groups, dblocks, cblocks, tiles;
-    int large_refs;    // trees that take the insertions at every step (kRefPathBodies)
     int *work;         // kBatchWorkInts batch-wide counters, zero before the first step
     int *used_prefix;  // nsys + 1: prefix over the cells each tree allocated this step (device-written)
 };
@@ -265,7 +264,8 @@ __device__ __forceinline__ DevSim system_view(const SysDesc &d) { return system_
 
 // Scratch of the build from sorted paths (k_build.cu).
 constexpr int kScanBlocks = 256;
-enum { kBuildBoxes = 0, kBuildBarrier = 1, kBuildTop = 2, kBuildPairs = 4, kBuildCtl = 8 };  // words of ctl
+// words of ctl (two a phase of the insertions, four phases)
+enum { kBuildBoxes = 0, kBuildTop = 2, kBuildPairs = 4, kBuildPhases = 8, kBuildCtl = 16 };
 struct BuildScratch {
     int levels;        // levels of the regions; 0: all bodies are ranked together
     int ref;           // 1: the reference's tree semantics

@@ -104,7 +104,7 @@ struct nb_server {
     int *d_pref[2] = {nullptr, nullptr}, *h_pref[2] = {nullptr, nullptr};
     int *d_work = nullptr;
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
-    int exec_totals[2][kBatchTotals + 1] = {};
+    int exec_totals[2][kBatchSpaces + 1] = {};
     cudaEvent_t round_ev[2] = {nullptr, nullptr};
 
     std::string err;
@@ -289,7 +289,7 @@ static cudaError_t launch_round(nb_server *s, std::vector<JobP> &run, int steps,
                                 std::deque<Delivery> &outs, std::vector<JobP> &finished) {
     const int ns = (int)run.size();
     for (int k = 0; k < ns; ++k) s->h_sys[buf][k] = run[k]->desc;
-    int totals[kBatchTotals];
+    int totals[kBatchSpaces];
     batch_prefixes(s->h_sys[buf], ns, batch_direct_block_bodies(s->variant), s->h_pref[buf], totals);
     cudaError_t e;
     if ((e = cudaMemcpyAsync(s->d_sys[buf], s->h_sys[buf], sizeof(SysDesc) * ns, cudaMemcpyHostToDevice,
@@ -298,7 +298,7 @@ static cudaError_t launch_round(nb_server *s, std::vector<JobP> &run, int steps,
     if ((e = cudaMemcpyAsync(s->d_pref[buf], s->h_pref[buf], sizeof(int) * batch_prefix_ints(ns),
                              cudaMemcpyHostToDevice, s->compute)) != cudaSuccess)
         return e;
-    int key[kBatchTotals + 1] = {ns};
+    int key[kBatchSpaces + 1] = {ns};
     memcpy(key + 1, totals, sizeof(totals));
     if (!s->exec[buf] || memcmp(key, s->exec_totals[buf], sizeof(key)) != 0) {
         // the kernels read everything else from the device tables; only the

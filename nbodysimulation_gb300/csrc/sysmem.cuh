@@ -149,8 +149,7 @@ inline SysDesc sysmem_desc(const SysMem &m, const nb_config &c, float dt) {
 
 // The batch-wide index spaces: box / insertion chunks, force warp groups,
 // direct-sum blocks, collision blocks, tiles of the sorted builds.
-// (The last total has no table: trees that always take the insertions.)
-constexpr int kBatchSpaces = 5, kBatchTotals = kBatchSpaces + 1;
+constexpr int kBatchSpaces = 5;
 // host-written prefix tables, nsys + 1 entries each
 inline size_t batch_prefix_ints(int nsys) { return (size_t)kBatchSpaces * (size_t)(nsys + 1); }
 // on the device they are followed by the device-written table of used cells
@@ -161,7 +160,7 @@ inline size_t batch_prefix_device_ints(int nsys) { return (size_t)(kBatchSpaces 
 // chunks of chunk_override bodies when > 0, else batch_chunk's).
 // Fills the *_begin fields of sys, the prefix tables (nsys + 1 entries each,
 // back to back in pref) and their totals.
-inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, int totals[kBatchTotals],
+inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, int totals[kBatchSpaces],
                            int chunk_override = 0) {
     int *chunk = pref, *group = pref + (nsys + 1), *dblock = pref + 2 * (nsys + 1), *cblock = pref + 3 * (nsys + 1),
         *tile = pref + 4 * (nsys + 1);
@@ -169,7 +168,7 @@ inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, 
     long long tree_bodies = 0;
     for (int k = 0; k < nsys; ++k)
         if (sys[k].active && sys[k].kind == kSysBH) tree_bodies += sys[k].v.n;
-    int body = 0, large_refs = 0;
+    int body = 0;
     for (int k = 0; k < nsys; ++k) {
         SysDesc &d = sys[k];
         const int n = d.v.n;
@@ -187,7 +186,6 @@ inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, 
         dblock[k + 1] = dblock[k] + (direct ? (n + direct_block - 1) / direct_block : 0);
         cblock[k + 1] = cblock[k] + (d.active && d.collide ? (n + kCollideBlockBodies - 1) / kCollideBlockBodies : 0);
         tile[k + 1] = tile[k] + (bh && !large_ref ? (n + kBuildTileBodies - 1) / kBuildTileBodies : 0);
-        large_refs += large_ref;
         body += n;
     }
     totals[0] = chunk[nsys];
@@ -195,12 +193,11 @@ inline void batch_prefixes(SysDesc *sys, int nsys, int direct_block, int *pref, 
     totals[2] = dblock[nsys];
     totals[3] = cblock[nsys];
     totals[4] = tile[nsys];
-    totals[5] = large_refs;
 }
 
 // d_pref holds the prefix tables of batch_prefixes followed by room for the
 // device-written table of used cells: batch_prefix_device_ints(nsys) ints.
-inline BatchTables batch_tables(const SysDesc *d_sys, int nsys, int *d_pref, const int totals[kBatchTotals],
+inline BatchTables batch_tables(const SysDesc *d_sys, int nsys, int *d_pref, const int totals[kBatchSpaces],
                                 int *work) {
     BatchTables t{};
     t.sys = d_sys;
@@ -215,7 +212,6 @@ inline BatchTables batch_tables(const SysDesc *d_sys, int nsys, int *d_pref, con
     t.dblocks = totals[2];
     t.cblocks = totals[3];
     t.tiles = totals[4];
-    t.large_refs = totals[5];
     t.work = work;
     t.used_prefix = d_pref + kBatchSpaces * (nsys + 1);
     return t;
