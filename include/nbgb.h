@@ -255,9 +255,9 @@ nb_status nb_force_error_probe(nb_sim *sim, const int32_t *sample, int32_t ns, d
 nb_status nb_diagnostics(nb_sim *sim, int32_t with_potential, double out[9]);
 
 /* ---- failure-path test hook ----
- * Caps the iterations of the tree stages' bounded waits (the build's lock
- * retries and the sort's wait for a parent's start) at `cap` (0 restores the
- * default, 2^24).  With a tiny cap a step gives up with NB_ERR_SPIN_TIMEOUT
+ * Caps the iterations of the tree stages' bounded waits at `cap` (0 restores the
+ * default, 2^24): the insertions' lock retries, which a capped step builds its
+ * tree by, and the large reference trees' sort waiting for a parent's start.  With a tiny cap a step gives up with NB_ERR_SPIN_TIMEOUT
  * instead of waiting, keeps its step-start state, and the handle stays
  * usable: the way the timeout path is exercised without hanging a GPU. */
 nb_status nb_debug_set_spin_cap(nb_sim *sim, int32_t cap);
@@ -352,8 +352,9 @@ nb_status nb_batch_system_status(nb_batch *b, int32_t k);
  * systems stay bit-identical to standalone handles for the tree path. */
 nb_status nb_batch_autotune(nb_batch *b, const char *cache_path, int32_t *chosen);
 /* The tree stages' launch shape: warps per block of the force walk, percent
- * of its resident blocks launched, bodies per bbox / build block (0: the
- * default rule) and the cap on the top levels built before the insertions. */
+ * of its resident blocks launched, bodies per block of the boxes and of
+ * insertions (0: the default rule) and the cap on the top levels built before
+ * insertions. */
 nb_status nb_batch_tree_shape(nb_batch *b, int32_t out[4]);
 /* out: systems, bodies, tree systems, direct systems, launches per step,
  * direct variant, kernels launched so far, body-node interactions of the

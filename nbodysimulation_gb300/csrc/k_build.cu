@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(256) k_box(DevSim s, BuildScratch b) {
         s.count[s.cap] = 0;
         s.parent[s.cap] = -1;
         b.ctl[kBuildBoxes] = 0;
+        b.ctl[kBuildScan] = 0;
         b.ctl[kBuildTop] = 1;
         b.top[0] = s.n + s.cap;
         *reinterpret_cast<u64 *>(&b.ctl[kBuildPairs]) = 0;
@@ -138,10 +139,10 @@ __global__ void __launch_bounds__(256) k_path(DevSim s, BuildScratch b) {
     }
 }
 
-// Exclusive scan of the region counts (a block adds up the totals of the
-// blocks before it as they appear; all blocks of the grid, at most kScanBlocks,
-// are resident together, and take as many chunks of kScanRegions as that
-// needs).  Clears the counts for the next step and adds up the pairs that
+// Exclusive scan of the region counts: a block adds up the totals of the
+// blocks before it as they appear.  The blocks, at most kScanBlocks with as many
+// chunks of kScanRegions each as that needs, take their places in the order in
+// which they start, so one waits only for blocks that run.  Clears the counts for the next step and adds up the pairs that
 // ranking the regions will compare.
 inline __host__ __device__ int scan_chunks(int levels) {
     const int chunks = ((1 << (3 * levels)) + kScanRegions - 1) / kScanRegions;
@@ -151,10 +152,11 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan(DevSim s, BuildScratch
     wait_for_previous();
     __shared__ int warp_tot[32];
     __shared__ u64 warp_sq[32];
-    __shared__ int before;
+    __shared__ int before, place;
+    if (threadIdx.x == 0) place = gridDim.x > 1 ? atomicAdd(&b.ctl[kBuildScan], 1) : 0;
     if (__syncthreads_or(build_off(s.ctrl))) return;  // a wait that gave up elsewhere stops whole blocks
     const int regions = 1 << (3 * b.levels), chunks = scan_chunks(b.levels);
-    const int begin = blockIdx.x * chunks * kScanRegions;
+    const int begin = place * chunks * kScanRegions;
     int4 c0, c1;
     auto load = [&](int chunk) {
         const int at = begin + chunk * kScanRegions + threadIdx.x * 8;
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan(DevSim s, BuildScratch
     }
     int total;
     int ex = block_exclusive_sum(sum, warp_tot, &total);
-    if (threadIdx.x == 0) st_volatile(&b.total[blockIdx.x], total + 1);
+    if (threadIdx.x == 0) st_volatile(&b.total[place], total + 1);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
     if ((threadIdx.x & 31) == 0) warp_sq[threadIdx.x >> 5] = sq;
@@ -187,7 +189,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan(DevSim s, BuildScratch
     }
     if (threadIdx.x < 32) {
         int acc = 0;
-        for (int k = threadIdx.x; k < (int)blockIdx.x; k += 32) {
+        for (int k = threadIdx.x; k < place; k += 32) {
             int t = ld_volatile(&b.total[k]);
             for (long long spins = 0; t == 0; t = ld_volatile(&b.total[k]))
                 if (++spins > kSpinCap) {
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan(DevSim s, BuildScratch
         }
         base += total;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) b.start[regions] = s.n;
+    if (place == 0 && threadIdx.x == 0) b.start[regions] = s.n;
 }
 __device__ __forceinline__ bool too_crowded(const DevSim &s, const BuildScratch &b) {
     return *reinterpret_cast<const volatile u64 *>(&b.ctl[kBuildPairs]) > (u64)s.n * kPairsPerBody;

@@ -265,7 +265,7 @@ __device__ __forceinline__ DevSim system_view(const SysDesc &d) { return system_
 // Scratch of the build from sorted paths (k_build.cu).
 constexpr int kScanBlocks = 256;
 // words of ctl (two a phase of the insertions, four phases)
-enum { kBuildBoxes = 0, kBuildTop = 2, kBuildPairs = 4, kBuildPhases = 8, kBuildCtl = 16 };
+enum { kBuildBoxes = 0, kBuildScan = 1, kBuildTop = 2, kBuildPairs = 4, kBuildPhases = 8, kBuildCtl = 16 };
 struct BuildScratch {
     int levels;        // levels of the regions; 0: all bodies are ranked together
     int ref;           // 1: the reference's tree semantics

@@ -559,8 +559,7 @@ nb_status nb_server_create(const nb_server_config *c, nb_job_fn fn, void *user, 
               cudaEventCreateWithFlags(&s->fork.fork, cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&s->fork.join, cudaEventDisableTiming) == cudaSuccess &&
               cudaMalloc(&s->d_work, sizeof(int) * kBatchWorkInts) == cudaSuccess &&
-              cudaMemset(s->d_work, 0, sizeof(int) * kBatchWorkInts) == cudaSuccess &&
-              cudaDeviceSynchronize() == cudaSuccess;
+              cudaMemsetAsync(s->d_work, 0, sizeof(int) * kBatchWorkInts, s->compute) == cudaSuccess;
     for (int b = 0; b < 2 && ok; ++b) {
         ok = cudaMalloc(&s->d_sys[b], sizeof(SysDesc) * ns) == cudaSuccess &&
              cudaMalloc(&s->d_pref[b], sizeof(int) * batch_prefix_device_ints((int)ns)) == cudaSuccess &&
