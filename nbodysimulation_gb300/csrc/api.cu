@@ -160,9 +160,11 @@ static int default_capacity(int n, int sm_count) {
 // current; on a host whose page tables the device shares, every other one too.
 // There a kernel costs what one copy does (9 us, 30 us at 4 MB) and replaces
 // one copy per array, and fills pages that the host never touched three times
-// as fast (4 MB 0.9 against 2.8 ms).
+// as fast (4 MB 0.9 against 2.8 ms).  Arrays of floats that are not aligned as
+// such go through the staging: a copy takes any address, a kernel's loads and
+// stores do not.
 void *nbgb::host_device_view(const void *p, int dev) {
-    if (!p) return nullptr;
+    if (!p || (uintptr_t)p % sizeof(float) != 0) return nullptr;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
