@@ -168,7 +168,8 @@ nb_status nb_get_config(const nb_sim *sim, nb_config *out);
  * src/MyApp.cpp:497-504).  n must equal num_of_bodies.  Page-locked arrays
  * (nb_host_alloc, cudaMallocHost, cudaHostRegister), and every array on a
  * host whose page tables the device shares, are read by the device directly,
- * without a staging copy; others are copied through a staging buffer. */
+ * without a staging copy; others, and arrays that are not aligned as floats,
+ * are copied through a staging buffer. */
 nb_status nb_set_state(nb_sim *sim, const float *pos3, const float *vel3, const float *mass, int32_t n);
 /* Any output pointer may be NULL.  Arrays that the device can reach (see
  * nb_set_state) are written by it directly. */

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstddef>
@@ -12,6 +13,8 @@
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "../../include/nbgb.h"
 #include "nbgb_internal.cuh"
@@ -154,16 +157,57 @@ static int default_capacity(int n, int sm_count) {
     return (int)c;
 }
 
-// Host arrays that kernels read and write in place, without a staging copy: one
+// Brings the pages of [p, p + bytes) into memory, for reading or for writing, if
+// they are not there already (asking takes 1 to 3 us, populating what is there 0.5
+// us a MB); false where they cannot be (nothing mapped there, an older kernel).
+static bool populate(const void *p, size_t bytes, bool write) {
+#ifndef MADV_POPULATE_READ  // Linux 5.14
+#define MADV_POPULATE_READ 22
+#define MADV_POPULATE_WRITE 23
+#endif
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t end = ((uintptr_t)p + bytes + page - 1) / page * page;
+    unsigned char in[1024];
+    for (uintptr_t at = (uintptr_t)p / page * page; at < end;) {
+        void *const chunk = reinterpret_cast<void *>(at);
+        const size_t pages = std::min((end - at) / page, sizeof(in));
+        if (mincore(chunk, pages * page, in) != 0) return false;
+        if (!std::all_of(in, in + pages, [](unsigned char c) { return c & 1; }) &&
+            madvise(chunk, pages * page, write ? MADV_POPULATE_WRITE : MADV_POPULATE_READ) != 0)
+            return false;
+        at += pages * page;
+    }
+    return true;
+}
+
+// Whether the device shares the host's page tables (asked once per device).
+static bool shares_page_tables(int dev) {
+    static std::atomic<signed char> known[64];  // 0: not asked yet
+    if (dev < 0 || dev >= 64) return false;
+    signed char k = known[dev].load(std::memory_order_relaxed);
+    if (!k) {
+        int v = 0;
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) != cudaSuccess) return false;
+        known[dev].store(k = v ? 1 : -1, std::memory_order_relaxed);
+    }
+    return k > 0;
+}
+
+// Host arrays that kernels read or write in place, without a staging copy: one
 // pass over the host link at full width.  Page-locked ones (nb_host_alloc,
 // cudaMallocHost, cudaHostRegister) allocated or registered while `dev` was
 // current; on a host whose page tables the device shares, every other one too.
 // There a kernel costs what one copy does (9 us, 30 us at 4 MB) and replaces
-// one copy per array, and fills pages that the host never touched three times
-// as fast (4 MB 0.9 against 2.8 ms).  Arrays of floats that are not aligned as
-// such go through the staging: a copy takes any address, a kernel's loads and
-// stores do not.
-void *nbgb::host_device_view(const void *p, int dev) {
+// one copy per array.  Pages that the host never touched the device would
+// populate one fault at a time, so those of larger arrays are populated first
+// (positions into untouched memory, us, faults of the device / staging /
+// populated first: 0.24 MB 84 / 180 / -, 0.6 MB 396 / 204 / 65, 1.2 MB 549 / 215 /
+// 82, 12 MB 2,950 / 588 / 457, 50 MB 13,200 / 1,960 / 1,780; below half a megabyte
+// the question costs more over a hundred calls than the first one's faults).  Arrays that cannot be populated, and arrays
+// of floats that are not aligned as such, go through the staging: a copy takes any
+// address, a kernel's loads and stores do not.
+constexpr size_t kInPlaceUntouched = 512 << 10;
+void *nbgb::host_device_view(const void *p, size_t bytes, bool write, int dev) {
     if (!p || (uintptr_t)p % sizeof(float) != 0) return nullptr;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
@@ -171,10 +215,8 @@ void *nbgb::host_device_view(const void *p, int dev) {
         return nullptr;
     }
     if (a.type == cudaMemoryTypeHost) return a.device == dev ? a.devicePointer : nullptr;
-    if (a.type != cudaMemoryTypeUnregistered) return nullptr;
-    int shared = 0;
-    if (cudaDeviceGetAttribute(&shared, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) != cudaSuccess || !shared)
-        return nullptr;
+    if (a.type != cudaMemoryTypeUnregistered || !shares_page_tables(dev)) return nullptr;
+    if (bytes > kInPlaceUntouched && !populate(p, bytes, write)) return nullptr;
     return const_cast<void *>(p);
 }
 
@@ -325,9 +367,9 @@ nb_status nb_set_state(nb_sim *s, const float *pos3, const float *vel3, const fl
     cudaSetDevice(s->dev);
     const size_t nn = (size_t)n;
     {
-        const float *dp = static_cast<const float *>(host_device_view(pos3, s->dev));
-        const float *dm = static_cast<const float *>(host_device_view(mass, s->dev));
-        const float *dv = static_cast<const float *>(host_device_view(vel3, s->dev));
+        const float *dp = static_cast<const float *>(host_device_view(pos3, 12 * nn, false, s->dev));
+        const float *dm = static_cast<const float *>(host_device_view(mass, 4 * nn, false, s->dev));
+        const float *dv = static_cast<const float *>(host_device_view(vel3, 12 * nn, false, s->dev));
         if (dp && dm && (!vel3 || dv)) {  // the kernel reads the host arrays
             NB_CUDA(s, launch_pack(dp, dm, dv, s->body[s->cur], s->vel, s->acc, n, s->stream));
             s->launches += 1;
@@ -375,7 +417,7 @@ nb_status nb_get_state(nb_sim *s, float *pos3, float *vel3, float *acc3, float *
     float *host[4] = {pos3, vel3, acc3, mass}, *dev[4];
     bool direct = pos3 || vel3 || acc3 || mass;
     for (int k = 0; k < 4; ++k) {
-        dev[k] = static_cast<float *>(host_device_view(host[k], s->dev));
+        dev[k] = static_cast<float *>(host_device_view(host[k], (k == 3 ? 4 : 12) * nn, true, s->dev));
         direct = direct && (!host[k] || dev[k]);
     }
     if (direct) {  // the kernel writes the host arrays
@@ -647,7 +689,7 @@ nb_status nb_copy_vertices(nb_sim *s, float *dst4, int32_t dst_is_device) {
         if (!aligned) return fail(s, NB_ERR_INVALID_ARGUMENT, "nb_copy_vertices: a device dst must be 16-byte aligned");
         NB_CUDA(s, launch_copy_vertices(s->body[s->cur], s->n, reinterpret_cast<float4 *>(dst4), s->stream));
         s->launches += 1;
-    } else if (float *hd = aligned ? static_cast<float *>(host_device_view(dst4, s->dev)) : nullptr) {  // host, in place
+    } else if (float *hd = aligned ? static_cast<float *>(host_device_view(dst4, 16 * (size_t)s->n, true, s->dev)) : nullptr) {  // host, in place
         NB_CUDA(s, launch_copy_vertices(s->body[s->cur], s->n, reinterpret_cast<float4 *>(hd), s->stream));
         s->launches += 1;
     } else {

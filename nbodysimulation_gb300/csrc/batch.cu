@@ -279,9 +279,9 @@ nb_status nb_batch_set_state(nb_batch *b, int32_t k, const float *pos3, const fl
     const SysMem &m = b->mem[k];
     const int par = b->h_ctrl[k].parity & 1;
     const size_t n = (size_t)m.n;
-    const float *dp = static_cast<const float *>(host_device_view(pos3, b->dev)),
-                *dm = static_cast<const float *>(host_device_view(mass, b->dev)),
-                *dv = static_cast<const float *>(host_device_view(vel3, b->dev));
+    const float *dp = static_cast<const float *>(host_device_view(pos3, 12 * n, false, b->dev)),
+                *dm = static_cast<const float *>(host_device_view(mass, 4 * n, false, b->dev)),
+                *dv = static_cast<const float *>(host_device_view(vel3, 12 * n, false, b->dev));
     if (dp && dm && (!vel3 || dv)) {  // the kernel reads the host arrays
         B_CUDA(b, launch_pack(dp, dm, dv, m.body[par], m.vel, m.acc, m.n, b->st));
         b->launches += 1;
@@ -310,7 +310,7 @@ nb_status nb_batch_get_state(nb_batch *b, int32_t k, float *pos3, float *vel3, f
     float *host[4] = {pos3, vel3, acc3, mass}, *dev[4];
     bool direct = pos3 || vel3 || acc3 || mass;
     for (int q = 0; q < 4; ++q) {
-        dev[q] = static_cast<float *>(host_device_view(host[q], b->dev));
+        dev[q] = static_cast<float *>(host_device_view(host[q], (q == 3 ? 4 : 12) * n, true, b->dev));
         direct = direct && (!host[q] || dev[q]);
     }
     if (direct) {  // the kernel writes the host arrays

@@ -357,9 +357,9 @@ constexpr int kCollideGridFrom = 5120;
 cudaError_t launch_collision(const DevSim &s, const CollideGrid &g, int tree, int sm_count, cudaStream_t st,
                              int *launches);
 cudaError_t launch_copy_vertices(const float4 *body, int n, float4 *dst, cudaStream_t st);
-// The device address of a host array that kernels can read and write where it
-// lies, else null (api.cu).
-void *host_device_view(const void *p, int dev);
+// The device address of a host array of `bytes` bytes that kernels can read (or
+// write) where it lies, else null (api.cu).
+void *host_device_view(const void *p, size_t bytes, bool write, int dev);
 cudaError_t launch_pack(const float *pos3, const float *mass, const float *vel3, float4 *body, float4 *vel,
                         float4 *acc, int n, cudaStream_t st);
 cudaError_t launch_unpack(const float4 *body, const float4 *vel, const float4 *acc, float *pos3, float *vel3,
