@@ -230,7 +230,7 @@ __device__ __forceinline__ void top_count_range(const DevSim &s, const TopTables
     for (int r = threadIdx.x; r < nbins; r += blockDim.x) bins[r] = 0;
     __syncthreads();
     for (int i = i0 + threadIdx.x; i < i1; i += stride)
-        atomicAdd(&bins[top_region(root_g, __ldg(&s.body_cur[i]), t.levels)], 1);
+        atomicAdd(&bins[top_region(root_g, s.body_cur[i], t.levels)], 1);
     __syncthreads();
     for (int r = threadIdx.x; r < nbins; r += blockDim.x)
         if (bins[r]) atomicAdd(&t.count[r], bins[r]);

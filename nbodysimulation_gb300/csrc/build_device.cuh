@@ -43,7 +43,7 @@ __device__ __forceinline__ bool build_off(const Ctrl *c) { return read_status(c)
 template <class Geo>
 __device__ __forceinline__ void path_body(const DevSim &s, const BuildScratch &b, const Geo &root, int i) {
     constexpr int kLevels = std::is_same<Geo, RefBox>::value ? kPathLevels - 1 : kPathLevels;
-    const u64 key = octant_path<Geo>(root, __ldg(&s.body_cur[i]), kLevels);
+    const u64 key = octant_path<Geo>(root, s.body_cur[i], kLevels);
     b.path[i] = key;
     if (b.levels) {
         // a warp whose bodies are all in one region (nearly every one when a body

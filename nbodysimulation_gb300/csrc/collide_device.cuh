@@ -84,9 +84,8 @@ __device__ __forceinline__ void reflect(const float4 me, const float4 q, float4 
 // in tiles by TMA bulk copies (double-buffered mbarriers, bounded waits).
 // Every thread of the block calls it.  Writes vel only when every wait
 // succeeded.
-__device__ __forceinline__ void collide_block(const float4 *__restrict__ pos, float4 *__restrict__ vel,
-                                              const int *__restrict__ order, int targets, int n, int i0,
-                                              Ctrl *ctrl) {
+__device__ __forceinline__ void collide_block(const float4 *pos, float4 *vel, const int *order, int targets,
+                                              int n, int i0, Ctrl *ctrl) {
     __shared__ __align__(128) float4 tile[2][kCollideTile];
     __shared__ __align__(8) uint64_t bar[2];
     const int it = i0 + (int)threadIdx.x;
@@ -142,8 +141,7 @@ __device__ __forceinline__ void collide_block(const float4 *__restrict__ pos, fl
 // group of 32 are then applied by every lane in ascending j (a ballot and a
 // broadcast of the contact's position), the same sequence of reflections as
 // the block form.  All 32 lanes call it.
-__device__ __forceinline__ void collide_warp(const float4 *__restrict__ pos, float4 *__restrict__ vel, int n, int i,
-                                             int lane) {
+__device__ __forceinline__ void collide_warp(const float4 *pos, float4 *vel, int n, int i, int lane) {
     if (i >= n) return;  // warp-uniform
     const float4 me = pos[i];
     float4 v = vel[i];
@@ -151,7 +149,7 @@ __device__ __forceinline__ void collide_warp(const float4 *__restrict__ pos, flo
     const bool me_finite = finite3(me);
     for (int j0 = 0; j0 < n; j0 += 32) {
         const int j = j0 + lane;
-        const float4 q = j < n ? __ldg(&pos[j]) : me;
+        const float4 q = j < n ? pos[j] : me;
         const bool fast = me_finite && finite3(q);
         unsigned hit = __ballot_sync(0xffffffffu, j < n && j != i && in_contact(me, q, rr, fast));
         while (hit) {

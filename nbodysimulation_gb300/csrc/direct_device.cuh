@@ -60,16 +60,16 @@ __device__ __forceinline__ void quirk_pair(float dx, float dy, float dz, float m
 // The warp's part of the sum: tiles w, w + kW, ... of [j0, j1).  i0: index of
 // the lane's first target, its others 32 apart (kZeroSkipsSelf).
 template <int kI, int kW, bool kQuirk, int kZero>
-__device__ __forceinline__ void direct_sum(const float4 *__restrict__ body, int j0, int j1, int i0, float eps,
-                                           int warp, int lane, DirectShared<kW> &sh, DirectTargets<kI> &T) {
+__device__ __forceinline__ void direct_sum(const float4 *body, int j0, int j1, int i0, float eps, int warp, int lane,
+                                           DirectShared<kW> &sh, DirectTargets<kI> &T) {
     const float2 eps2 = dup(eps * eps);
     const int tiles = (j1 - j0 + kDirectTile - 1) / kDirectTile;
     float4 p0, p1;
     // bodies beyond the range: the range's last one without mass
     auto load = [&](int t) {
         const int j = j0 + t * kDirectTile + 2 * lane;
-        p0 = __ldg(&body[min(j, j1 - 1)]);
-        p1 = __ldg(&body[min(j + 1, j1 - 1)]);
+        p0 = body[min(j, j1 - 1)];
+        p1 = body[min(j + 1, j1 - 1)];
         if (j >= j1) p0.w = 0.0f;
         if (j + 1 >= j1) p1.w = 0.0f;
     };
@@ -144,8 +144,7 @@ __device__ __forceinline__ float3 direct_block_sum(DirectShared<kW> &sh, const D
 }
 
 template <int kI>
-__device__ __forceinline__ void direct_load_targets(const float4 *__restrict__ body, int i0, int n,
-                                                    DirectTargets<kI> &T) {
+__device__ __forceinline__ void direct_load_targets(const float4 *body, int i0, int n, DirectTargets<kI> &T) {
 #pragma unroll
     for (int r = 0; r < kI; ++r) {
         const float4 P = body[min(i0 + 32 * r, n - 1)];

@@ -382,7 +382,7 @@ __device__ __forceinline__ void force_group(const DevSim &s, const StepParams &p
                     const int k = (kQuad ? nc : nb) + __popc(ma & below);
                     float *at4 = (kQuad ? &ws.cell[0][0].x : &ws.src[0][0].x) + ((k >> 1) * 4 + (k & 1));
                     put_source(at4, ws.upm[nu + lane]);
-                    if constexpr (kQuad) put_moments(at4, __ldg(&s.wqa[me.y]), __ldg(&s.wqb[me.y]));
+                    if constexpr (kQuad) put_moments(at4, s.wqa[me.y], s.wqb[me.y]);
                 } else {
                     const int k = sp + __popc(mr & below);
                     if (k < kStack) ws.stack[k] = me.x;

@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(32 * kRankWarps) k_rank_all(DevSim s, BuildScr
     b.placed[less] = key;
 }
 
-__global__ void __launch_bounds__(kTile) k_cells(DevSim s, BuildScratch b, const u64 *__restrict__ path) {
+__global__ void __launch_bounds__(kTile) k_cells(DevSim s, BuildScratch b, const u64 *path) {
     wait_for_previous();
     cells_tile(s, b, path, blockIdx.x);
 }
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kTile) k_cells(DevSim s, BuildScratch b, const
 // 0.092 / 0.084, 100,003 with quadrupoles 0.0579 / 0.0585; six 0.659 at 4M; four
 // asked for, 0.785: another schedule).
 template <bool kQuad, int kBlocks>
-__global__ void __launch_bounds__(kTile, kBlocks) k_link(DevSim s, BuildScratch b, const u64 *__restrict__ path) {
+__global__ void __launch_bounds__(kTile, kBlocks) k_link(DevSim s, BuildScratch b, const u64 *path) {
     wait_for_previous();
     link_tile<kQuad>(s, b, path, blockIdx.x);
 }

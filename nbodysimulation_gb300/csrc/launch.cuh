@@ -8,6 +8,12 @@
 // (4,096-body direct steps 13.5 -> 11.6 us; the nine kernels of a 100,003-body
 // tree step 258 -> 245 us).
 //
+// Such a kernel exists while earlier ones still write what it will read.  So it
+// reads their results with plain loads (or past L1, __ldcg): read-only loads
+// (__ldg, const __restrict__ parameters) are for memory that nothing writes as long
+// as the kernel exists, and may be moved above the wait.  Tables the host wrote
+// before the step (the prefixes of a batch) may be read so.
+//
 // Blocks placed early go where there is room, not evenly: a kernel of few long
 // blocks (the force walk of a small system) must not be, nor the first kernel of
 // a step behind the force walk, whose last blocks it would share SMs with
