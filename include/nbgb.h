@@ -284,8 +284,7 @@ void nb_host_free(void *p);
  * bodies of d_body4 (device float4 {x,y,z,m}, 16-byte aligned) into d_acc4
  * (device float4 {ax,ay,az,0}, 16-byte aligned), on `stream` (a
  * cudaStream_t; NULL for the default stream) of the current device.  The
- * call is synchronous: it returns after its work on `stream` has finished
- * (it synchronises that stream to read the status of its bounded waits).
+ * call is synchronous: it returns after its work on `stream` has finished.
  * Same arithmetic as the NB_BRUTE_FORCE_LOCAL Plummer sum.
  *
  * Limit: n <= NB_NOALLOC_MAX_BODIES; larger n returns NB_ERR_INVALID_ARGUMENT.
@@ -295,7 +294,8 @@ void nb_host_free(void *p);
  * any stream capture.  The address is kept for the life of the process, so
  * after a cudaDeviceReset of a device this entry point must not be called on
  * that device again.  All calls share the array, so calls that overlap on
- * the GPU race: serialise them. */
+ * the GPU race and their results are wrong: serialise them.  Later calls are
+ * not affected. */
 #define NB_NOALLOC_MAX_BODIES 65536
 nb_status nb_direct_accel_noalloc(const float *d_body4, int32_t n, float eps, float G, float *d_acc4,
                                   void *stream);

@@ -248,7 +248,9 @@ namespace nbgb {
 // partial accelerations of the body slices -- lives in a file-scope device
 // array of fixed size, together with the counters of the slices that are
 // done.  Every GPU that loads this library holds that array (1 MiB + 8 KiB)
-// until the process exits.  All calls share it: calls that overlap on the GPU race.
+// until the process exits.  All calls share it: calls that overlap on the GPU
+// race, and only they: the counters they may leave behind are cleared by the next
+// call that has the array to itself (NoAllocCall).
 // ===========================================================================
 constexpr int kNoAllocMaxBodies = 65536;  // = NB_NOALLOC_MAX_BODIES
 static __device__ __align__(256) float4 g_noalloc_part[kNoAllocMaxBodies];
@@ -270,23 +272,48 @@ namespace {
 // a reset of the device's primary context) unloads the module, after which
 // this entry point must not be called on that device again.
 constexpr int kMaxDevices = 64;
+struct NoAllocDevice {
+    void *part = nullptr, *arrived = nullptr;
+    int calls = 0;         // between their first launch and the end of their synchronisation
+    bool unclean = false;  // calls overlapped, or one failed: its counters may not be zero
+};
 std::mutex g_noalloc_mu;
-void *g_noalloc_part_ptr[kMaxDevices] = {};
-void *g_noalloc_arrived_ptr[kMaxDevices] = {};
+NoAllocDevice g_noalloc_dev[kMaxDevices];
 
-bool noalloc_setup(int dev, float4 **part, int **arrived) {
-    std::lock_guard<std::mutex> lk(g_noalloc_mu);
-    if (!g_noalloc_part_ptr[dev]) {
-        void *p = nullptr, *c = nullptr;
-        if (cudaGetSymbolAddress(&p, nbgb::g_noalloc_part) != cudaSuccess) return false;
-        if (cudaGetSymbolAddress(&c, nbgb::g_noalloc_arrived) != cudaSuccess) return false;
-        g_noalloc_part_ptr[dev] = p;
-        g_noalloc_arrived_ptr[dev] = c;
+// One call's turn on the shared array.  A call that meets no other finds the
+// counters at zero, as its own last blocks leave them, or clears them first.
+class NoAllocCall {
+  public:
+    explicit NoAllocCall(int dev) : d_(g_noalloc_dev[dev]) {
+        std::lock_guard<std::mutex> lk(g_noalloc_mu);
+        if (!d_.part) {
+            void *p = nullptr, *c = nullptr;
+            if (cudaGetSymbolAddress(&p, nbgb::g_noalloc_part) != cudaSuccess) return;
+            if (cudaGetSymbolAddress(&c, nbgb::g_noalloc_arrived) != cudaSuccess) return;
+            d_.part = p;
+            d_.arrived = c;
+        }
+        ok_ = true;
+        if (d_.calls++ > 0) d_.unclean = true;
+        clear_ = d_.unclean && d_.calls == 1;
+        if (clear_) d_.unclean = false;
     }
-    *part = static_cast<float4 *>(g_noalloc_part_ptr[dev]);
-    *arrived = static_cast<int *>(g_noalloc_arrived_ptr[dev]);
-    return true;
-}
+    ~NoAllocCall() {
+        std::lock_guard<std::mutex> lk(g_noalloc_mu);
+        if (!ok_) return;
+        --d_.calls;
+        if (!done_) d_.unclean = true;
+    }
+    bool ok() const { return ok_; }
+    bool clear() const { return clear_; }
+    float4 *part() const { return static_cast<float4 *>(d_.part); }
+    int *arrived() const { return static_cast<int *>(d_.arrived); }
+    void done() { done_ = true; }
+
+  private:
+    NoAllocDevice &d_;
+    bool ok_ = false, clear_ = false, done_ = false;
+};
 }  // namespace
 
 extern "C" nb_status nb_direct_accel_noalloc(const float *d_body4, int32_t n, float eps, float G, float *d_acc4,
@@ -297,10 +324,13 @@ extern "C" nb_status nb_direct_accel_noalloc(const float *d_body4, int32_t n, fl
     if (((uintptr_t)d_body4 & 15u) || ((uintptr_t)d_acc4 & 15u)) return NB_ERR_INVALID_ARGUMENT;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return NB_ERR_NO_DEVICE;
-    float4 *part = nullptr;
-    int *arrived = nullptr;
-    if (!noalloc_setup(dev, &part, &arrived)) return NB_ERR_CUDA;
+    NoAllocCall call(dev);
+    if (!call.ok()) return NB_ERR_CUDA;
+    float4 *part = call.part();
+    int *arrived = call.arrived();
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (call.clear() && cudaMemsetAsync(arrived, 0, sizeof(int) * (kNoAllocMaxBodies / 32), st) != cudaSuccess)
+        return NB_ERR_CUDA;
     int sm_count = 0;
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     DevSim s{};
@@ -321,5 +351,7 @@ extern "C" nb_status nb_direct_accel_noalloc(const float *d_body4, int32_t n, fl
     if (e != cudaSuccess) return NB_ERR_CUDA;
     if (overlap && cudaMemcpyAsync(d_acc4, part, bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
         return NB_ERR_CUDA;
-    return cudaStreamSynchronize(st) == cudaSuccess ? NB_OK : NB_ERR_CUDA;
+    if (cudaStreamSynchronize(st) != cudaSuccess) return NB_ERR_CUDA;
+    call.done();
+    return NB_OK;
 }
