@@ -371,6 +371,14 @@ static nb_status enqueue_steps(nb_batch *b, float dt, int nsteps) {
 static nb_status check_status(nb_batch *b) {
     nb_status r = read_ctrls(b);
     if (r != NB_OK) return r;
+    // insertions whose wait gave up may leave top-level counts, which must be zero
+    // between steps
+    for (int k = 0; k < b->nsys; ++k) {
+        int *p = nullptr;
+        size_t bytes = 0;
+        if (b->h_ctrl[k].status == kStSpinTimeout) sysmem_top_counts(b->mem[k], &p, &bytes);
+        if (bytes) B_CUDA(b, cudaMemsetAsync(p, 0, bytes, b->st));
+    }
     for (int k = 0; k < b->nsys; ++k) {
         if (b->h_ctrl[k].status) {
             char buf[128];

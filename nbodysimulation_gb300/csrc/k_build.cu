@@ -142,8 +142,10 @@ __global__ void __launch_bounds__(256) k_path(DevSim s, BuildScratch b) {
 // Exclusive scan of the region counts: a block adds up the totals of the
 // blocks before it as they appear.  The blocks, at most kScanBlocks with as many
 // chunks of kScanRegions each as that needs, take their places in the order in
-// which they start, so one waits only for blocks that run.  Clears the counts for the next step and adds up the pairs that
-// ranking the regions will compare.
+// which they start, so one waits only for blocks that run.  Clears the counts for
+// the next step and adds up the pairs that ranking the regions will compare.  No
+// block leaves early: the counts must be zero before the next step, also when a
+// wait gives up (a step that failed before this kernel counted nothing).
 inline __host__ __device__ int scan_chunks(int levels) {
     const int chunks = ((1 << (3 * levels)) + kScanRegions - 1) / kScanRegions;
     return (chunks + kScanBlocks - 1) / kScanBlocks;
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kScanThreads, 2) k_scan(DevSim s, BuildScratch
     __shared__ u64 warp_sq[32];
     __shared__ int before, place;
     if (threadIdx.x == 0) place = gridDim.x > 1 ? atomicAdd(&b.ctl[kBuildScan], 1) : 0;
-    if (__syncthreads_or(build_off(s.ctrl))) return;  // a wait that gave up elsewhere stops whole blocks
+    __syncthreads();
     const int regions = 1 << (3 * b.levels), chunks = scan_chunks(b.levels);
     const int begin = place * chunks * kScanRegions;
     int4 c0, c1;
