@@ -256,11 +256,11 @@ nb_status nb_force_error_probe(nb_sim *sim, const int32_t *sample, int32_t ns, d
 nb_status nb_diagnostics(nb_sim *sim, int32_t with_potential, double out[9]);
 
 /* ---- failure-path test hook ----
- * Caps the iterations of the tree stages' bounded waits at `cap` (0 restores the
- * default, 2^24): the insertions' lock retries, which a capped step builds its
- * tree by, and the large reference trees' sort waiting for a parent's start.  With a tiny cap a step gives up with NB_ERR_SPIN_TIMEOUT
- * instead of waiting, keeps its step-start state, and the handle stays
- * usable: the way the timeout path is exercised without hanging a GPU. */
+ * Caps the iterations of the insertions' lock retries, by which a capped step
+ * builds its tree, at `cap` (0 restores the default, 2^24, and the build that
+ * needs none).  With a tiny cap a step gives up with NB_ERR_SPIN_TIMEOUT instead
+ * of waiting, keeps its step-start state, and the handle stays usable: the way
+ * the timeout path is exercised without hanging a GPU. */
 nb_status nb_debug_set_spin_cap(nb_sim *sim, int32_t cap);
 
 /* ---- last error ---- */

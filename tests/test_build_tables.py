@@ -41,3 +41,15 @@ def test_steps_after_failed_ones(gpu, n):
         s.step(1e-3, 2)
         for got, w in zip(s.get_state(), want):
             np.testing.assert_array_equal(got, w)
+
+
+def test_large_reference_sort_waits_for_nobody():
+    """The sort of large trees with the reference's semantics (k_tree.cu) runs on a
+    plain grid, whose blocks may start in any order and late: no loop of it waits
+    for what another thread writes (a bounded climb to the root is all there is)."""
+    called = "sort_cell"
+    assert called in dict(kernels(source(CSRC + "/k_tree.cu")))["k_sort"]
+    device = source(CSRC + "/bh_device.cuh")
+    at = device.index(f" {called}(const DevSim")
+    function = device[at:device.index("\n}\n", at)]
+    assert "__nanosleep" not in function and "while" not in function and "spin" not in function.lower().replace("kstspintimeout", "")
