@@ -312,11 +312,14 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
     s->stage3 = reinterpret_cast<float *>(s->part + n);
     s->stage1 = s->stage3 + 3 * n;
     if (cudaMallocHost((void **)&s->h_ctrl, sizeof(Ctrl)) != cudaSuccess) return cleanup(NB_ERR_OUT_OF_MEMORY);
-    cudaMemset(s->ctrl, 0, sizeof(Ctrl));
-    cudaMemset(s->vel, 0, sizeof(float4) * n);
-    cudaMemset(s->acc, 0, sizeof(float4) * n);
+    // cleared and waited for on the handle's own stream: a wait for the whole
+    // device would fail another thread's graph capture
     int *zeroed = reinterpret_cast<int *>(s->part + part);
-    if (tables) cudaMemset(zeroed, 0, sizeof(int) * tables);
+    if (cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), s->stream) != cudaSuccess ||
+        cudaMemsetAsync(s->vel, 0, sizeof(float4) * n, s->stream) != cudaSuccess ||
+        cudaMemsetAsync(s->acc, 0, sizeof(float4) * n, s->stream) != cudaSuccess ||
+        (tables && cudaMemsetAsync(zeroed, 0, sizeof(int) * tables, s->stream) != cudaSuccess))
+        return cleanup(NB_ERR_CUDA);
     if (!s->tree) s->arrived = zeroed;
     // the build's paths and places lie in the transfer staging, which no step uses
     else if (tables) s->build = build_scratch(s->n, s->sm_count, ref, zeroed, s->part, s->stage3);
@@ -333,7 +336,7 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
         return cleanup(NB_ERR_OUT_OF_MEMORY);
     if (cudaEventCreate(&s->t_begin) != cudaSuccess || cudaEventCreate(&s->t_end) != cudaSuccess)
         return cleanup(NB_ERR_CUDA);
-    if (cudaDeviceSynchronize() != cudaSuccess) return cleanup(NB_ERR_CUDA);
+    if (cudaStreamSynchronize(s->stream) != cudaSuccess) return cleanup(NB_ERR_CUDA);
     *out = s;
     return NB_OK;
 }

@@ -210,29 +210,32 @@ nb_status nb_batch_create(const nb_config *cfgs, int32_t nsys, nb_batch **out) {
         cudaMalloc(&b->d_sys, sizeof(SysDesc) * nsys) != cudaSuccess ||
         cudaMalloc(&b->d_pref, sizeof(int) * batch_prefix_device_ints(nsys)) != cudaSuccess ||
         cudaMalloc(&b->d_work, sizeof(int) * kBatchWorkInts) != cudaSuccess ||
-        cudaMemset(b->d_work, 0, sizeof(int) * kBatchWorkInts) != cudaSuccess ||
         cudaMalloc(&b->d_stage, sizeof(float) * 4 * (size_t)maxn) != cudaSuccess)
         return fail_all(NB_ERR_OUT_OF_MEMORY);
     memset(b->h_ctrl, 0, sizeof(Ctrl) * nsys);
     for (int k = 0; k < nsys; ++k) b->h_ctrl[k].budget = -1;  // no step limit
-    if (cudaMemcpy(b->d_ctrl, b->h_ctrl, sizeof(Ctrl) * nsys, cudaMemcpyHostToDevice) != cudaSuccess)
+    // written, cleared and waited for on the batch's own stream: a wait for the
+    // whole device would fail another thread's graph capture
+    if (cudaMemcpyAsync(b->d_ctrl, b->h_ctrl, sizeof(Ctrl) * nsys, cudaMemcpyHostToDevice, b->st) != cudaSuccess)
         return fail_all(NB_ERR_CUDA);
+    auto clear = [&](void *p, size_t bytes) { return cudaMemsetAsync(p, 0, bytes, b->st) == cudaSuccess; };
+    bool cleared = clear(b->d_work, sizeof(int) * kBatchWorkInts);
     b->h_sys.resize(nsys);
     for (int k = 0; k < nsys; ++k) {
         SysMem &m = b->mem[k];
         m.ctrl = b->d_ctrl + k;
-        cudaMemset(m.vel, 0, sizeof(float4) * m.n);
-        cudaMemset(m.acc, 0, sizeof(float4) * m.n);
-        cudaMemset(m.body[0], 0, sizeof(float4) * m.n);
+        const size_t bytes = sizeof(float4) * (size_t)m.n;
+        cleared = cleared && clear(m.vel, bytes) && clear(m.acc, bytes) && clear(m.body[0], bytes);
         int *top_counts = nullptr;
         size_t top_bytes = 0;
         sysmem_top_counts(m, &top_counts, &top_bytes);
-        if (top_bytes) cudaMemset(top_counts, 0, top_bytes);
+        if (top_bytes) cleared = cleared && clear(top_counts, top_bytes);
         b->h_sys[k] = sysmem_desc(m, cfgs[k], 0.0f);
     }
+    if (!cleared) return fail_all(NB_ERR_CUDA);
     if (cudaEventCreate(&b->e0) != cudaSuccess || cudaEventCreate(&b->e1) != cudaSuccess) return fail_all(NB_ERR_CUDA);
     if (rebuild_tables(b) != NB_OK) return fail_all(NB_ERR_CUDA);
-    if (cudaDeviceSynchronize() != cudaSuccess) return fail_all(NB_ERR_CUDA);
+    if (cudaStreamSynchronize(b->st) != cudaSuccess) return fail_all(NB_ERR_CUDA);
     *out = b;
     return NB_OK;
 }

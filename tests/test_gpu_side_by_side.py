@@ -1,6 +1,7 @@
-"""Steps of large trees with the reference's semantics, whose stages are kernels
-of their own, from several threads at once: none of their blocks waits for
-another, so they finish beside one another, each with what it gives alone."""
+"""Handles and batches of several threads at once, each of which gives what it
+gives alone: steps of large trees with the reference's semantics, whose stages
+are kernels of their own and none of whose blocks waits for another, and handles
+created and closed while other threads capture the graphs of their first steps."""
 import threading
 
 import numpy as np
@@ -52,3 +53,48 @@ def test_large_reference_trees(gpu):
             np.testing.assert_array_equal(g, w)
     for s in sims:
         s.close()
+
+
+def test_created_and_closed_side_by_side(gpu):
+    nb = gpu
+    n, rounds = 6007, 12
+    pos, mass = system(n)
+    kind = dict(theta=0.7, epsilon=0.01, gravitational_constant=1.0)
+    tree = nb.default_config(num_of_bodies=n, algo_config=nb.BARNES_HUT, **kind)
+    direct = nb.default_config(num_of_bodies=n, algo_config=nb.BRUTE_FORCE_LOCAL, **kind)
+
+    def handle(cfg):
+        got = []
+        for _ in range(rounds):
+            with nb.Simulation(cfg) as s:
+                s.set_state(pos, mass)
+                got.append((s.step(1e-3, 2, check=False), s.get_state()[:2]))
+        return got
+
+    def batch(cfg):
+        got = []
+        for _ in range(rounds):
+            with nb.Batch([cfg, cfg]) as b:
+                b.set_state(0, pos, mass)
+                b.set_state(1, pos, mass)
+                got.append((b.step(1e-3, 2, check=False), b.get_state(1)[:2]))
+        return got
+
+    def server(cfg):
+        got = []
+        for _ in range(rounds):
+            with nb.Server(max_jobs=4, snapshot_every=0) as v:
+                ids = [v.submit(cfg, 2, 1e-3, pos, mass) for _ in range(3)]
+                got.append((v.wait(), v.result(ids[-1], n)))
+        return got
+
+    work = [lambda: handle(tree), lambda: batch(tree), lambda: handle(direct), lambda: batch(direct),
+            lambda: server(tree), lambda: batch(tree), lambda: handle(tree), lambda: batch(tree)]
+    alone = {k: work[k]()[0] for k in range(5)}
+    alone |= {5: alone[1], 6: alone[0], 7: alone[1]}
+    for k, results in enumerate(run_together(work)):
+        assert results is not None, k
+        for status, got in results:
+            assert status == 0, k
+            for g, w in zip(got, alone[k][1]):
+                np.testing.assert_array_equal(g, w)
