@@ -224,6 +224,14 @@ __device__ __forceinline__ float dist2(const float4 q, float x, float y, float z
     return fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, eps2)));
 }
 
+// max(a, b, 0), not a number where a or b is not: a cell without mass has no
+// centre, and no distance accepts it
+__device__ __forceinline__ float outside(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, 0f00000000;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 __device__ __forceinline__ float warp_min(float v) { return key2f(__reduce_min_sync(0xffffffffu, f2key(v))); }
 __device__ __forceinline__ float warp_max(float v) { return key2f(__reduce_max_sync(0xffffffffu, f2key(v))); }
 
@@ -312,9 +320,9 @@ __device__ __forceinline__ void force_group(const DevSim &s, const StepParams &p
             const int lv = (int)((unsigned)e[h] >> kNodeBits);
             const float thr = dq[lv];
             const bool isb = ch >= 0 && ch < n, isc = ch >= n;
-            const float ex = fmaxf(fmaxf(b0.x - q.x, q.x - b0.w), 0.0f);
-            const float ey = fmaxf(fmaxf(b0.y - q.y, q.y - b1.x), 0.0f);
-            const float ez = fmaxf(fmaxf(b0.z - q.z, q.z - b1.y), 0.0f);
+            const float ex = outside(b0.x - q.x, q.x - b0.w);
+            const float ey = outside(b0.y - q.y, q.y - b1.x);
+            const float ez = outside(b0.z - q.z, q.z - b1.y);
             const float lower = fmaf(ez, ez, fmaf(ey, ey, fmaf(ex, ex, eps2)));
             const bool acc = isc && lower >= thr;
             const bool rej = isc && !acc && (dist2(q, b1.z, b1.w, b2.x, eps2) < thr || dist2(q, b2.y, b2.z, b2.w, eps2) < thr);
