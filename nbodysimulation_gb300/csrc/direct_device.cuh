@@ -2,10 +2,12 @@
 // kernels/brute_force_update.cl), shared by the single-system and
 // allocation-free kernels (k_direct.cu) and the batched one (k_batch.cu).
 //
-// A block of kW warps sums 32 kI targets over the bodies [j0, j1): every warp
-// has all the targets (kI per lane, in registers for the whole sum) and takes
-// every kW-th tile of 64 bodies, at its own pace -- no block barrier until the
-// warps' sums are added, in warp order, at the end.  A lane loads two
+// A block of kW warps sums 32 kI targets over the bodies [j0, j1).  The bodies'
+// tiles of 64 are dealt to eight streams, whatever kW and kI are, so a target's sum
+// depends on the bodies alone: no shape of a batch's kernel changes a result.
+// Every warp has all the targets (kI per lane, in registers for the whole sum) and
+// sums its streams one after another, at its own pace -- no block barrier until the
+// streams' sums are added, in their order, at the end.  A lane loads two
 // consecutive bodies of the next tile while the warp sums this one, and stores
 // them as a pair {x0,x1,y0,y1}, {z0,z1,m0,m1}: what the packed FP32
 // instructions take, so one pair of broadcast loads feeds 2 kI interactions
@@ -25,7 +27,8 @@
 
 namespace nbgb {
 
-constexpr int kDirectTile = 64;  // bodies per tile of one warp: two per lane
+constexpr int kDirectTile = 64;   // bodies per tile of one warp: two per lane
+constexpr int kDirectStreams = 8;  // stream w: tiles w, w + 8, ...
 // how a pair at zero distance counts
 enum { kZeroAdds = 0,      // eps > 0: nothing special
        kZeroSkips = 1,     // eps = 0, update_local's form: adds nothing
@@ -38,9 +41,14 @@ struct DirectTargets {
     float2 ax[kI], ay[kI], az[kI];  // sums over the even and the odd bodies
 };
 
-template <int kW>
+template <int kI, int kW>
 struct __align__(16) DirectShared {
-    float4 tile[kW][2][kDirectTile];  // per warp, double-buffered: 32 x {x0,x1,y0,y1}, 32 x {z0,z1,m0,m1}
+    static_assert(kDirectStreams % kW == 0, "every warp has as many streams");
+    static constexpr bool kOver = kW == kDirectStreams;  // the streams' sums lie where the tiles were
+    static constexpr int kSums = (3 * kI * kDirectStreams * 32 * 4 + 2047) / 2048;  // in warps' tiles
+    static_assert(!kOver || kW >= kSums, "the sums fit in the tiles' memory");
+    float4 tile[kOver ? kW : kW + kSums][2][kDirectTile];  // per warp, double-buffered: 32 x {x0,x1,y0,y1}, 32 x {z0,z1,m0,m1}
+    __device__ __forceinline__ float *sums() { return reinterpret_cast<float *>(tile[kOver ? 0 : kW]); }  // [stream][component][target]
 };
 
 // the reference's brute-force arithmetic: n = normalize(r), s = m / (|n|^2 +
@@ -57,11 +65,11 @@ __device__ __forceinline__ void quirk_pair(float dx, float dy, float dz, float m
     az = fmaf(nz, s, az);
 }
 
-// The warp's part of the sum: tiles w, w + kW, ... of [j0, j1).  i0: index of
-// the lane's first target, its others 32 apart (kZeroSkipsSelf).
-template <int kI, int kW, bool kQuirk, int kZero>
-__device__ __forceinline__ void direct_sum(const float4 *body, int j0, int j1, int i0, float eps, int warp, int lane,
-                                           DirectShared<kW> &sh, DirectTargets<kI> &T) {
+// One stream of [j0, j1).  i0: index of the lane's first target, its others 32
+// apart (kZeroSkipsSelf); buffers: the warp's two tiles.
+template <int kI, bool kQuirk, int kZero>
+__device__ __forceinline__ void direct_stream(const float4 *body, int j0, int j1, int i0, float eps, int stream,
+                                              int lane, float4 (*buffers)[kDirectTile], DirectTargets<kI> &T) {
     const float2 eps2 = dup(eps * eps);
     const int tiles = (j1 - j0 + kDirectTile - 1) / kDirectTile;
     float4 p0, p1;
@@ -73,15 +81,15 @@ __device__ __forceinline__ void direct_sum(const float4 *body, int j0, int j1, i
         if (j >= j1) p0.w = 0.0f;
         if (j + 1 >= j1) p1.w = 0.0f;
     };
-    if (warp < tiles) load(warp);
+    if (stream < tiles) load(stream);
     int buf = 0;
-    for (int t = warp; t < tiles; t += kW) {
-        float4 *tl = sh.tile[warp][buf];
+    for (int t = stream; t < tiles; t += kDirectStreams) {
+        float4 *tl = buffers[buf];
         buf ^= 1;
         tl[lane] = make_float4(p0.x, p1.x, p0.y, p1.y);
         tl[32 + lane] = make_float4(p0.z, p1.z, p0.w, p1.w);
         __syncwarp();  // also: the tile before last is no longer read
-        if (t + kW < tiles) load(t + kW);
+        if (t + kDirectStreams < tiles) load(t + kDirectStreams);
 #pragma unroll 4
         for (int k = 0; k < kDirectTile / 2; ++k) {
             const float4 xy = tl[k], zm = tl[32 + k];
@@ -114,35 +122,6 @@ __device__ __forceinline__ void direct_sum(const float4 *body, int j0, int j1, i
     }
 }
 
-// Adds the warps' sums in warp order.  Every thread of the block calls it;
-// thread t < 32 kI gets the sum of target number t of the block.
-template <int kI, int kW>
-__device__ __forceinline__ float3 direct_block_sum(DirectShared<kW> &sh, const DirectTargets<kI> &T, int warp,
-                                                   int lane) {
-    static_assert(kW >= kI, "a thread for every target");
-    static_assert(sizeof(DirectShared<kW>) >= sizeof(float) * 3 * 32 * kI * kW, "the sums fit in the tiles' memory");
-    float *red = reinterpret_cast<float *>(&sh);  // [warp][component][target]
-    __syncthreads();                              // the tiles are no longer read
-#pragma unroll
-    for (int r = 0; r < kI; ++r) {
-        float *at = red + warp * (3 * 32 * kI) + 32 * r + lane;
-        at[0] = T.ax[r].x + T.ax[r].y;
-        at[32 * kI] = T.ay[r].x + T.ay[r].y;
-        at[64 * kI] = T.az[r].x + T.az[r].y;
-    }
-    __syncthreads();
-    float3 a = make_float3(0.0f, 0.0f, 0.0f);
-    for (int t = threadIdx.x; t < 32 * kI; t += 32 * kW) {  // one round: a block has 32 kW >= 32 kI threads
-        for (int w = 0; w < kW; ++w) {
-            const float *at = red + w * (3 * 32 * kI) + t;
-            a.x += at[0];
-            a.y += at[32 * kI];
-            a.z += at[64 * kI];
-        }
-    }
-    return a;
-}
-
 template <int kI>
 __device__ __forceinline__ void direct_load_targets(const float4 *body, int i0, int n, DirectTargets<kI> &T) {
 #pragma unroll
@@ -153,6 +132,52 @@ __device__ __forceinline__ void direct_load_targets(const float4 *body, int i0, 
         T.nz[r] = dup(-P.z);
         T.ax[r] = T.ay[r] = T.az[r] = make_float2(0.0f, 0.0f);
     }
+}
+
+// The streams' sums of the block's targets (the first one `base`).  Every thread
+// of the block calls it.
+template <int kI, int kW, bool kQuirk, int kZero>
+__device__ __forceinline__ void direct_sum(const float4 *body, int n, int j0, int j1, int base, float eps, int warp,
+                                           int lane, DirectShared<kI, kW> &sh) {
+    const int i0 = base + lane;
+    DirectTargets<kI> T;
+    direct_load_targets<kI>(body, i0, n, T);
+    const auto store = [&](int stream) {
+#pragma unroll
+        for (int r = 0; r < kI; ++r) {
+            float *at = sh.sums() + stream * (3 * 32 * kI) + 32 * r + lane;
+            at[0] = T.ax[r].x + T.ax[r].y;
+            at[32 * kI] = T.ay[r].x + T.ay[r].y;
+            at[64 * kI] = T.az[r].x + T.az[r].y;
+        }
+    };
+    if constexpr (DirectShared<kI, kW>::kOver) {
+        direct_stream<kI, kQuirk, kZero>(body, j0, j1, i0, eps, warp, lane, sh.tile[warp], T);
+        __syncthreads();  // the tiles are no longer read
+        store(warp);
+    } else {
+        for (int stream = warp; stream < kDirectStreams; stream += kW) {
+            direct_stream<kI, kQuirk, kZero>(body, j0, j1, i0, eps, stream, lane, sh.tile[warp], T);
+            store(stream);
+#pragma unroll
+            for (int r = 0; r < kI; ++r) T.ax[r] = T.ay[r] = T.az[r] = make_float2(0.0f, 0.0f);
+            __syncwarp();  // the next stream's tiles go where this one's were read
+        }
+    }
+    __syncthreads();
+}
+
+// the sum of target number t of the block: the streams' in order
+template <int kI, int kW>
+__device__ __forceinline__ float3 direct_target_sum(DirectShared<kI, kW> &sh, int t) {
+    float3 a = make_float3(0.0f, 0.0f, 0.0f);
+    for (int w = 0; w < kDirectStreams; ++w) {
+        const float *at = sh.sums() + w * (3 * 32 * kI) + t;
+        a.x += at[0];
+        a.y += at[32 * kI];
+        a.z += at[64 * kI];
+    }
+    return a;
 }
 
 }  // namespace nbgb

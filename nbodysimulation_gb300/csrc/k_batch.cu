@@ -101,12 +101,11 @@ __global__ void __maxnreg__(kMany ? 96 : 128) k_batch_force(BatchTables t) {
 // ---------------------------------------------------------------------------
 // direct: one block per 32 kI targets of one system, its kW warps sharing the
 // system's bodies (direct_device.cuh); Plummer softening; fused integrator.  kI
-// and kW come from the autotuner; a system's sums depend on them and on nothing
-// beside it.
+// and kW come from the autotuner; a system's sums do not depend on them.
 // ---------------------------------------------------------------------------
 template <int kI, int kW>
 __global__ void __launch_bounds__(32 * kW) k_batch_direct(BatchTables t) {
-    __shared__ DirectShared<kW> sh;
+    __shared__ DirectShared<kI, kW> sh;
     const int k = find_system(t.dblock_prefix, t.nsys, blockIdx.x);
     const SysDesc &d = t.sys[k];
     if (!system_live(d.v.ctrl)) return;  // block-uniform, before any barrier
@@ -114,14 +113,13 @@ __global__ void __launch_bounds__(32 * kW) k_batch_direct(BatchTables t) {
     StepParams p = d.p;
     p.kdk_primed = s.ctrl->kdk_primed;
     const int n = s.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int base = (blockIdx.x - d.dblock_begin) * (32 * kI), i0 = base + lane;
-    DirectTargets<kI> T;
-    direct_load_targets<kI>(s.body_cur, i0, n, T);
-    direct_sum<kI, kW, false, kZeroAdds>(s.body_cur, 0, n, i0, p.eps, warp, lane, sh, T);
-    const float3 a = direct_block_sum<kI, kW>(sh, T, warp, lane);
-    const int i = base + (int)threadIdx.x;
-    if (threadIdx.x < 32 * kI && i < n)
-        integrate_any(s, p, i, s.body_cur[i], a.x * p.G, a.y * p.G, a.z * p.G);
+    const int base = (blockIdx.x - d.dblock_begin) * (32 * kI);
+    direct_sum<kI, kW, false, kZeroAdds>(s.body_cur, n, 0, n, base, p.eps, warp, lane, sh);
+    for (int q = threadIdx.x; q < 32 * kI; q += 32 * kW) {  // one round where kW >= kI
+        const float3 a = direct_target_sum<kI, kW>(sh, q);
+        const int i = base + q;
+        if (i < n) integrate_any(s, p, i, s.body_cur[i], a.x * p.G, a.y * p.G, a.z * p.G);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -167,8 +165,8 @@ __global__ void __launch_bounds__(kCollideThreads) k_batch_collision(BatchTables
 struct DirectVariant {
     int ki, warps;
 };
-static const DirectVariant kDirectVariants[] = {{1, 4}, {1, 8},  {2, 4}, {2, 8},  {4, 4}, {4, 8},
-                                                {1, 2}, {1, 16}, {2, 2}, {2, 16}, {4, 16}};
+static const DirectVariant kDirectVariants[] = {{1, 4}, {1, 8}, {2, 4}, {2, 8}, {4, 4}, {4, 8},
+                                                {1, 2}, {1, 1}, {2, 2}, {2, 1}, {4, 2}};
 constexpr int kNumDirectVariants = sizeof(kDirectVariants) / sizeof(kDirectVariants[0]);
 static_assert(kBatchDirectDefault < kNumDirectVariants, "the default is one of the variants");
 
@@ -185,10 +183,10 @@ static cudaError_t launch_direct_variant(const BatchTables &t, int variant, cuda
     case 4: k_batch_direct<4, 4><<<b, 128, 0, st>>>(t); break;
     case 5: k_batch_direct<4, 8><<<b, 256, 0, st>>>(t); break;
     case 6: k_batch_direct<1, 2><<<b, 64, 0, st>>>(t); break;
-    case 7: k_batch_direct<1, 16><<<b, 512, 0, st>>>(t); break;
+    case 7: k_batch_direct<1, 1><<<b, 32, 0, st>>>(t); break;
     case 8: k_batch_direct<2, 2><<<b, 64, 0, st>>>(t); break;
-    case 9: k_batch_direct<2, 16><<<b, 512, 0, st>>>(t); break;
-    default: k_batch_direct<4, 16><<<b, 512, 0, st>>>(t); break;
+    case 9: k_batch_direct<2, 1><<<b, 32, 0, st>>>(t); break;
+    default: k_batch_direct<4, 2><<<b, 64, 0, st>>>(t); break;
     }
     return cudaGetLastError();
 }

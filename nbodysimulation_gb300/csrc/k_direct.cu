@@ -20,23 +20,22 @@ namespace nbgb {
 // of each set that are done; the last one puts it back to zero.
 // out (allocation-free form): accelerations instead of the integrator.
 // ---------------------------------------------------------------------------
-constexpr int kDirectWarps = 8;
+constexpr int kDirectWarps = kDirectStreams;
 template <int kI, bool kQuirk, int kZero>
 __global__ void __launch_bounds__(32 * kDirectWarps, kI == 4 ? 2 : 3)
     k_direct(DevSim s, StepParams p, float4 *part, int *arrived, float4 *out) {
     wait_for_previous();
-    __shared__ DirectShared<kDirectWarps> sh;
+    __shared__ DirectShared<kI, kDirectWarps> sh;
     __shared__ int last;
     const int n = s.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int base = blockIdx.x * (32 * kI), i0 = base + lane;
+    const int base = blockIdx.x * (32 * kI);
     // slices of whole tiles
     const int tiles = (n + kDirectTile - 1) / kDirectTile;
     const int per = (tiles + gridDim.y - 1) / gridDim.y * kDirectTile;
     const int j0 = blockIdx.y * per, j1 = min(n, j0 + per);
-    DirectTargets<kI> T;
-    direct_load_targets<kI>(s.body_cur, i0, n, T);
-    direct_sum<kI, kDirectWarps, kQuirk, kZero>(s.body_cur, j0, j1, i0, p.eps, warp, lane, sh, T);
-    float3 a = direct_block_sum<kI, kDirectWarps>(sh, T, warp, lane);
+    direct_sum<kI, kDirectWarps, kQuirk, kZero>(s.body_cur, n, j0, j1, base, p.eps, warp, lane, sh);
+    float3 a = make_float3(0.0f, 0.0f, 0.0f);
+    if (threadIdx.x < 32 * kI) a = direct_target_sum<kI, kDirectWarps>(sh, threadIdx.x);
     const int i = base + (int)threadIdx.x;
     const bool mine = threadIdx.x < 32 * kI && i < n;
     if (gridDim.y > 1) {
