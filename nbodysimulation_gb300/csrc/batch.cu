@@ -96,12 +96,14 @@ static nb_status rebuild_tables(nb_batch *b) {
     return NB_OK;
 }
 
+// The keys of the tuning cache name what the numbers under them stand for, so
+// that a file of a build with other shapes is not taken for this one's.
 static std::string tune_key(const nb_batch *b) {
     std::map<int, int> hist;  // log2 size bucket of the direct systems
     for (int k = 0; k < b->nsys; ++k)
         if (b->h_sys[k].kind == kSysDirect) hist[(int)std::floor(std::log2((double)b->mem[k].n))] += 1;
     std::ostringstream os;
-    os << "batch_direct/sm" << b->sm;
+    os << "batch_direct/" << batch_direct_names() << "/sm" << b->sm;
     for (auto &kv : hist) os << "/" << kv.first << "x" << kv.second;
     return os.str();
 }
@@ -503,7 +505,7 @@ static std::string tree_tune_key(const nb_batch *b) {
     for (int k = 0; k < b->nsys; ++k)
         if (b->h_sys[k].kind == kSysBH) hist[(int)std::floor(std::log2((double)b->mem[k].n))] += 1;
     std::ostringstream os;
-    os << "batch_tree/sm" << b->sm << "/quad" << b->quad << "/comp" << b->comp;
+    os << "batch_tree/paths/sm" << b->sm << "/quad" << b->quad << "/comp" << b->comp;
     for (auto &kv : hist) os << "/" << kv.first << "x" << kv.second;
     return os.str();
 }

@@ -8,6 +8,8 @@
 // (direct_device.cuh).  A step is: box, paths, places, ranks, cells, sums in
 // tiles, sums above, insertions, force, direct, flip -- captured once into a CUDA
 // graph by the host.
+#include <string>
+
 #include "collide_device.cuh"
 #include "direct_device.cuh"
 #include "force_device.cuh"
@@ -171,6 +173,12 @@ constexpr int kNumDirectVariants = sizeof(kDirectVariants) / sizeof(kDirectVaria
 static_assert(kBatchDirectDefault < kNumDirectVariants, "the default is one of the variants");
 
 int batch_direct_variants() { return kNumDirectVariants; }
+std::string batch_direct_names() {  // "1w4.1w8. ...": targets per lane, warps
+    std::string s;
+    for (const DirectVariant &v : kDirectVariants)
+        s += (s.empty() ? "" : ".") + std::to_string(v.ki) + "w" + std::to_string(v.warps);
+    return s;
+}
 int batch_direct_block_bodies(int variant) { return 32 * kDirectVariants[variant].ki; }
 
 static cudaError_t launch_direct_variant(const BatchTables &t, int variant, cudaStream_t st) {

@@ -17,6 +17,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <string>
+
 namespace nbgb {
 
 constexpr int kMaxDepth = 64;
@@ -383,6 +385,7 @@ inline int batch_chunk(int n, long long batch_tree_bodies) {
 }
 constexpr int kBatchDirectDefault = 3;  // the variant of a batch that is not tuned
 int batch_direct_variants();
+std::string batch_direct_names();  // of all variants, in order
 int batch_direct_block_bodies(int variant);
 // Optional second stream of a captured batched step: the small systems'
 // direct sum runs on it beside the tree stages (a parallel branch of the

@@ -51,3 +51,27 @@ def test_served_variants(gpu, variant):
         ids = [s.submit(cfg(nb, n, False, 3), 3, 1e-3, *st) for n, st in zip(SIZES, states())]
         assert s.wait() == 0
         same([s.result(job, n) for job, n in zip(ids, SIZES)], batched(nb, False))
+
+
+def test_cache_of_another_build(gpu, tmp_path):
+    """Numbers that an earlier build wrote for its shapes name other kernels here:
+    its entries are left alone and the batch is tuned."""
+    import json
+
+    nb = gpu
+    cache = tmp_path / "tune.json"
+    sizes = [(600, False), (3000, False), (5000, True)]
+
+    def tune():
+        with nb.Batch([cfg(nb, n, tree) for n, tree in sizes]) as b:
+            for k, (n, _) in enumerate(sizes):
+                rng = np.random.default_rng(n)
+                b.set_state(k, rng.normal(size=(n, 3)).astype(np.float32), np.full(n, 1.0 / n, np.float32))
+            b.autotune(str(cache))
+        return json.loads(cache.read_text())
+
+    sm = next(p for p in next(iter(tune())).split("/") if p.startswith("sm"))
+    old = {f"batch_direct/{sm}/9x1/11x1": 10, f"batch_tree/{sm}/quad0/comp0/12x1": 107}
+    cache.write_text(json.dumps(old))
+    table = tune()
+    assert len(table) == 4 and {k: table[k] for k in old} == old
