@@ -545,8 +545,8 @@ static cudaError_t time_shapes(nb_batch *b, float *ms) {
     return e;
 }
 
-// One pass of coordinate descent over the four shape parameters (top-level
-// cap, build chunk, warps per block, grid fraction), each timed in whole
+// One pass of coordinate descent over the shape parameters (top-level cap and
+// build chunk where trees insert, warps per block, grid fraction), each timed in whole
 // steps of this batch; every shape gives the same results, only the time
 // differs.
 static nb_status tune_tree_shape(nb_batch *b, TreeShape &best) {
@@ -575,8 +575,14 @@ static nb_status tune_tree_shape(nb_batch *b, TreeShape &best) {
         }
     };
     trial(best);
-    for (int v : kTuneLevels) { TreeShape t = best; t.top_levels = v; if (v != best.top_levels) trial(t); }
-    for (int v : kTuneChunk) { TreeShape t = best; t.build_chunk = v; if (v != best.build_chunk) trial(t); }
+    // two of the parameters are the insertions': without any in the timed steps the
+    // clock's noise would choose what a step that has them runs with
+    bool inserts = false;
+    for (int k = 0; k < b->nsys; ++k) inserts |= b->h_sys[k].kind == kSysBH && b->h_ctrl[k].insert != 0;
+    if (inserts) {
+        for (int v : kTuneLevels) { TreeShape t = best; t.top_levels = v; if (v != best.top_levels) trial(t); }
+        for (int v : kTuneChunk) { TreeShape t = best; t.build_chunk = v; if (v != best.build_chunk) trial(t); }
+    }
     for (int v : kTuneWarps) { TreeShape t = best; t.force_warps = v; if (v != best.force_warps) trial(t); }
     for (int v : kTunePct) { TreeShape t = best; t.force_grid_pct = v; if (v != best.force_grid_pct) trial(t); }
     for (auto &d : b->h_sys) d.p.dt = keep_dt;
