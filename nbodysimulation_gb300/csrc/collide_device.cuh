@@ -147,9 +147,11 @@ __device__ __forceinline__ void collide_warp(const float4 *pos, float4 *vel, int
     float4 v = vel[i];
     const float rr = contact_distance();
     const bool me_finite = finite3(me);
+    float4 next = lane < n ? pos[lane] : me;
     for (int j0 = 0; j0 < n; j0 += 32) {
         const int j = j0 + lane;
-        const float4 q = j < n ? pos[j] : me;
+        const float4 q = next;
+        if (j + 32 < n) next = pos[j + 32];  // on its way during the votes, which no load passes
         const bool fast = me_finite && finite3(q);
         unsigned hit = __ballot_sync(0xffffffffu, j < n && j != i && in_contact(me, q, rr, fast));
         while (hit) {

@@ -49,6 +49,12 @@ __global__ void __launch_bounds__(kCollideWarps * 32) k_collision_warp(DevSim s)
 // ---------------------------------------------------------------------------
 constexpr int kGridThreads = 128;
 constexpr int kGridContacts = 64;
+// A target with more than n / 128 bodies around it goes to the overflow list at
+// once: a thread takes 0.4 us a candidate where nothing hides its latencies, a warp
+// n / 32 steps of 0.1 us for a target.  Targets ask for it where some bucket holds
+// more than its share of that, and more than kGridQuiet.
+constexpr int kGridCrowd = 128;
+constexpr int kGridQuiet = 8;
 constexpr int kScanBuckets = 1024;  // buckets per block of the scan: consecutive in memory
 constexpr float kGridLimit = 262144.0f;
 
@@ -94,6 +100,7 @@ __global__ void __launch_bounds__(kScanBuckets / 4) k_grid_scan(DevSim s, Collid
     const int at = blockIdx.x * (kScanBuckets / 4) + threadIdx.x;
     const int4 c = reinterpret_cast<const int4 *>(g.count)[at];
     const int sum = c.x + c.y + c.z + c.w;
+    if (max(max(c.x, c.y), max(c.z, c.w)) > max(kGridQuiet, s.n / (27 * kGridCrowd))) g.ctl[kGridCrowded] = 1;
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -143,11 +150,20 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_collide(DevSim s, Collide
     const float inv = grid_inv(), rr = contact_distance();
     GridCell c;
     grid_cell(me, inv, c);
+    // the rows' three buckets: one range when the scan laid them end to end
     int cnt = 0;
-    for (int row = 0; row < 9; ++row) {
+    if (g.ctl[kGridCrowded]) {
+        int crowd = 0;
+#pragma unroll
+        for (int row = 0; row < 9; ++row) {
+            const unsigned b0 = (grid_row(c.y + row / 3 - 1, c.z + row % 3 - 1) + (unsigned)(c.x - 1)) & g.mask;
+            if ((b0 & (kScanBuckets - 1)) + 2 < kScanBuckets) crowd += g.start[b0 + 2] + g.count[b0 + 2] - g.start[b0];
+        }
+        if (crowd > s.n / kGridCrowd) cnt = kGridContacts + 1;
+    }
+    for (int row = 0; row < 9 && cnt <= kGridContacts; ++row) {
         const int cy = c.y + row / 3 - 1, cz = c.z + row % 3 - 1;
         const unsigned b0 = (grid_row(cy, cz) + (unsigned)(c.x - 1)) & g.mask;
-        // three buckets in one range when the scan laid them end to end
         const bool whole = (b0 & (kScanBuckets - 1)) + 2 < kScanBuckets;
         for (int part = 0; part < (whole ? 1 : 3); ++part) {
             const unsigned first = (b0 + part) & g.mask, last = whole ? b0 + 2 : first;
@@ -185,20 +201,40 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_collide(DevSim s, Collide
     s.vel[i] = v;
 }
 
-// What the grid left: every target when some body has no cell, else the
-// targets of the overflow list.  Few of them take one warp each, many one
-// thread each (as collide_warp_form_below decides between whole systems).
-__global__ void __launch_bounds__(kCollideThreads) k_grid_rest(DevSim s, CollideGrid g, const int *order, int few) {
+// What the grid left: every target when some body has no cell, else the targets
+// of the overflow list.  Few of them take one warp each, many one thread each, as
+// collide_warp_form_below decides between whole systems.
+//
+// The warps' form.  Targets' times differ with their contacts, so after the first
+// one a warp draws the next; a block per eight targets did as well, but blocks that
+// find nothing to do cost 6 us at 38,000 bodies.  Not inlined: around the loop the
+// compiler gives it 42 registers, or spills (38,000 targets, one body far out: 1.57
+// ms, with 42 registers 1.89, a warp a target and no grid before it 1.47).
+__device__ __noinline__ void collide_one(const float4 *pos, float4 *vel, int n, int i) {
+    collide_warp(pos, vel, n, i, threadIdx.x & 31);
+}
+__device__ __forceinline__ void rest_by_warps(const DevSim &s, const CollideGrid &g, bool all, int cnt) {
+    const int warps = gridDim.x * kCollideWarps;
+    for (int k = blockIdx.x * kCollideWarps + (threadIdx.x >> 5); k < cnt;) {
+        collide_one(s.body_next, s.vel, s.n, all ? k : g.rank[k]);
+        if (cnt <= warps) return;
+        if ((threadIdx.x & 31) == 0) k = warps + atomicAdd(&g.ctl[kGridNext], 1);
+        k = __shfl_sync(0xffffffffu, k, 0);
+    }
+}
+// systems that cannot have many
+__global__ void __launch_bounds__(kCollideWarps * 32, 8) k_grid_rest_few(DevSim s, CollideGrid g) {
+    wait_for_previous();
+    if (read_status(s.ctrl)) return;  // warp-uniform
+    const bool all = g.ctl[kGridNoCell] != 0;
+    rest_by_warps(s, g, all, all ? s.n : g.ctl[kGridOverflow]);
+}
+__global__ void __launch_bounds__(kCollideThreads, 8) k_grid_rest(DevSim s, CollideGrid g, const int *order, int few) {
     wait_for_previous();
     if (read_status(s.ctrl)) return;  // block-uniform, before any barrier
     const bool all = g.ctl[kGridNoCell] != 0;
     const int cnt = all ? s.n : g.ctl[kGridOverflow];
-    if (cnt < few) {
-        const int lane = threadIdx.x & 31;
-        for (int k = blockIdx.x * kCollideWarps + (threadIdx.x >> 5); k < cnt; k += gridDim.x * kCollideWarps)
-            collide_warp(s.body_next, s.vel, s.n, all ? k : g.rank[k], lane);
-        return;
-    }
+    if (cnt < few) return rest_by_warps(s, g, all, cnt);
     if ((int)blockIdx.x * kCollideThreads >= cnt) return;
     collide_block(s.body_next, s.vel, all ? order : g.rank, cnt, s.n, blockIdx.x * kCollideThreads, s.ctrl);
 }
@@ -220,10 +256,16 @@ cudaError_t launch_collision(const DevSim &s, const CollideGrid &g, int tree, in
     if (e == cudaSuccess) e = launch_next(k_grid_place, blocks, 256, st, s, g);
     if (e == cudaSuccess)
         e = launch_next(k_grid_collide, (s.n + kGridThreads - 1) / kGridThreads, kGridThreads, st, s, g);
-    if (e == cudaSuccess)
-        e = launch_next(k_grid_rest, (s.n + kCollideThreads - 1) / kCollideThreads, kCollideThreads, st, s, g,
-                        tree ? s.sorted : nullptr, collide_warp_form_below(sm_count) * kCollideThreads);
-    return e;
+    if (e != cudaSuccess) return e;
+    const int few = collide_warp_form_below(sm_count) * kCollideThreads;
+    if (s.n < few)
+        return launch_next(k_grid_rest_few, std::min((s.n + kCollideWarps - 1) / kCollideWarps, 8 * sm_count),
+                           kCollideWarps * 32, st, s, g);
+    // not early, so that the block form's few long blocks spread evenly (launch.cuh;
+    // 60,001 bodies, one far out: 3.50 ms, early 4.02)
+    k_grid_rest<<<(s.n + kCollideThreads - 1) / kCollideThreads, kCollideThreads, 0, st>>>(
+        s, g, tree ? s.sorted : nullptr, few);
+    return cudaGetLastError();
 }
 
 }  // namespace nbgb
