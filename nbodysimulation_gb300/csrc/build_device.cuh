@@ -39,7 +39,24 @@ __device__ __forceinline__ int common_levels(u64 a, u64 b) {
 __device__ __forceinline__ int octant_at(u64 key, int level) { return (int)(key >> (3 * (kPathLevels - 1 - level))) & 7; }
 __device__ __forceinline__ bool build_off(const Ctrl *c) { return read_status(c) != 0 || c->insert != 0; }
 
-// Path of body i; its region and its place there.
+// Crowded regions: a block ranks its bodies against all of their regions, at 20 to
+// 60 ns a body there, which the insertions beat from some number of bodies in one
+// region on, the larger the system the later, or when the system has more than
+// kPairsPerBody pairs a body.  (Normal positions and one body far out, ms up to the
+// sums, insertions / ranking, by the most bodies in a region: 4,000 of 4,000 0.14 /
+// 0.14; 3,433 of 20,000 0.17 / 0.29, 6,089 0.17 / 0.41; 4,047 of 30,011 0.18 / 0.30;
+// 8,402 of 262,144 0.39 / 0.60; 4,870 of 1,000,003 0.83 / 0.70.)  With the
+// reference's semantics, whose boxes part bodies later, a system that is all in one
+// region mostly inserts in the end (3,000 bodies 0.15, ranked first 0.22).
+constexpr int kCrowd = 2048;
+constexpr int kPairsPerBody = 4096;
+__device__ __forceinline__ int crowd_limit(int n, int ref) {
+    return !ref && n <= 2 * kCrowd ? n : kCrowd + (n >> 6);
+}
+
+// Path of body i; its region and its place there.  One body too many in a region
+// sends the step to the insertions (it alone: a store by every body behind it took
+// 0.3 ms).
 template <class Geo>
 __device__ __forceinline__ void path_body(const DevSim &s, const BuildScratch &b, const Geo &root, int i) {
     constexpr int kLevels = std::is_same<Geo, RefBox>::value ? kPathLevels - 1 : kPathLevels;
@@ -51,20 +68,17 @@ __device__ __forceinline__ void path_body(const DevSim &s, const BuildScratch &b
         const int r = region_of(key, b), lane = threadIdx.x & 31;
         const unsigned active = __activemask();
         const int first = __ffs(active) - 1;
+        int at = 0;
         if (__all_sync(active, r == __shfl_sync(active, r, first))) {
-            int at = 0;
             if (lane == first) at = atomicAdd(&b.count[r], __popc(active));
-            b.rank[i] = __shfl_sync(active, at, first) + __popc(active & ((1u << lane) - 1u));
+            at = __shfl_sync(active, at, first) + __popc(active & ((1u << lane) - 1u));
         } else {
-            b.rank[i] = atomicAdd(&b.count[r], 1);
+            at = atomicAdd(&b.count[r], 1);
         }
+        b.rank[i] = at;
+        if (at == crowd_limit(s.n, b.ref)) s.ctrl->insert = 1;
     }
 }
-
-// more pairs to compare than this a body and the insertions are faster (all
-// bodies in one region, insertions / ranking, a step: 3,000 bodies 0.20 / 0.17
-// ms, 10,000 0.22 / 0.31)
-constexpr int kPairsPerBody = 4096;
 
 // Body i into its region.
 __device__ __forceinline__ void place_body(const BuildScratch &b, int i) {

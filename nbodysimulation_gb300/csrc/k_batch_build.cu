@@ -203,23 +203,26 @@ __global__ void __launch_bounds__(kTile) k_batch_path(BatchTables t) {
     __shared__ int last;
     const BuildSystem v = build_system(t, blockIdx.x, kTileBlocks);
     const int blocks = (v.s.n + kTile - 1) / kTile;
-    if (v.part >= blocks || left_alone(v.s.ctrl)) return;  // block-uniform: the last block sets `insert`
-    float box[6];
-    load_box(v.s.ctrl, box);
+    Ctrl *c = v.s.ctrl;
+    // block-uniform: only earlier kernels set a status (`insert` may appear meanwhile)
+    if (v.part >= blocks || !system_live(c) || read_status(c)) return;
     const int i = v.part * kTile + threadIdx.x;
-    if (i < v.s.n) {
+    if (i < v.s.n && !ld_volatile(&c->insert)) {
+        float box[6];
+        load_box(c, box);
         if (v.b.ref) path_body(v.s, v.b, RefBox::root(box), i);
         else path_body(v.s, v.b, GeoCube::root(box), i);
     }
     __syncthreads();  // the block's counts are in (its atomics have returned)
     if (threadIdx.x == 0) {
         __threadfence();
-        last = atomicAdd(&v.s.ctrl->work, 1) == blocks - 1;
+        last = atomicAdd(&c->work, 1) == blocks - 1;
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
-    if (threadIdx.x == 0) v.s.ctrl->work = 0;
+    if (threadIdx.x == 0) c->work = 0;
+    if (ld_volatile(&c->insert)) return;  // every block has arrived
     scan_regions(v.s, v.b);
 }
 

@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(256) k_path(DevSim s, BuildScratch b) {
     if (build_off(s.ctrl)) return;
     float box[6];
     load_box(s.ctrl, box);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    for (int i = first; i < s.n; i += stride) {
+        if (i > first && ld_volatile(&s.ctrl->insert)) return;  // a crowded region: the paths are of no use
         if (b.ref) path_body(s, b, RefBox::root(box), i);
         else path_body(s, b, GeoCube::root(box), i);
     }
