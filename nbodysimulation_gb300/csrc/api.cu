@@ -322,7 +322,7 @@ nb_status nb_create(const nb_config *cfg, nb_sim **out) {
         return cleanup(NB_ERR_CUDA);
     if (!s->tree) s->arrived = zeroed;
     // the build's paths and places lie in the transfer staging, which no step uses
-    else if (tables) s->build = build_scratch(s->n, s->sm_count, ref, zeroed, s->part, s->stage3);
+    else if (tables) s->build = build_scratch(s->n, ref, zeroed, s->part, s->stage3);
     s->quad = cfg->multipole == NB_MULTIPOLE_QUADRUPOLE;
     if (s->tree) {
         int cap = cfg->cell_capacity > 0 ? cfg->cell_capacity : default_capacity(s->n, s->sm_count);

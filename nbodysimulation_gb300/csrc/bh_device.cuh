@@ -242,7 +242,7 @@ __device__ __forceinline__ void top_count_range(const DevSim &s, const TopTables
 // the level-L counts for the next step in every case.   Every thread of
 // the block calls it; blockDim.x is a power of two with 8^L <= 32 *
 // blockDim.x, so a thread takes at most 32 regions of a level and a level has
-// at most kTopRegions / 32 (round, warp) pairs.
+// at most 8^L / 32 (round, warp) pairs.
 __device__ __forceinline__ void top_cells_block(const DevSim &s, const TopTables &t) {
     constexpr int kRegions = 1 << (3 * kBatchTopMaxLevels), kInner = (kRegions - 8) / 7;
     __shared__ int cnt_sh[kInner];          // body counts, regions of levels 1..L-1

@@ -373,7 +373,7 @@ size_t build_scratch_ints(int n, int sm_count) {
     return kBuildCtl + kScanBlocks + (size_t)6 * 4 * sm_count + build_top_cells(n) + 2 * regions + 4;
 }
 
-BuildScratch build_scratch(int n, int sm_count, int ref, int *mem, void *keys16, void *ints12) {
+BuildScratch build_scratch(int n, int ref, int *mem, void *keys16, void *ints12) {
     BuildScratch b{};
     b.ref = ref;
     b.levels = build_levels(n);
@@ -389,7 +389,6 @@ BuildScratch build_scratch(int n, int sm_count, int ref, int *mem, void *keys16,
     b.rank = static_cast<int *>(ints12);
     b.who = b.rank + n;
     b.base = b.who + n;
-    (void)sm_count;
     return b;
 }
 

@@ -6,15 +6,16 @@
 
 namespace nbgb {
 
-// kBlocks: resident blocks per SM the registers allow.  Eight (128 registers),
-// or nine (96) where the groups fill the GPU more than twice over: the extra
-// warps then hide more of the walk than its tighter schedule costs.  With
-// quadrupoles and without compensation they do not (GB300, the walk in ms,
-// eight / nine blocks: monopoles, ball, 6,007 bodies 0.0635 / 0.0657, 131,072
-// 0.207 / 0.207, 200,000 0.290 / 0.287, 262,144 0.365 / 0.353, 1,000,000 1.303 /
-// 1.246; quadrupoles compensated, 200,000 0.522 / 0.515, 4,194,304 11.78 / 11.57;
-// quadrupoles, 1,000,000 1.305 / 1.310; ten blocks 0.362 and 11.99 where nine
-// take 0.353 and 11.57).
+// kBlocks: the launch bound that the registers follow.  Eight blocks per SM (128
+// registers), or nine (96) where the groups fill the GPU more than twice over.
+// What is resident follows from the shared memory too: of monopoles ten blocks with
+// 96 registers, whose extra warps hide more of the walk than its tighter schedule
+// costs; of compensated quadrupoles eight either way (26 KB a block), where the
+// schedule itself is the faster one.  With quadrupoles and without compensation
+// neither is (GB300, the walk in ms, bound eight / nine: monopoles, ball, 6,007
+// bodies 0.0635 / 0.0657, 131,072 0.207 / 0.207, 200,000 0.290 / 0.287, 262,144
+// 0.365 / 0.353, 1,000,000 1.303 / 1.246; quadrupoles compensated, 200,000 0.522 /
+// 0.515, 4,194,304 11.78 / 11.57; quadrupoles, 1,000,000 1.305 / 1.310).
 constexpr int kFewGroups = 8, kManyGroups = 9;
 template <int kMethod, bool kComp, bool kEpsZero, bool kQuad, int kBlocks>
 __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force(DevSim s, StepParams p) {
@@ -69,10 +70,10 @@ static cudaError_t launch_force_b(const DevSim &s, const StepParams &p, int sm_c
 
 template <int kMethod, bool kComp, bool kQuad>
 static cudaError_t launch_force_t(const DevSim &s, const StepParams &p, int sm_count, cudaStream_t st) {
-    if constexpr (kQuad && !kComp) return launch_force_b<kMethod, kComp, kQuad, kFewGroups>(s, p, sm_count, st);
-    const bool many = (s.n + 31) / 32 >= 2 * kFewGroups * kForceWarps * sm_count;
-    return many ? launch_force_b<kMethod, kComp, kQuad, kManyGroups>(s, p, sm_count, st)
-                : launch_force_b<kMethod, kComp, kQuad, kFewGroups>(s, p, sm_count, st);
+    if constexpr (!kQuad || kComp)
+        if ((s.n + 31) / 32 >= 2 * kFewGroups * kForceWarps * sm_count)
+            return launch_force_b<kMethod, kComp, kQuad, kManyGroups>(s, p, sm_count, st);
+    return launch_force_b<kMethod, kComp, kQuad, kFewGroups>(s, p, sm_count, st);
 }
 
 template <int kMethod>

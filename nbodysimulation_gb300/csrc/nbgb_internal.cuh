@@ -298,18 +298,13 @@ inline size_t batch_build_ints(int n, int ref) {
 size_t build_scratch_ints(int n, int sm_count);
 // mem: build_scratch_ints ints, zeroed; keys16 / ints12: 16 n and 12 n bytes
 // that the step may overwrite
-BuildScratch build_scratch(int n, int sm_count, int ref, int *mem, void *keys16, void *ints12);
+BuildScratch build_scratch(int n, int ref, int *mem, void *keys16, void *ints12);
 // bbox; paths, sort and cells (*launches kernels); sums (two kernels)
 cudaError_t launch_tree_box(const DevSim &s, const BuildScratch &b, int sm_count, cudaStream_t st);
 cudaError_t launch_tree_cells(const DevSim &s, const BuildScratch &b, int sm_count, cudaStream_t st, int *launches);
 cudaError_t launch_tree_sums(const DevSim &s, const BuildScratch &b, int quadrupole, int sm_count, cudaStream_t st);
 
 // Launch helpers implemented in the kernel translation units.
-struct LaunchShape {
-    int blocks;
-    int threads;
-};
-
 // trees with the reference's semantics beyond kRefPathBodies (k_tree.cu):
 // insertions from the root
 cudaError_t launch_reset(const DevSim &s, cudaStream_t st);

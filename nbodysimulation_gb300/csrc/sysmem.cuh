@@ -82,15 +82,6 @@ inline void sysmem_top_counts(const SysMem &m, int **p, size_t *bytes) {
     *bytes = m.top ? sizeof(int) << (3 * m.top_levels) : 0;
 }
 
-inline size_t sysmem_bytes(int n, bool tree, bool quad, int cap) {
-    SysMem m;
-    m.n = n;
-    m.tree = tree;
-    m.quad = quad;
-    m.cap = cap;
-    return sysmem_layout(m, nullptr);
-}
-
 // Descriptor of a system: its buffers and the step parameters of its config
 // (the same choices as the standalone step).
 // The top-level tables of a system building min(m.top_levels, cap) top
