@@ -35,10 +35,10 @@ constexpr int kCollideWarps = 8;                      // targets per block of th
 
 // Where the grid form (k_collide.cu) does not apply, the warp form serves fewer
 // blocks of targets than SMs (38,912 targets on 152 SMs), the block form the
-// rest.  Measured on a GB300,
-// unit ball, tree systems (targets in sort order), warp against block form:
-// N = 8,192 0.078 / 0.467 ms, 32,768 1.12 / 1.79 ms, 65,536 4.09 / 3.67 ms,
-// 262,144 62.0 / 25.6 ms.
+// rest.  Measured on a GB300, unit ball, tree systems (targets in sort order),
+// warp against block form: N = 8,192 0.078 / 0.467 ms, 32,768 1.12 / 1.79 ms, 65,536
+// 4.09 / 3.67 ms, 262,144 62.0 / 25.6 ms (the warp form before it loaded its bodies
+// ahead of the votes, which takes 8 to 14 % off it).
 inline int collide_warp_form_below(int sm_count) { return sm_count; }
 
 __device__ __forceinline__ float contact_distance() { return __fadd_rn(0.015f, 0.015f); }

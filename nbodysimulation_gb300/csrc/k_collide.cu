@@ -12,8 +12,9 @@
 // The pair tests of the first two are all there is to their time (n^2); the
 // grid leaves about 27 h^3 n / V candidates a target and is bound by its
 // scattered reads of them and, below 100,000 bodies, by its six launches.
-// Unit ball, tree systems, GB300, warp or block form against grid: N = 16,384
-// 0.307 -> 0.052 ms, 65,537 3.69 -> 0.064 ms, 262,144 25.6 -> 0.230 ms.
+// Unit ball, tree systems, GB300, warp or block form against grid: N = 20,000 0.49
+// -> 0.043 ms, 60,001 3.38 -> 0.063, 131,072 8.54 -> 0.117.  What the grid cannot
+// serve takes as long as without it (k_grid_rest_few, k_grid_rest).
 #include <algorithm>
 
 #include "collide_device.cuh"

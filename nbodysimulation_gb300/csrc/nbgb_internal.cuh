@@ -345,8 +345,8 @@ inline int collide_buckets(int n) {
     return b;
 }
 // Smallest system that takes the grid form: its six launches cost more than
-// the pair tests of a small system (unit ball, warp form against grid: N =
-// 2,048 0.024 / 0.044 ms, 4,096 0.042 / 0.046, 8,192 0.078 / 0.048).
+// the pair tests of a small system (unit ball, warp form against grid: N = 2,048
+// 0.024 / 0.044 ms, 4,096 0.042 / 0.046; 5,119 0.047, 5,120 0.035).
 constexpr int kCollideGridFrom = 5120;
 // tree != 0: s.sorted holds this step's in-order sort (the block form hands
 // its targets out in it); *launches gets the kernel count
