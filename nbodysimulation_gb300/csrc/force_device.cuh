@@ -45,13 +45,13 @@
 // Softened gravity F = m rsqrt(d^2)^3 (MUFU rsqrt), d^2 = |d|^2 + eps^2 as
 // FMAs; accepted cells optionally add their traceless quadrupole.
 //
-// Stack bound: kBatch cells are popped only while the stack holds at most
-// kBatchBelow entries, so a batch leaves at most kBatchBelow - 8 + 8*kBatch
-// entries and 7 more that wait for their vote (= kBatchBelow - 1 + 8*kBatch
-// together); beyond that the walk pops one cell at a time (depth first) and
-// votes at once, which adds at most 7 pending siblings per tree level: at most
-// 127 + 64 + 7*63 + 1 = 633 <= kStack entries for any tree of fewer than
-// kMaxDepth levels.  Entries pack (level << 26) | node.
+// Stack bound: kBatch cells are popped only while the stack holds at most `room`
+// entries, so a batch leaves at most room - 8 + 8*kBatch entries and 7 more that
+// wait for their vote (= room - 1 + 8*kBatch together); beyond that the walk pops
+// one cell at a time (depth first) and votes at once, which adds at most 7 pending
+// siblings per level of the tree and one more.  So room = kStack - 8*kBatch - 7 *
+// levels - 1: 255 for a tree of 63 levels, the most there are, and 549 for one of
+// 21.  Entries pack (level << 26) | node.
 //
 // The integrator writes the next position buffer, so every force of the step
 // sees step-start positions (the reference integrates in place while other
@@ -64,10 +64,17 @@ namespace nbgb {
 
 constexpr int kForceWarps = 2;
 constexpr int kForceThreads = kForceWarps * 32;
-constexpr int kStack = 640;
+constexpr int kStack = 768;
 constexpr int kBatch = 8;
 static_assert(kBatch == 8, "lane L holds child slot L%8 of popped cells L/8 and 4 + L/8");
-constexpr int kBatchBelow = 128;  // batch pops only while the stack holds at most this many
+// A single pop costs a whole round: with batches up to 128 entries only, the walks
+// of long stacks (the reference's opening rule, which opens every cell within
+// sqrt(eps)) took longer than the walk with a vote a cell did (ms, that walk / up
+// to 128 / now: cusps, 6,869 bodies 0.51 / 0.75 / 0.32, 60,000 6.01 / 12.4 / 3.49; 4M in
+// the reference's boxes, theta 1.5, 4.88 / 6.20 / 5.08).
+__device__ __forceinline__ int stack_room(int levels) {
+    return kStack - 8 * kBatch - 7 * min(levels, kMaxDepth - 1) - 1;
+}
 constexpr int kNodeBits = 26;
 constexpr int kNodeMask = (1 << kNodeBits) - 1;
 
@@ -240,11 +247,11 @@ __device__ __forceinline__ float warp_max(float v) { return key2f(__reduce_max_s
 // half, and the three additions across them.
 constexpr int kFlushTiles = 24;
 
-// Walk of warp group g of system s (dq: its 64 thresholds), with the fused
-// integrator.  All 32 lanes call it together.
+// Walk of warp group g of system s (dq: its 64 thresholds, room: its tree's
+// stack_room), with the fused integrator.  All 32 lanes call it together.
 template <int kMethod, bool kComp, bool kEpsZero, bool kQuad>
-__device__ __forceinline__ void force_group(const DevSim &s, const StepParams &p, const float *dq, int g, int lane,
-                                            WarpLists<kQuad> &ws) {
+__device__ __forceinline__ void force_group(const DevSim &s, const StepParams &p, const float *dq, int room, int g,
+                                            int lane, WarpLists<kQuad> &ws) {
     Ctrl *ctrl = s.ctrl;
     const int n = s.n, root = n + s.cap;
     const float eps2 = __fmul_rn(p.eps, p.eps);
@@ -360,7 +367,7 @@ __device__ __forceinline__ void force_group(const DevSim &s, const StepParams &p
         __syncwarp();
         // the undecided cells: every body of the group votes, eight cells at a
         // time (a lane tests cells L%4 and 4 + L%4 against its four bodies)
-        while (nu >= kTile8 || (nu > 0 && (sp == 0 || sp > kBatchBelow))) {
+        while (nu >= kTile8 || (nu > 0 && (sp == 0 || sp > room))) {
             const int cnt = min(nu, kTile8);
             nu -= cnt;
             const int i0 = nu + min(col, cnt - 1), i1 = nu + min(col + 4, cnt - 1);
@@ -404,7 +411,7 @@ __device__ __forceinline__ void force_group(const DevSim &s, const StepParams &p
         }
         // the next round's cells are popped and fetched before this round's
         // sums, which outlast the fetch
-        np = sp > kBatchBelow ? min(sp, 1) : min(sp, kBatch);
+        np = sp > room ? min(sp, 1) : min(sp, kBatch);
         sp -= np;
         n_open += np;
         e[0] = cidx < np ? ws.stack[sp + cidx] : 0;

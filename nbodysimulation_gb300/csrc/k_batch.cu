@@ -33,10 +33,10 @@ struct BatchForceWarp {
     // parameters, instead of holding them in registers
     DevSim view;
     StepParams par;
-    // the current system, its first group and its mode (0 walk, 1 keep the
-    // step-start state of a failed step, 2 inert): in shared memory, so
+    // the current system, its first group, its mode (0 walk, 1 keep the step-start
+    // state of a failed step, 2 inert) and its stack_room: in shared memory, so
     // nothing of the outer loop stays live in registers during a walk
-    int cur, begin, mode;
+    int cur, begin, mode, room;
 };
 constexpr int kBatchForceMaxWarps = 8;
 
@@ -84,6 +84,7 @@ __global__ void __maxnreg__(kMany ? 96 : 128) k_batch_force(BatchTables t) {
                 s_cur_w = k;
                 s_begin_w = d.group_begin;
                 s_mode_w = sk;
+                me.room = stack_room(v.ctrl->max_depth);
             }
             __syncwarp();
         }
@@ -96,7 +97,7 @@ __global__ void __maxnreg__(kMany ? 96 : 128) k_batch_force(BatchTables t) {
             if (i < s.n) s.body_next[i] = s.body_cur[i];
             continue;
         }
-        force_group<kMethod, kComp, false, kQuad>(s, s_par_w, s_dq_w, g, lane, me.lists);
+        force_group<kMethod, kComp, false, kQuad>(s, s_par_w, s_dq_w, me.room, g, lane, me.lists);
     }
 }
 

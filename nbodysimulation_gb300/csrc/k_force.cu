@@ -10,7 +10,7 @@ namespace nbgb {
 // registers), or nine (96) where the groups fill the GPU more than twice over.
 // What is resident follows from the shared memory too: of monopoles ten blocks with
 // 96 registers, whose extra warps hide more of the walk than its tighter schedule
-// costs; of compensated quadrupoles eight either way (26 KB a block), where the
+// costs; of compensated quadrupoles eight either way (27 KB a block), where the
 // schedule itself is the faster one.  With quadrupoles and without compensation
 // neither is (GB300, the walk in ms, bound eight / nine: monopoles, ball, 6,007
 // bodies 0.0635 / 0.0657, 131,072 0.207 / 0.207, 200,000 0.290 / 0.287, 262,144
@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force(DevSim s, Step
     wait_for_previous();
     __shared__ float s_dq[kMaxDepth];
     __shared__ WarpLists<kQuad> s_lists[kForceWarps];
-    __shared__ int s_skip;
+    __shared__ int s_skip, s_room;
     Ctrl *ctrl = s.ctrl;
     const int n = s.n;
     if (threadIdx.x == 0) {
@@ -32,6 +32,7 @@ __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force(DevSim s, Step
             skip = 1;
         }
         s_skip = skip;
+        s_room = stack_room(ctrl->max_depth);  // once a block: the line is busy with the counters
         float box[6];
         load_box(ctrl, box);
         make_thresholds(box, p.theta, p.eps, p.crit_ref, s_dq);
@@ -49,7 +50,7 @@ __global__ void __launch_bounds__(kForceThreads, kBlocks) k_force(DevSim s, Step
         if (lane == 0) g = atomicAdd(&ctrl->work, 1);
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= ngroups) break;
-        force_group<kMethod, kComp, kEpsZero, kQuad>(s, p, s_dq, g, lane, s_lists[w]);
+        force_group<kMethod, kComp, kEpsZero, kQuad>(s, p, s_dq, s_room, g, lane, s_lists[w]);
     }
 }
 
