@@ -50,11 +50,13 @@ __global__ void __launch_bounds__(kCollideWarps * 32) k_collision_warp(DevSim s)
 // ---------------------------------------------------------------------------
 constexpr int kGridThreads = 128;
 constexpr int kGridContacts = 64;
-// A target with more than n / 128 bodies around it goes to the overflow list at
-// once: a thread takes 0.4 us a candidate where nothing hides its latencies, a warp
-// n / 32 steps of 0.1 us for a target.  Targets ask for it where some bucket holds
-// more than its share of that, and more than kGridQuiet.
-constexpr int kGridCrowd = 128;
+// A target with too many bodies around it goes to the overflow list at once: a
+// thread takes 0.4 us a candidate where nothing hides its latencies, the warp form
+// about n^2 / 2^20 us for all n targets, of which the candidates may take two fifths;
+// and with 16 kGridContacts around it, it has more contacts than its list holds.
+// Targets ask for it where some bucket holds more than its share of that, and more
+// than kGridQuiet.
+__device__ __forceinline__ int grid_crowd(int n) { return (int)min((long long)n * n >> 20, 16LL * kGridContacts); }
 constexpr int kGridQuiet = 8;
 constexpr int kScanBuckets = 1024;  // buckets per block of the scan: consecutive in memory
 constexpr float kGridLimit = 262144.0f;
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(kScanBuckets / 4) k_grid_scan(DevSim s, Collid
     const int at = blockIdx.x * (kScanBuckets / 4) + threadIdx.x;
     const int4 c = reinterpret_cast<const int4 *>(g.count)[at];
     const int sum = c.x + c.y + c.z + c.w;
-    if (max(max(c.x, c.y), max(c.z, c.w)) > max(kGridQuiet, s.n / (27 * kGridCrowd))) g.ctl[kGridCrowded] = 1;
+    if (max(max(c.x, c.y), max(c.z, c.w)) > max(kGridQuiet, grid_crowd(s.n) / 27)) g.ctl[kGridCrowded] = 1;
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -152,15 +154,15 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_collide(DevSim s, Collide
     GridCell c;
     grid_cell(me, inv, c);
     // the rows' three buckets: one range when the scan laid them end to end
-    int cnt = 0;
+    int cnt = 0, crowd = 8 * kGridContacts;  // about that many bodies are around a target with kGridContacts contacts
     if (g.ctl[kGridCrowded]) {
-        int crowd = 0;
+        crowd = 0;
 #pragma unroll
         for (int row = 0; row < 9; ++row) {
             const unsigned b0 = (grid_row(c.y + row / 3 - 1, c.z + row % 3 - 1) + (unsigned)(c.x - 1)) & g.mask;
             if ((b0 & (kScanBuckets - 1)) + 2 < kScanBuckets) crowd += g.start[b0 + 2] + g.count[b0 + 2] - g.start[b0];
         }
-        if (crowd > s.n / kGridCrowd) cnt = kGridContacts + 1;
+        if (crowd > grid_crowd(s.n)) cnt = kGridContacts + 1;
     }
     for (int row = 0; row < 9 && cnt <= kGridContacts; ++row) {
         const int cy = c.y + row / 3 - 1, cz = c.z + row % 3 - 1;
@@ -184,6 +186,7 @@ __global__ void __launch_bounds__(kGridThreads) k_grid_collide(DevSim s, Collide
     if (cnt == 0) return;
     if (cnt > kGridContacts) {
         g.rank[atomicAdd(&g.ctl[kGridOverflow], 1)] = i;  // the ranks are no longer needed
+        atomicAdd(reinterpret_cast<unsigned long long *>(&g.ctl[kGridAround]), (unsigned long long)crowd);
         return;
     }
     float4 v = s.vel[i];
@@ -230,12 +233,29 @@ __global__ void __launch_bounds__(kCollideWarps * 32, 8) k_grid_rest_few(DevSim 
     const bool all = g.ctl[kGridNoCell] != 0;
     rest_by_warps(s, g, all, all ? s.n : g.ctl[kGridOverflow]);
 }
-__global__ void __launch_bounds__(kCollideThreads, 8) k_grid_rest(DevSim s, CollideGrid g, const int *order, int few) {
+// Systems that may have many.  A target that meets few bodies is the warps' (32 of
+// its pairs a step), one that meets thousands a thread's: its reflections follow one
+// another, and 32 targets share a warp.  An eighth of the bodies around a target
+// (`around`, all targets together) are its contacts.  In us, from the times of both
+// forms alone: a warp's step 0.1, its contact 0.15, up to 24 warps per SM; a body of
+// the blocks' tiles 0.05, up to three blocks per SM, their contact 0.3.  (60,001
+// bodies, an eighth in a core: warps 2.6 ms, blocks 3.9; 59,157 bodies of a cusp 92
+// and 11.)
+__device__ __forceinline__ bool warps_are_faster(int n, int cnt, unsigned long long around, int sm_count) {
+    const int warps = min(min(cnt, (int)gridDim.x * kCollideWarps), 24 * sm_count);
+    const float contacts = 0.125f * (float)around, targets = (float)cnt;
+    return (0.1f * targets * (float)n / 32.0f + 0.15f * contacts) / (float)warps <
+           0.05f * (float)n * fmaxf(1.0f, targets / (float)(3 * kCollideThreads * sm_count)) + 0.3f * contacts / targets;
+}
+__global__ void __launch_bounds__(kCollideThreads, 8) k_grid_rest(DevSim s, CollideGrid g, const int *order,
+                                                                  int sm_count) {
     wait_for_previous();
     if (read_status(s.ctrl)) return;  // block-uniform, before any barrier
     const bool all = g.ctl[kGridNoCell] != 0;
     const int cnt = all ? s.n : g.ctl[kGridOverflow];
-    if (cnt < few) return rest_by_warps(s, g, all, cnt);
+    if (cnt == 0) return;
+    if (!all && warps_are_faster(s.n, cnt, *reinterpret_cast<const unsigned long long *>(&g.ctl[kGridAround]), sm_count))
+        return rest_by_warps(s, g, all, cnt);
     if ((int)blockIdx.x * kCollideThreads >= cnt) return;
     collide_block(s.body_next, s.vel, all ? order : g.rank, cnt, s.n, blockIdx.x * kCollideThreads, s.ctrl);
 }
@@ -265,7 +285,7 @@ cudaError_t launch_collision(const DevSim &s, const CollideGrid &g, int tree, in
     // not early, so that the block form's few long blocks spread evenly (launch.cuh;
     // 60,001 bodies, one far out: 3.50 ms, early 4.02)
     k_grid_rest<<<(s.n + kCollideThreads - 1) / kCollideThreads, kCollideThreads, 0, st>>>(
-        s, g, tree ? s.sorted : nullptr, few);
+        s, g, tree ? s.sorted : nullptr, sm_count);
     return cudaGetLastError();
 }
 

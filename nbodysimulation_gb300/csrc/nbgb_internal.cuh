@@ -332,7 +332,7 @@ cudaError_t launch_direct(const DevSim &s, const StepParams &p, const DirectPlan
 // and, behind them, the control words; bucket starts; each body's place in its
 // bucket (then the overflow list); the bodies in bucket order.  All null: the
 // system takes the warp form.
-enum { kGridCursor = 0, kGridNoCell = 1, kGridOverflow = 2, kGridNext = 3, kGridCrowded = 4, kGridCtl = 8 };
+enum { kGridCursor = 0, kGridNoCell = 1, kGridOverflow = 2, kGridNext = 3, kGridCrowded = 4, kGridAround = 6, kGridCtl = 8 };
 struct CollideGrid {
     int *count, *ctl, *start, *rank;
     float4 *body;

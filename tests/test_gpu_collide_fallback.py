@@ -62,3 +62,38 @@ def test_fallbacks_take_little_longer(gpu, kind):
                 took.append(s.timings()["collision"])
             ms.append(min(took))
     assert ms[1] < 3.0 * ms[0]
+
+
+def cusp(n, inner=-4.0):
+    """Half of the bodies within the contact distance of one another."""
+    rng = np.random.default_rng(n)
+    d = rng.normal(size=(n, 3))
+    return (d / np.linalg.norm(d, axis=1)[:, None] * 10.0 ** rng.uniform(inner, 1, (n, 1))).astype(np.float32)
+
+
+@pytest.mark.parametrize("n,inner", [(5120, -4.0), (20011, -1.0), (38912, -1.5), (38913, -4.0)])
+def test_cusp_bit_exact(gpu, oracle, n, inner):
+    """Targets with thousands of contacts, and ones between those and the grid's."""
+    pos = cusp(n, inner)
+    vel = (0.1 * np.random.default_rng(n + 1).normal(size=(n, 3))).astype(np.float32)
+    with handle(gpu, pos, vel) as s:
+        s.step(0.0, 1)
+        got = s.get_state()[1]
+    np.testing.assert_array_equal(got, oracle.collision(pos, vel))
+
+
+def test_thousands_of_contacts_take_the_block_form(gpu):
+    """59,157 bodies of a cusp against as many in a ball with one far out, which
+    all go through the blocks: their reflections take three times as long as all
+    pair tests, a warp a target 25 times."""
+    ms = []
+    for pos in (layout("far", 59157), cusp(59157)):
+        with handle(gpu, pos) as s:
+            s.step(0.0, 1)
+            s.set_profiling(True)
+            took = []
+            for _ in range(3):
+                s.step(0.0, 1)
+                took.append(s.timings()["collision"])
+            ms.append(min(took))
+    assert ms[1] < 8.0 * ms[0]
