@@ -97,3 +97,15 @@ def test_thousands_of_contacts_take_the_block_form(gpu):
                 took.append(s.timings()["collision"])
             ms.append(min(took))
     assert ms[1] < 8.0 * ms[0]
+
+
+def test_all_in_contact_behind_the_direct_sums(gpu):
+    """2,859 bodies, each in contact with all: the update is all there is to the step
+    (0.64 ms of it) and takes a direct system what it takes a tree system."""
+    pos = (1e-12 * np.random.default_rng(2859).uniform(-1, 1, (2859, 3))).astype(np.float32)
+    ms = []
+    for algo in (0, 1):
+        with handle(gpu, pos, algo=algo) as s:
+            s.step(0.0, 2)
+            ms.append(min(s.time_steps(0.0, 4) for _ in range(6)))
+    assert ms[1] < 1.2 * ms[0]
